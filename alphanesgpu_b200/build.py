@@ -23,6 +23,10 @@ SOURCES = {
     "neighbor.cu": ["-fmad=false"],
     "ops.cu": [],
     "fused.cu": [],
+    "sweep_f32.cu": [],
+    "sweep_f64.cu": [],
+    "mlp_f32.cu": [],
+    "mlp_f64.cu": [],
     "peer.cu": [],
     "halo.cu": [],
     "libstaf_api.cu": [],

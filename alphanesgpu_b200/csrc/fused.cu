@@ -6,78 +6,12 @@
 // their derivatives, neighbour ids, grouped by species: ~2 KB, common.cuh) and every sweep (sweep.cuh)
 // rebuilds the triplet geometry in registers from the record staged in shared memory.
 //
-// This file: the evaluation's housekeeping kernel, the loss, Adam, the model handle and the launch
+// This file: the evaluation's housekeeping kernel, the loss, Adam, the making of the model handle and the launch
 // sequences behind the fused entry points of include/stafb.h.  Math: STAF/staf_models/staf_model.py:168-258.
-#include <math.h>
-#include <stdlib.h>
-#include <string.h>
-#include <type_traits>
-#include "common.cuh"
+#include <algorithm>
+#include "model.cuh"
 
 namespace stafb {
-
-constexpr int ML_THREADS = 256;
-
-struct ModelDev {
-  int nt, C, N, ncls;
-  int tipos[STAFB_MAX_TYPES], shift[STAFB_MAX_TYPES + 1], Fr[STAFB_MAX_TYPES], Fa[STAFB_MAX_TYPES];
-  int off_a2[STAFB_MAX_TYPES], off_a3[STAFB_MAX_TYPES], off_mu[STAFB_MAX_TYPES], off_w[STAFB_MAX_TYPES];
-  int off_emb[STAFB_MAX_TYPES];
-  int n_dense, width[STAFB_MAX_DENSE];
-  int Fmax, Frmax, Famax, Hsum, maxw;
-  __host__ __device__ int in_of(int t, int l) const { return l == 0 ? Fr[t] + Fa[t] : width[l - 1]; }
-  __host__ __device__ int w_off(int t, int l) const {
-    int s = 0;
-    for (int k = 0; k < l; k++) s += in_of(t, k) * width[k] + width[k];
-    return s;
-  }
-  __host__ __device__ int h_off(int l) const {  // offset of the output of Dense l in the activation row
-    int s = 0;
-    for (int k = 0; k < l; k++) s += width[k];
-    return s;
-  }
-  __host__ __device__ int type_of(int id) const {
-    int t = 0;
-    while (t < nt - 1 && id >= shift[t + 1]) t++;
-    return t;
-  }
-};
-
-// species-major enumeration: block -> (species t, index q0 of its first atom among the nf*tipos[t]
-// atoms of that species); W atoms per block, blocks never mix species
-__device__ __forceinline__ void locate_block(const ModelDev& md, int nf, int W, int& t, int& q0) {
-  int blk = blockIdx.x;
-  t = 0;
-  while (t < md.nt - 1) {
-    const int nb = (nf * md.tipos[t] + W - 1) / W;
-    if (blk < nb) break;
-    blk -= nb;
-    t++;
-  }
-  q0 = blk * W;
-}
-
-__device__ __forceinline__ bool locate_atom(const ModelDev& md, int nf, int W, int slot, int& t, int& b, int& i) {
-  int q0;
-  locate_block(md, nf, W, t, q0);
-  const int q = q0 + slot;
-  if (q >= nf * md.tipos[t]) return false;
-  b = q / md.tipos[t];
-  i = md.shift[t] + (q - b * md.tipos[t]);
-  return true;
-}
-
-static inline int species_blocks(const ModelDev& md, int nf, int W) {
-  int s = 0;
-  for (int t = 0; t < md.nt; t++) s += (nf * md.tipos[t] + W - 1) / W;
-  return s;
-}
-
-#include "sweep.cuh"
-
-// ---------------------------------------------------------------------------- MLP head
-#include "mlp.cuh"
-#include "mlp_mma.cuh"
 
 // ---------------------------------------------------------------------------- energy, loss
 template <class T>
@@ -325,88 +259,6 @@ __global__ void k_adam_dev(int n, T* __restrict__ theta, const T* __restrict__ g
 
 }  // namespace stafb
 
-using namespace stafb;
-
-struct stafb_model {
-  stafb_ctx* ctx;
-  ModelDev md;
-  int n_params, n_emb;
-  int blk_size[STAFB_MAX_TYPES];
-  size_t es;
-  int cap_atoms;  // atoms per frame the scratch was sized for
-  int aw;   // atoms per warp of the MLP kernels (4, 2 or 1; a block of eight warps owns 8*aw atoms)
-  int stage;  // Dense layers in shared memory: 2 all at kernel start, 1 one at a time, 0 none
-  size_t mlp_fwd_smem, mlp_bwd_smem;
-  // scratch for max_batch frames
-  void *rows, *af, *nd, *acts, *e_atom, *force, *flab, *ebar, *gradnet, *gaf, *energy, *vrow;
-  int row_stride;      // bytes per neighbour record (common.cuh)
-  unsigned char* spar;  // per-species parameter blocks of the sweeps, rewritten by k_prep at every evaluation
-  SparLayout sl;
-  void* wpack;  // packed, padded Dense layers of every species (k_prep), wstride elements per species
-  int wstride;
-  int nv;  // row length of vrow: nt*Frmax + C*3*Famax
-  // tensor-core MLP kernels (fp32): on/off, warps per block (16 atoms), the fragment-ordered pack and its
-  // per-species stride, dynamic shared memory of the two kernels
-  int mma, mma_nw, mma_stage, wm_stride;
-  void* wm;
-  size_t mma_fwd_smem, mma_bwd_smem;
-  double* epart;     // partial energy sums of k_loss: [nf][eb]; from [max_batch][LOSS_EB_MAX] on: one arrival counter per frame
-  double* losses_d;  // [0..4] the four losses + the done-counter of k_loss; [8 + b] sum of the atomic energies of
-                     // frame b (accumulated by the MLP kernel); from [8 + max_batch] on the virial accumulators [b][9][VIR_SLOTS]
-  // staging for the *_host entry points
-  // two pipelined slots for stafb_train_step_host_begin/_end: pinned input block (pos | f_label | box | e_label),
-  // pinned results (4 losses + status) and the event that marks the slot's step complete
-  char* slot_in_h[3];  // slots 0, 1: the pipelined calls; slot 2: the synchronous stafb_train_step_host
-  double* slot_out_h[3];
-  cudaEvent_t slot_done[3];
-  int slot_busy[3];
-  // per slot: the captured graph of (copy in, step, copy out) and the call signature it was captured for
-  struct SlotKey {
-    int nf, loss_kind;
-    const void *theta, *emb, *grad, *stream;
-    double pe, pf, pb, bound, pv;
-    int with_v;
-  } slot_key[3];
-  double* mirror_next;  // mapped host memory the next training evaluation's k_loss writes its results to
-  void* vlab_d;         // device copy of the virial labels of a host-buffer step [max_batch][9]
-  int slot_state[3];  // 0: nothing yet, 1: signature seen once (ran eagerly), 2: graph instantiated, -1: capture failed
-  cudaGraphExec_t slot_exec[3];
-  // Two more sets of neighbour rows (a context of their own for the search scratch + the compact rows), so that
-  // the geometry of the NEXT step, which depends on no trainable parameter, can be built on another stream while
-  // this step's sweeps still read theirs.  Allocated on first use.
-  struct NlSet {
-    stafb_ctx* ctx;
-    void* rows;
-    cudaEvent_t ready;
-    int nf;  // frames the set currently describes (0: nothing)
-  } nl[2];
-  cudaStream_t side;  // stream of the prefetches issued by stafb_train_step_host_begin
-  cudaGraphExec_t nl_exec[2];
-  size_t smem_limit;
-};
-
-// words of shared memory the staged Dense layers need: stage 1 = the largest (in + 1) x row stride over the
-// layers, stage 2 = all layers of one species back to back
-static size_t mlp_stage_words(const ModelDev& d, int stage) {
-  size_t best = 0;
-  for (int t = 0; t < d.nt; t++) {
-    size_t sum = 0;
-    for (int l = 0; l < d.n_dense; l++) {
-      const size_t wds = (size_t)(d.in_of(t, l) + 1) * ml_ld(d.width[l]);
-      sum += wds;
-      if (stage == 1) best = wds > best ? wds : best;
-    }
-    if (stage == 2) best = sum > best ? sum : best;
-  }
-  return stage ? best : 0;
-}
-static size_t mlp_smem_fwd(const ModelDev& d, size_t es, int aw, int stage) {
-  return es * (ML_WARPS * ml_fwd_words(d.Fmax, d.Hsum, d.maxw, aw) + mlp_stage_words(d, stage));
-}
-static size_t mlp_smem_bwd(const ModelDev& d, size_t es, int aw, int stage) {
-  return es * (ML_WARPS * ml_bwd_words(d.Fmax, d.Hsum, d.maxw, aw) + mlp_stage_words(d, stage));
-}
-
 extern "C" int stafb_model_create(stafb_ctx* c, const int* sd, stafb_model** out) {
   if (!c || !sd || !out) return STAFB_ERR_INVALID;
   stafb_model* m = (stafb_model*)calloc(1, sizeof(stafb_model));
@@ -601,74 +453,6 @@ extern "C" void stafb_model_offsets(const stafb_model* m, int t, int out6[6]) {
   out6[4] = m->md.off_emb[t]; out6[5] = m->blk_size[t];
 }
 
-// cudaFuncSetAttribute applies to the device that is current when it is called, and one process may drive
-// several GPUs (staf_load honours StafOptions.device_id; stafb_peer_connect_local exists for that use): the
-// "already opted in" notes of the launchers below are therefore kept per device, as the reference keeps its
-// per-device context map (STAF/src/descriptor_builder/reforce.cc:143-158).
-constexpr int MAX_DEVICES = 64;
-static inline int device_slot() {
-  int d = 0;
-  cudaGetDevice(&d);
-  return (d >= 0 && d < MAX_DEVICES) ? d : 0;
-}
-
-// what a sweep launch needs besides the model: the records of this evaluation and the per-call buffers
-template <class T>
-struct SweepCall {
-  const void* rows;
-  int nf, nall;
-  const T* chan_in;
-  const T* force;  // force-backward sweep: the forces, their labels and the loss's scale (dL/dF is formed on the fly)
-  const T* flab;
-  T fscale;
-  int loss_kind;
-  T* out;
-  T* grad;
-  T* vout;
-  double* vir;
-  const double* vacc;  // force backward with a virial loss: the virials, their labels, the loss's scale
-  const T* vlab;
-  T vscale;
-  int* status;
-};
-
-template <class T, int MODE>
-static int launch_sweep(stafb_model* m, cudaStream_t s, const SweepCall<T>& call) {
-  const ModelDev& d = m->md;
-  const int nr = m->ctx->nr;
-  const SweepSmem L = sweep_smem<T>(d, m->sl, nr, MODE);
-  const size_t sm = (size_t)L.total;
-  if (sm > m->smem_limit) return STAFB_ERR_CAPACITY;
-  static bool attr_dev[MAX_DEVICES] = {false};  // per instantiation (T, MODE) and device
-  bool& attr_done = attr_dev[device_slot()];
-  if (sm > 48 * 1024 && !attr_done) {
-    STAFB_CUDA_OK(cudaFuncSetAttribute(k_sweep<T, MODE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)m->smem_limit));
-    if (MODE == MODE_FORCE)
-      STAFB_CUDA_OK(cudaFuncSetAttribute(k_sweep<T, MODE, MODE == MODE_FORCE>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m->smem_limit));
-    attr_done = true;
-  }
-  SweepArgs<T> a;
-  a.rows = static_cast<const unsigned char*>(call.rows);
-  a.row_stride = m->row_stride;
-  a.nr = nr; a.nf = call.nf; a.nall = call.nall;
-  a.spar = m->spar;
-  a.spar_stride = m->sl.total;
-  a.sl = m->sl;
-  a.chan_in = call.chan_in; a.force = call.force; a.flab = call.flab; a.fscale = call.fscale;
-  a.loss_kind = call.loss_kind; a.out = call.out; a.grad = call.grad;
-  a.vout = call.vout; a.nv = m->nv; a.vir = call.vir; a.status = call.status;
-  a.vacc = call.vacc; a.vlab = call.vlab; a.vscale = call.vscale;
-  const int blocks = call.nf * d.N;
-  if (MODE == MODE_FORCE && call.vir)
-    STAFB_CUDA_OK(launch_chained(k_sweep<T, MODE, MODE == MODE_FORCE>, blocks, 32, sm, s, d, a, L));
-  else
-    STAFB_CUDA_OK(launch_chained(k_sweep<T, MODE, false>, blocks, 32, sm, s, d, a, L));
-  m->ctx->launches++;
-  return STAFB_OK;
-}
-
 // where the neighbour kernels leave the records of a model's atoms
 static RowSink row_sink(const stafb_model* m, void* rows, const int* tmap) {
   RowSink sk;
@@ -679,106 +463,6 @@ static RowSink row_sink(const stafb_model* m, void* rows, const int* tmap) {
   for (int t = 0; t <= m->md.nt; t++) sk.shift[t] = m->md.shift[t];
   sk.tmap = tmap;
   return sk;
-}
-
-template <class T, int AW, bool WG, bool WIDE>
-static int launch_mlp_fwd_t(stafb_model* m, cudaStream_t s, int nf, const T* theta, const T* af, T* acts, T* e_atom,
-                            T* nd) {
-  static size_t attr_dev[MAX_DEVICES] = {0};  // largest dynamic shared-memory size opted in for, per device
-  size_t& attr = attr_dev[device_slot()];
-  if (m->mlp_fwd_smem > 48 * 1024 && m->mlp_fwd_smem > attr) {
-    STAFB_CUDA_OK(cudaFuncSetAttribute(k_mlp_fwd<T, AW, WG, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)m->mlp_fwd_smem));
-    attr = m->mlp_fwd_smem;
-  }
-  STAFB_CUDA_OK(launch_chained(k_mlp_fwd<T, AW, WG, WIDE>, species_blocks(m->md, nf, ML_WARPS * AW), ML_THREADS,
-                               m->mlp_fwd_smem, s, m->md, nf, theta, (const T*)m->wpack, m->wstride, af, acts, e_atom,
-                               nd, m->stage, (int)mlp_stage_words(m->md, m->stage)));
-  m->ctx->launches++;
-  return STAFB_OK;
-}
-
-template <class T, int AW, bool WG, bool WIDE>
-static int launch_mlp_bwd_t(stafb_model* m, cudaStream_t s, int nf, const T* theta, const T* af, const T* acts,
-                            const T* ebar, const T* u, T* gaf, T* grad) {
-  static size_t attr_dev[MAX_DEVICES] = {0};
-  size_t& attr = attr_dev[device_slot()];
-  const T* vrow = (const T*)m->vrow;
-  if (m->mlp_bwd_smem > 48 * 1024 && m->mlp_bwd_smem > attr) {
-    STAFB_CUDA_OK(cudaFuncSetAttribute(k_mlp_bwd<T, AW, WG, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)m->mlp_bwd_smem));
-    attr = m->mlp_bwd_smem;
-  }
-  STAFB_CUDA_OK(launch_chained(k_mlp_bwd<T, AW, WG, WIDE>, species_blocks(m->md, nf, ML_WARPS * AW), ML_THREADS,
-                               m->mlp_bwd_smem, s, m->md, nf, theta, (const T*)m->wpack, m->wstride, af, acts, ebar, u,
-                               vrow, m->nv, gaf, grad, m->stage, (int)mlp_stage_words(m->md, m->stage)));
-  m->ctx->launches++;
-  return STAFB_OK;
-}
-
-static int launch_mlp_fwd_mma(stafb_model* m, cudaStream_t s, int nf, const float* theta, const float* af, float* acts,
-                              float* e_atom, float* nd) {
-  static size_t attr_dev[MAX_DEVICES] = {0};
-  size_t& attr = attr_dev[device_slot()];
-  if (m->mma_fwd_smem > 48 * 1024 && m->mma_fwd_smem > attr) {
-    STAFB_CUDA_OK(cudaFuncSetAttribute(k_mlp_fwd_mma, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)m->mma_fwd_smem));
-    attr = m->mma_fwd_smem;
-  }
-  STAFB_CUDA_OK(launch_chained(k_mlp_fwd_mma, species_blocks(m->md, nf, MM_ATOMS), 32 * m->mma_nw, m->mma_fwd_smem, s,
-                               m->md, nf, theta, (const float*)m->wm, m->wm_stride, af, acts, e_atom, nd));
-  m->ctx->launches++;
-  return STAFB_OK;
-}
-
-static int launch_mlp_bwd_mma(stafb_model* m, cudaStream_t s, int nf, const float* theta, const float* af,
-                              const float* acts, const float* ebar, const float* u, float* gaf, float* grad) {
-  static size_t attr_dev[MAX_DEVICES] = {0};
-  size_t& attr = attr_dev[device_slot()];
-  if (m->mma_bwd_smem > 48 * 1024 && m->mma_bwd_smem > attr) {
-    STAFB_CUDA_OK(cudaFuncSetAttribute(k_mlp_bwd_mma, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)m->mma_bwd_smem));
-    attr = m->mma_bwd_smem;
-  }
-  STAFB_CUDA_OK(launch_chained(k_mlp_bwd_mma, species_blocks(m->md, nf, MM_ATOMS), 32 * m->mma_nw, m->mma_bwd_smem, s,
-                               m->md, nf, theta, (const float*)m->wm, m->wm_stride, af, acts, ebar, u,
-                               (const float*)m->vrow, m->nv, gaf, grad));
-  m->ctx->launches++;
-  return STAFB_OK;
-}
-
-template <class T>
-static int launch_mlp_fwd(stafb_model* m, cudaStream_t s, int nf, const T* theta, const T* af, T* acts, T* e_atom,
-                          T* nd) {
-  if constexpr (std::is_same<T, float>::value) {
-    if (m->mma) return launch_mlp_fwd_mma(m, s, nf, theta, af, acts, e_atom, nd);
-  }
-  const bool wg = m->stage == 0, wide = m->md.maxw > 64;  // the dense products' form: see mlp.cuh
-  switch (m->aw) {
-    case 4: return wg ? (wide ? launch_mlp_fwd_t<T, 4, true, true>(m, s, nf, theta, af, acts, e_atom, nd) : launch_mlp_fwd_t<T, 4, true, false>(m, s, nf, theta, af, acts, e_atom, nd))
-                      : (wide ? launch_mlp_fwd_t<T, 4, false, true>(m, s, nf, theta, af, acts, e_atom, nd) : launch_mlp_fwd_t<T, 4, false, false>(m, s, nf, theta, af, acts, e_atom, nd));
-    case 2: return wg ? (wide ? launch_mlp_fwd_t<T, 2, true, true>(m, s, nf, theta, af, acts, e_atom, nd) : launch_mlp_fwd_t<T, 2, true, false>(m, s, nf, theta, af, acts, e_atom, nd))
-                      : (wide ? launch_mlp_fwd_t<T, 2, false, true>(m, s, nf, theta, af, acts, e_atom, nd) : launch_mlp_fwd_t<T, 2, false, false>(m, s, nf, theta, af, acts, e_atom, nd));
-    default: return wg ? (wide ? launch_mlp_fwd_t<T, 1, true, true>(m, s, nf, theta, af, acts, e_atom, nd) : launch_mlp_fwd_t<T, 1, true, false>(m, s, nf, theta, af, acts, e_atom, nd))
-                       : (wide ? launch_mlp_fwd_t<T, 1, false, true>(m, s, nf, theta, af, acts, e_atom, nd) : launch_mlp_fwd_t<T, 1, false, false>(m, s, nf, theta, af, acts, e_atom, nd));
-  }
-}
-
-template <class T>
-static int launch_mlp_bwd(stafb_model* m, cudaStream_t s, int nf, const T* theta, const T* af, const T* acts,
-                          const T* ebar, const T* u, T* gaf, T* grad) {
-  if constexpr (std::is_same<T, float>::value) {
-    if (m->mma) return launch_mlp_bwd_mma(m, s, nf, theta, af, acts, ebar, u, gaf, grad);
-  }
-  const bool wg = m->stage == 0, wide = m->md.maxw > 64;  // the dense products' form: see mlp.cuh
-  switch (m->aw) {
-    case 4: return wg ? (wide ? launch_mlp_bwd_t<T, 4, true, true>(m, s, nf, theta, af, acts, ebar, u, gaf, grad) : launch_mlp_bwd_t<T, 4, true, false>(m, s, nf, theta, af, acts, ebar, u, gaf, grad))
-                      : (wide ? launch_mlp_bwd_t<T, 4, false, true>(m, s, nf, theta, af, acts, ebar, u, gaf, grad) : launch_mlp_bwd_t<T, 4, false, false>(m, s, nf, theta, af, acts, ebar, u, gaf, grad));
-    case 2: return wg ? (wide ? launch_mlp_bwd_t<T, 2, true, true>(m, s, nf, theta, af, acts, ebar, u, gaf, grad) : launch_mlp_bwd_t<T, 2, true, false>(m, s, nf, theta, af, acts, ebar, u, gaf, grad))
-                      : (wide ? launch_mlp_bwd_t<T, 2, false, true>(m, s, nf, theta, af, acts, ebar, u, gaf, grad) : launch_mlp_bwd_t<T, 2, false, false>(m, s, nf, theta, af, acts, ebar, u, gaf, grad));
-    default: return wg ? (wide ? launch_mlp_bwd_t<T, 1, true, true>(m, s, nf, theta, af, acts, ebar, u, gaf, grad) : launch_mlp_bwd_t<T, 1, true, false>(m, s, nf, theta, af, acts, ebar, u, gaf, grad))
-                       : (wide ? launch_mlp_bwd_t<T, 1, false, true>(m, s, nf, theta, af, acts, ebar, u, gaf, grad) : launch_mlp_bwd_t<T, 1, false, false>(m, s, nf, theta, af, acts, ebar, u, gaf, grad));
-  }
 }
 
 // Domain mode of the fused path: one frame of nall atoms whose first N (the model's species-sorted

@@ -1,4 +1,4 @@
-// Per-species MLP energy head of the fused path (included by fused.cu inside namespace stafb).
+// Per-species MLP energy head of the fused path (included by model.cuh inside namespace stafb).
 //
 // x = log(AF+1e-3) - mu ; Dense(tanh)... Dense(1)  (staf_models/staf_model.py:188-191,
 // libstaf/src/mlp/staf_mlp_ort.cc:196-242 of the reference).

@@ -1,4 +1,4 @@
-// fp32 MLP energy head on the tensor cores (included by fused.cu inside namespace stafb, after mlp.cuh): the
+// fp32 MLP energy head on the tensor cores (included by model.cuh inside namespace stafb, after mlp.cuh): the
 // opt-in arm of the MLP kernels (STAFB_MLP_MMA=1 when the model is created).
 //
 // Same mathematics as k_mlp_fwd / k_mlp_bwd of mlp.cuh (staf_models/staf_model.py:188-195,225-228 of the
@@ -227,7 +227,7 @@ __device__ __forceinline__ void mm_gemm(const float* __restrict__ A1, const floa
 
 // Forward: e_i, the activations for the backward kernel ([block][16][padded widths]) and
 // netderiv = d(sum e)/dAF.  Block = 16 atoms, gw = blockDim.x / 32 warps.
-__global__ void __launch_bounds__(32 * MM_MAX_WARPS)
+static __global__ void __launch_bounds__(32 * MM_MAX_WARPS)
     k_mlp_fwd_mma(ModelDev md, int nf, const float* __restrict__ theta, const float* __restrict__ wm, int wm_stride,
                   const float* __restrict__ af, float* __restrict__ acts, float* __restrict__ e_atom,
                   float* __restrict__ netderiv) {
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(32 * MM_MAX_WARPS)
 // Backward of  S = sum_a ebar[a] e[a] + sum_{a,c} u[a,c] netderiv[a,c]  with respect to the weights, mu and AF
 // (the second term: tangent v = u/(AF + eps) pushed forward, then reversed), and the contraction of dL/dAF with
 // the per-atom d(AF)/d(alpha) rows of the fingerprint sweep - as k_mlp_bwd of mlp.cuh.
-__global__ void __launch_bounds__(32 * MM_MAX_WARPS)
+static __global__ void __launch_bounds__(32 * MM_MAX_WARPS)
     k_mlp_bwd_mma(ModelDev md, int nf, const float* __restrict__ theta, const float* __restrict__ wm, int wm_stride,
                   const float* __restrict__ af, const float* __restrict__ acts, const float* __restrict__ ebar,
                   const float* __restrict__ u, const float* __restrict__ vrow, int nv, float* __restrict__ gaf,

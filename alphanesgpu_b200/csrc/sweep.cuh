@@ -1,4 +1,4 @@
-// Sweep kernels of the fused path (included by fused.cu inside namespace stafb): atomic fingerprints, forces and
+// Sweep kernels of the fused path (included by model.cuh inside namespace stafb): atomic fingerprints, forces and
 // the backward of the forces, each as one pass over the triplets of every central atom.
 //
 // One warp owns one central atom.  Its neighbour record (common.cuh: unit vectors, cutoffs, radial descriptors,

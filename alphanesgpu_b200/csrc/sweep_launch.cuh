@@ -1,0 +1,44 @@
+// Launches of the sweeps (sweep.cuh), instantiated for REAL by sweep_f32.cu and sweep_f64.cu.
+#include "model.cuh"
+
+template <class T, int MODE>
+int launch_sweep(stafb_model* m, cudaStream_t s, const SweepCall<T>& call) {
+  const ModelDev& d = m->md;
+  const int nr = m->ctx->nr;
+  const SweepSmem L = sweep_smem<T>(d, m->sl, nr, MODE);
+  const size_t sm = (size_t)L.total;
+  if (sm > m->smem_limit) return STAFB_ERR_CAPACITY;
+  static bool attr_dev[MAX_DEVICES] = {false};  // per instantiation (T, MODE) and device
+  bool& attr_done = attr_dev[device_slot()];
+  if (sm > 48 * 1024 && !attr_done) {
+    STAFB_CUDA_OK(cudaFuncSetAttribute(k_sweep<T, MODE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)m->smem_limit));
+    if (MODE == MODE_FORCE)
+      STAFB_CUDA_OK(cudaFuncSetAttribute(k_sweep<T, MODE, MODE == MODE_FORCE>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m->smem_limit));
+    attr_done = true;
+  }
+  SweepArgs<T> a;
+  a.rows = static_cast<const unsigned char*>(call.rows);
+  a.row_stride = m->row_stride;
+  a.nr = nr; a.nf = call.nf; a.nall = call.nall;
+  a.spar = m->spar;
+  a.spar_stride = m->sl.total;
+  a.sl = m->sl;
+  a.chan_in = call.chan_in; a.force = call.force; a.flab = call.flab; a.fscale = call.fscale;
+  a.loss_kind = call.loss_kind; a.out = call.out; a.grad = call.grad;
+  a.vout = call.vout; a.nv = m->nv; a.vir = call.vir; a.status = call.status;
+  a.vacc = call.vacc; a.vlab = call.vlab; a.vscale = call.vscale;
+  const int blocks = call.nf * d.N;
+  if (MODE == MODE_FORCE && call.vir)
+    STAFB_CUDA_OK(launch_chained(k_sweep<T, MODE, MODE == MODE_FORCE>, blocks, 32, sm, s, d, a, L));
+  else
+    STAFB_CUDA_OK(launch_chained(k_sweep<T, MODE, false>, blocks, 32, sm, s, d, a, L));
+  m->ctx->launches++;
+  return STAFB_OK;
+}
+
+template int launch_sweep<REAL, MODE_AF>(stafb_model*, cudaStream_t, const SweepCall<REAL>&);
+template int launch_sweep<REAL, MODE_AFV>(stafb_model*, cudaStream_t, const SweepCall<REAL>&);
+template int launch_sweep<REAL, MODE_FORCE>(stafb_model*, cudaStream_t, const SweepCall<REAL>&);
+template int launch_sweep<REAL, MODE_FGRAD>(stafb_model*, cudaStream_t, const SweepCall<REAL>&);
