@@ -62,31 +62,70 @@ __device__ __forceinline__ float ex2_fast(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// exp(x) in double precision, table-driven (P. T. P. Tang, ACM TOMS 15, 1989): with n = round(16 x / ln 2), x = n ln2/16 +
+// r, |r| <= ln2/32, exp(x) = 2^(n div 16) * 2^((n mod 16)/16) * e^r and e^r - 1 = r + r^2 q(r), q the degree-4 Chebyshev
+// interpolant of (e^r - 1 - r)/r^2 (error 2.8e-17).  Eleven double operations; the table is sixteen doubles in shared
+// memory = all 32 banks once, so lanes with different n never conflict.  The sweeps in double precision evaluate
+// little else: the library's exp takes 58 issue cycles per warp on this GPU, a double fma 2.  The exponent saturates
+// (below 2^-1022; above 2^1024 as a NaN, never a finite value); no branch, which would keep the exponentials of a
+// pair's channels from overlapping.
+__device__ const double EXP16_TABLE[16] = {
+    1.0,                1.0442737824274138, 1.0905077326652577, 1.1387886347566916, 1.189207115002721,  1.241857812073484,
+    1.2968395546510096, 1.3542555469368927, 1.4142135623730951, 1.4768261459394993, 1.5422108254079407, 1.6104903319492543,
+    1.681792830507429,  1.7562521603732995, 1.8340080864093424, 1.9152065613971474};
+__device__ __forceinline__ double exp_table16(double x, const double* tab) {
+  const double magic = 6755399441055744.0;  // 1.5 * 2^52: the integer lands in the low word
+  const double t = fma(x, 23.083120654223414, magic);
+  const int n = __double2loint(t);
+  const double nf = t - magic;
+  double r = fma(nf, -0.043321698780346196, x);  // ln2/16 with 33 bits: exact products
+  r = fma(nf, -4.650385693757748e-12, r);
+  double q = fma(0.0013889034348599464, r, 0.008333449701253456);
+  q = fma(q, r, 0.04166666666496045);
+  q = fma(q, r, 0.1666666666530169);
+  q = fma(q, r, 0.5);
+  const double T0 = tab[n & 15];
+  const double e = fma(T0, fma(r * r, q, r), T0);
+  const int k = max(-1022, min(n >> 4, 1024));
+  return __hiloint2double(__double2hiint(e) + (k << 20), __double2loint(e));
+}
+
+// exponential of a pre-scaled argument; et: the 16-entry table in shared memory (double only)
 template <class T> struct Ex;
 template <> struct Ex<float> {
   static __host__ __device__ __forceinline__ float scale() { return 1.4426950408889634f; }
-  static __device__ __forceinline__ float f(float x) { return ex2_fast(x); }
+  static __device__ __forceinline__ float f(float x, const float*) { return ex2_fast(x); }
 };
 template <> struct Ex<double> {
   static __host__ __device__ __forceinline__ double scale() { return 1.0; }
-  static __device__ __forceinline__ double f(double x) { return exp(x); }
+  static __device__ __forceinline__ double f(double x, const double* et) { return exp_table16(x, et); }
 };
 
 // Two-channel packed arithmetic.  On sm_100 a float2 multiply / add / fma is ONE instruction (__fmul2_rn,
 // __fadd2_rn, __ffma2_rn), so the channel loops carry two channels per instruction; double pairs are two scalar
-// operations.
-__device__ __forceinline__ float2 p_mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 p_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 p_fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ double2 p_mul(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
-__device__ __forceinline__ double2 p_add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 p_fma(double2 a, double2 b, double2 c) {
-  return make_double2(a.x * b.x + c.x, a.y * b.y + c.y);
+// operations.  `one`: only the first channel of the pair exists (double; an odd channel count would otherwise cost
+// the exponentials of a channel that contributes nothing - in fp32 the padding channel rides along in the packed
+// instruction).  It is a compile-time constant once the channel loops are unrolled.
+__device__ __forceinline__ float2 p_mul(float2 a, float2 b, bool = false) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 p_add(float2 a, float2 b, bool = false) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 p_fma(float2 a, float2 b, float2 c, bool = false) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ double2 p_mul(double2 a, double2 b, bool one = false) {
+  return make_double2(a.x * b.x, one ? 0.0 : a.y * b.y);
+}
+__device__ __forceinline__ double2 p_add(double2 a, double2 b, bool one = false) {
+  return make_double2(a.x + b.x, one ? 0.0 : a.y + b.y);
+}
+__device__ __forceinline__ double2 p_fma(double2 a, double2 b, double2 c, bool one = false) {
+  return make_double2(a.x * b.x + c.x, one ? c.y : a.y * b.y + c.y);
 }
 __device__ __forceinline__ float2 mk2(float x, float y) { return make_float2(x, y); }
 __device__ __forceinline__ double2 mk2(double x, double y) { return make_double2(x, y); }
-__device__ __forceinline__ float2 p_ex(float2 a) { return make_float2(Ex<float>::f(a.x), Ex<float>::f(a.y)); }
-__device__ __forceinline__ double2 p_ex(double2 a) { return make_double2(Ex<double>::f(a.x), Ex<double>::f(a.y)); }
+__device__ __forceinline__ float2 p_ex(float2 a, const float* et, bool = false) {
+  return make_float2(Ex<float>::f(a.x, et), Ex<float>::f(a.y, et));
+}
+__device__ __forceinline__ double2 p_ex(double2 a, const double* et, bool one = false) {
+  return make_double2(Ex<double>::f(a.x, et), one ? 0.0 : Ex<double>::f(a.y, et));
+}
 
 // AFV = fingerprints that also leave d(AF)/d(alpha) per atom (training)
 enum { MODE_AF = 0, MODE_FORCE = 1, MODE_FGRAD = 2, MODE_AFV = 4 };
@@ -218,7 +257,7 @@ struct SweepArgs {
 
 // shared-memory layout of a sweep block (byte offsets)
 struct SweepSmem {
-  int row, spar, tab, xtra, acc, rsum, wch, red, mbar, total;
+  int row, spar, tab, xtra, acc, rsum, wch, red, etab, mbar, total;
 };
 template <class T>
 static inline SweepSmem sweep_smem(const ModelDev& d, const SparLayout& sl, int nr, int mode) {
@@ -234,6 +273,7 @@ static inline SweepSmem sweep_smem(const ModelDev& d, const SparLayout& sl, int 
   L.rsum = take(d.nt * (d.Frmax > 0 ? d.Frmax : 1) * es);
   L.wch = take(mode == MODE_FORCE ? d.ncls * sl.maxp * 2 * es : 0);
   L.red = take(32 * es);  // group offsets
+  L.etab = take(es == 8 ? 16 * es : 0);  // table of the double exponential
   L.mbar = take(16);
   L.total = o;
   return L;
@@ -300,13 +340,14 @@ struct PairWalk {
 
 // ---- unordered pairs: fingerprints (AF), fingerprints + d(AF)/d(alpha) (AFV), backward of the forces (FGRAD).
 // Per-lane sums r[v][lp] (v = 0: fingerprint / gradnet, 1..3: alpha1, alpha2, beta terms) for NCHP channel pairs.
-template <class T, int MODE, int NCHP, bool SAME>
+template <class T, int MODE, int NCH, bool SAME, int NCHP = (NCH + 1) / 2>
 __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __restrict__ U,
                                                 const typename Vec4<T>::type* __restrict__ V,
                                                 const typename Vec4<T>::type* __restrict__ dF,
                                                 const typename Vec4<T>::type* __restrict__ tab4, int nr,
                                                 const typename Vec4<T>::type* __restrict__ chq,
-                                                const typename Vec4<T>::type* __restrict__ chr, int oa, int ob,
+                                                const typename Vec4<T>::type* __restrict__ chr, const T* __restrict__ et,
+                                                int oa, int ob,
                                                 int na_, int nb_, int lane,
                                                 typename Vec2<T>::type (&r0)[NCHP], typename Vec2<T>::type (&r1)[NCHP],
                                                 typename Vec2<T>::type (&r2)[NCHP],
@@ -316,6 +357,7 @@ __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __
 #pragma unroll
   for (int lp = 0; lp < NCHP; lp++) r0[lp] = r1[lp] = r2[lp] = r3[lp] = mk2(T(0), T(0));
   const T2 one2 = mk2(T(1), T(1));
+  constexpr bool ODD = sizeof(T) == 8 && (NCH & 1);
   const int np = PairWalk<SAME>::count(na_, nb_);
   PairWalk<SAME> pw;
   pw.init(na_, nb_, lane);
@@ -343,16 +385,17 @@ __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __
     if (MODE != MODE_FGRAD) {
 #pragma unroll
       for (int lp = 0; lp < NCHP; lp++) {
+        const bool h = ODD && lp == NCHP - 1;
         const T4 A = tab4[j * TSTR + lp], B = tab4[k * TSTR + lp];
-        const T2 S1 = p_mul(mk2(A.z, A.w), mk2(B.x, B.y));  // exp(a2*sj + a1*sk)
-        const T2 S2 = p_mul(mk2(A.x, A.y), mk2(B.z, B.w));  // exp(a1*sj + a2*sk)
-        const T2 cm = p_mul(p_ex(p_mul(bsc[lp], tt2)), tt2);  // t*exp(beta*t)
-        const T2 ss = p_add(S1, S2);
-        r0[lp] = p_fma(cm, ss, r0[lp]);  // the channel coefficient is applied after the reduction
+        const T2 S1 = p_mul(mk2(A.z, A.w), mk2(B.x, B.y), h);  // exp(a2*sj + a1*sk)
+        const T2 S2 = p_mul(mk2(A.x, A.y), mk2(B.z, B.w), h);  // exp(a1*sj + a2*sk)
+        const T2 cm = p_mul(p_ex(p_mul(bsc[lp], tt2, h), et, h), tt2, h);  // t*exp(beta*t)
+        const T2 ss = p_add(S1, S2, h);
+        r0[lp] = p_fma(cm, ss, r0[lp], h);  // the channel coefficient is applied after the reduction
         if (MODE == MODE_AFV) {
-          r1[lp] = p_fma(cm, p_fma(S2, fcj2, p_mul(S1, fck2)), r1[lp]);
-          r2[lp] = p_fma(cm, p_fma(S2, fck2, p_mul(S1, fcj2)), r2[lp]);
-          r3[lp] = p_fma(p_mul(cm, tt2), ss, r3[lp]);
+          r1[lp] = p_fma(cm, p_fma(S2, fcj2, p_mul(S1, fck2, h), h), r1[lp], h);
+          r2[lp] = p_fma(cm, p_fma(S2, fck2, p_mul(S1, fcj2, h), h), r2[lp], h);
+          r3[lp] = p_fma(p_mul(cm, tt2, h), ss, r3[lp], h);
         }
       }
     } else {
@@ -378,17 +421,18 @@ __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __
       const T2 Qh2 = mk2(Qh, Qh), Pj2 = mk2(Pjh, Pjh), Pk2 = mk2(Pkh, Pkh);
 #pragma unroll
       for (int lp = 0; lp < NCHP; lp++) {
+        const bool h = ODD && lp == NCHP - 1;
         const T4 A = tab4[j * TSTR + lp], B = tab4[k * TSTR + lp], cq = chq[lp], cr = chr[lp];
         const T2 al1 = mk2(cq.x, cq.y), al2 = mk2(cq.z, cq.w);
-        const T2 E = p_ex(p_mul(mk2(cr.z, cr.w), tt2));
-        const T2 Z1 = p_mul(E, p_mul(mk2(A.x, A.y), mk2(B.z, B.w)));
-        const T2 Z2 = p_mul(E, p_mul(mk2(A.z, A.w), mk2(B.x, B.y)));
-        const T2 gQ = p_mul(p_fma(mk2(cr.x, cr.y), tt2, one2), Qh2);
-        const T2 H1 = p_fma(al1, Pj2, p_fma(al2, Pk2, gQ)), H2 = p_fma(al1, Pk2, p_fma(al2, Pj2, gQ));
-        r0[lp] = p_fma(Z1, H1, p_fma(Z2, H2, r0[lp]));
-        r1[lp] = p_fma(Z1, p_fma(fcj2, H1, Pj2), p_fma(Z2, p_fma(fck2, H2, Pk2), r1[lp]));
-        r2[lp] = p_fma(Z1, p_fma(fck2, H1, Pk2), p_fma(Z2, p_fma(fcj2, H2, Pj2), r2[lp]));
-        r3[lp] = p_fma(tt2, p_fma(Z1, p_add(H1, Qh2), p_mul(Z2, p_add(H2, Qh2))), r3[lp]);
+        const T2 E = p_ex(p_mul(mk2(cr.z, cr.w), tt2, h), et, h);
+        const T2 Z1 = p_mul(E, p_mul(mk2(A.x, A.y), mk2(B.z, B.w), h), h);
+        const T2 Z2 = p_mul(E, p_mul(mk2(A.z, A.w), mk2(B.x, B.y), h), h);
+        const T2 gQ = p_mul(p_fma(mk2(cr.x, cr.y), tt2, one2, h), Qh2, h);
+        const T2 H1 = p_fma(al1, Pj2, p_fma(al2, Pk2, gQ, h), h), H2 = p_fma(al1, Pk2, p_fma(al2, Pj2, gQ, h), h);
+        r0[lp] = p_fma(Z1, H1, p_fma(Z2, H2, r0[lp], h), h);
+        r1[lp] = p_fma(Z1, p_fma(fcj2, H1, Pj2, h), p_fma(Z2, p_fma(fck2, H2, Pk2, h), r1[lp], h), h);
+        r2[lp] = p_fma(Z1, p_fma(fck2, H1, Pk2, h), p_fma(Z2, p_fma(fcj2, H2, Pj2, h), r2[lp], h), h);
+        r3[lp] = p_fma(tt2, p_fma(Z1, p_add(H1, Qh2, h), p_mul(Z2, p_add(H2, Qh2, h), h), h), r3[lp], h);
       }
     }
   }
@@ -399,13 +443,14 @@ __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __
 // channel weights - and its force accumulator stay in registers for the whole segment, all lanes run the same
 // number of iterations, and the accumulators are flushed once per round (S lanes share an owner).  S in 1..4 is
 // chosen per class to fill the 32 lanes.  fo[k*3 + a]: force on neighbour k; (fix, fiy, fiz): on the centre.
-template <class T, int NCHP, bool SAME>
+template <class T, int NCH, bool SAME, int NCHP = (NCH + 1) / 2>
 __device__ __forceinline__ void pairs_force(const typename Vec4<T>::type* __restrict__ U,
                                             const typename Vec4<T>::type* __restrict__ V,
                                             const typename Vec4<T>::type* __restrict__ tab4,
                                             const typename Vec4<T>::type* __restrict__ chq,
                                             const typename Vec4<T>::type* __restrict__ chr,
-                                            const typename Vec2<T>::type* __restrict__ wch, int oo, int op, int no,
+                                            const typename Vec2<T>::type* __restrict__ wch, const T* __restrict__ et,
+                                            int oo, int op, int no,
                                             int npt, int lane, T* __restrict__ fo, T& fix, T& fiy, T& fiz) {
   typedef typename Vec4<T>::type T4;
   typedef typename Vec2<T>::type T2;
@@ -418,6 +463,7 @@ __device__ __forceinline__ void pairs_force(const typename Vec4<T>::type* __rest
     if (cost < best) { best = cost; S = s; seg = sg; }
   }
   constexpr int FORCE_UNROLL = sizeof(T) == 4 ? 2 : 1;  // two partners in flight where the registers allow it
+  constexpr bool ODD = sizeof(T) == 8 && (NCH & 1);
   const int nseg = no * S;
   const T2 one2 = mk2(T(1), T(1));
   for (int base = 0; base < nseg; base += 32) {
@@ -456,10 +502,11 @@ __device__ __forceinline__ void pairs_force(const typename Vec4<T>::type* __rest
         for (int lp = 0; lp < NCHP; lp++) {
           const T4 B = tab4[k * TSTR + lp], cr = chr[lp];
           const T2 A1k = mk2(B.x, B.y), A2k = mk2(B.z, B.w);
-          const T2 Ex2 = p_ex(p_mul(mk2(cr.z, cr.w), tt2));
-          const T2 sum = p_fma(a1w[lp], A2k, p_mul(a2w[lp], A1k));            // w (S2 + S1)
-          D2 = p_fma(p_mul(p_fma(mk2(cr.x, cr.y), tt2, one2), Ex2), sum, D2);  // w e^{bt} (1 + bt) (S1 + S2)
-          BJ2 = p_fma(Ex2, p_fma(b1w[lp], A2k, p_mul(b2w[lp], A1k)), BJ2);     // w e^{bt} (a1 S2 + a2 S1)
+          const bool h = ODD && lp == NCHP - 1;
+          const T2 Ex2 = p_ex(p_mul(mk2(cr.z, cr.w), tt2, h), et, h);
+          const T2 sum = p_fma(a1w[lp], A2k, p_mul(a2w[lp], A1k, h), h);                // w (S2 + S1)
+          D2 = p_fma(p_mul(p_fma(mk2(cr.x, cr.y), tt2, one2, h), Ex2, h), sum, D2, h);  // w e^{bt} (1 + bt) (S1 + S2)
+          BJ2 = p_fma(Ex2, p_fma(b1w[lp], A2k, p_mul(b2w[lp], A1k, h), h), BJ2, h);     // w e^{bt} (a1 S2 + a2 S1)
         }
         const T D = D2.x + D2.y, BJ = (BJ2.x + BJ2.y) * tt;
         // f_ij = cjk*u_k + (...)*u_j
@@ -474,6 +521,31 @@ __device__ __forceinline__ void pairs_force(const typename Vec4<T>::type* __rest
       atomicAdd(&fo[j * 3 + 1], fy);
       atomicAdd(&fo[j * 3 + 2], fz);
       fix -= fx; fiy -= fy; fiz -= fz;
+    }
+  }
+}
+
+// Calls fn with the number of channels of this pass as a compile-time constant: every number in double precision,
+// the next even one in fp32 (pairs of channels, the last one padded).
+template <class T, class Fn>
+__device__ __forceinline__ void by_channels(int nch, Fn&& fn) {
+  if constexpr (sizeof(T) == 8) {
+    switch (nch) {
+      case 1: fn(std::integral_constant<int, 1>()); break;
+      case 2: fn(std::integral_constant<int, 2>()); break;
+      case 3: fn(std::integral_constant<int, 3>()); break;
+      case 4: fn(std::integral_constant<int, 4>()); break;
+      case 5: fn(std::integral_constant<int, 5>()); break;
+      case 6: fn(std::integral_constant<int, 6>()); break;
+      case 7: fn(std::integral_constant<int, 7>()); break;
+      default: fn(std::integral_constant<int, 8>()); break;
+    }
+  } else {
+    switch ((nch + 1) >> 1) {
+      case 1: fn(std::integral_constant<int, 2>()); break;
+      case 2: fn(std::integral_constant<int, 4>()); break;
+      case 3: fn(std::integral_constant<int, 6>()); break;
+      default: fn(std::integral_constant<int, 8>()); break;
     }
   }
 }
@@ -513,6 +585,7 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
   T* rsum = reinterpret_cast<T*>(smem_raw + L.rsum);
   T2* wch_all = reinterpret_cast<T2*>(smem_raw + L.wch);
   int* off = reinterpret_cast<int*>(smem_raw + L.red);  // [STAFB_MAX_TYPES + 1]
+  T* et = reinterpret_cast<T*>(smem_raw + L.etab);
   const unsigned bar = smem_addr(smem_raw + L.mbar);
   // accumulator regions: the first nv entries are the d(AF)/d(alpha) row of the AFV mode
   const int ACC_A2 = 0;                      // [nt*Frmax]  alpha2b terms
@@ -534,6 +607,7 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
   }
   if (MODE != MODE_FORCE)
     for (int q = lane; q < NACC; q += 32) acc[q] = T(0);
+  if (ES == 8 && lane < 16) et[lane] = (T)EXP16_TABLE[lane];
   chain_wait();
   if (IS_AF && lane == 0) {
     mbar_expect_tx(bar, (unsigned)sl.total);
@@ -641,7 +715,7 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
         for (int c = 0; c < Fr; c++) {
           const T4 rp = rpar[tk * Frmax + c];
           if (rp.z == T(0)) continue;
-          w += chrow[c] * (T(0.5) * rp.z * Ex<T>::f(rp.x * dk) * (T(1) + rp.y * dk));
+          w += chrow[c] * (T(0.5) * rp.z * Ex<T>::f(rp.x * dk, et) * (T(1) + rp.y * dk));
         }
         const T g = w * v.w;
         gx = g * u.x; gy = g * u.y; gz = g * u.z;
@@ -668,7 +742,7 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
           for (int r = r0_; r < r1_; r++) {
             const T4 v = V[r];
             const T dk = v.z;
-            const T ex = Ex<T>::f(als * dk);
+            const T ex = Ex<T>::f(als * dk, et);
             if (MODE == MODE_FGRAD) {
               const T qq = T(0.5) * v.w * dF[r].w;
               gn += qq * ex * (T(1) + al * dk);
@@ -706,6 +780,7 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
       const int npair = (nact + 1) >> 1;
       for (int p0 = 0; p0 < npair; p0 += MAXP) {
         const int nchp = (npair - p0) < MAXP ? (npair - p0) : MAXP;
+        const int nch = sizeof(T) == 4 ? 2 * nchp : ((nact - 2 * p0) < 2 * MAXP ? (nact - 2 * p0) : 2 * MAXP);
         const T4* chq = chq_all + s * sl.maxp + p0;
         const T4* chr = chr_all + s * sl.maxp + p0;
         // tables exp(a1*fc_k), exp(a2*fc_k) of the neighbours of the two species, all channel pairs of a
@@ -719,7 +794,7 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
           for (int lp = 0; lp < MAXP; lp++) {
             if (lp < nchp) {
               const T4 q = chq[lp];
-              const T2 e1 = p_ex(p_mul(mk2(q.x, q.y), f2)), e2 = p_ex(p_mul(mk2(q.z, q.w), f2));
+              const T2 e1 = p_ex(p_mul(mk2(q.x, q.y), f2), et), e2 = p_ex(p_mul(mk2(q.z, q.w), f2), et);
               T4 v;
               v.x = e1.x; v.y = e1.y; v.z = e2.x; v.w = e2.y;
               tab4[k * TSTR + lp] = v;
@@ -735,16 +810,13 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
             const int no = pass == 0 ? na_ : nb_;
             const int npt = same ? na_ - 1 : (pass == 0 ? nb_ : na_);
             auto go = [&](auto tag) {
-              constexpr int NCHP = decltype(tag)::value;
-              if (same) pairs_force<T, NCHP, true>(U, V, tab4, chq, chr, wch, oo, op, no, npt, lane, xtra, fix, fiy, fiz);
-              else pairs_force<T, NCHP, false>(U, V, tab4, chq, chr, wch, oo, op, no, npt, lane, xtra, fix, fiy, fiz);
+              constexpr int NCH = decltype(tag)::value;
+              if (same)
+                pairs_force<T, NCH, true>(U, V, tab4, chq, chr, wch, et, oo, op, no, npt, lane, xtra, fix, fiy, fiz);
+              else
+                pairs_force<T, NCH, false>(U, V, tab4, chq, chr, wch, et, oo, op, no, npt, lane, xtra, fix, fiy, fiz);
             };
-            switch (nchp) {
-              case 1: go(std::integral_constant<int, 1>()); break;
-              case 2: go(std::integral_constant<int, 2>()); break;
-              case 3: go(std::integral_constant<int, 3>()); break;
-              default: go(std::integral_constant<int, 4>()); break;
-            }
+            by_channels<T>(nch, go);
           }
         } else {
           // per-lane sums, then the transposing butterfly: lane L ends up with the total of value index L (or
@@ -754,11 +826,13 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
           const T4* dF = reinterpret_cast<const T4*>(xtra);
           T tot = T(0);
           int vidx = -1;  // value index this lane holds after the reduction (-1: none)
-          auto run = [&](auto nchp_tag) {
-            constexpr int NCHP = decltype(nchp_tag)::value;
+          auto run = [&](auto nch_tag) {
+            constexpr int NCH = decltype(nch_tag)::value, NCHP = (NCH + 1) / 2;
             T2 r0[NCHP], r1[NCHP], r2[NCHP], r3[NCHP];
-            if (same) pairs_unordered<T, MODE, NCHP, true>(U, V, dF, tab4, nr, chq, chr, oa, ob, na_, nb_, lane, r0, r1, r2, r3);
-            else pairs_unordered<T, MODE, NCHP, false>(U, V, dF, tab4, nr, chq, chr, oa, ob, na_, nb_, lane, r0, r1, r2, r3);
+            if (same)
+              pairs_unordered<T, MODE, NCH, true>(U, V, dF, tab4, nr, chq, chr, et, oa, ob, na_, nb_, lane, r0, r1, r2, r3);
+            else
+              pairs_unordered<T, MODE, NCH, false>(U, V, dF, tab4, nr, chq, chr, et, oa, ob, na_, nb_, lane, r0, r1, r2, r3);
             if (MODE == MODE_AF) {
               constexpr int NV = NCHP == 1 ? 2 : (NCHP == 2 ? 4 : 8);
               T v[NV];
@@ -785,12 +859,7 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
               vidx = ((lane & ((1 << SH) - 1)) == 0) ? (lane >> SH) : -1;
             }
           };
-          switch (nchp) {
-            case 1: run(std::integral_constant<int, 1>()); break;
-            case 2: run(std::integral_constant<int, 2>()); break;
-            case 3: run(std::integral_constant<int, 3>()); break;
-            default: run(std::integral_constant<int, 4>()); break;
-          }
+          by_channels<T>(nch, run);
           if (vidx >= 0) {
             const int lp = vidx >> 3, h = (vidx >> 2) & 1, v = vidx & 3;
             const int slot = 2 * (p0 + lp) + h;

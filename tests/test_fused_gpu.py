@@ -266,6 +266,25 @@ def test_train_step_losses_and_gradient(oracle, frame0, name, seeds, loss, dtype
     m.close()
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("channels", [(1, 2, 3), (4, 6, 7), (8, 9, 0)])
+def test_train_step_with_other_channel_counts(oracle, frame0, channels, dtype):
+    """Every number of active channels per species-pair class that a pass of the sweeps takes (1 to 8; 9: a second
+    pass of one channel; 0: an empty class)."""
+    from alphanesgpu_b200 import train as T
+    from alphanesgpu_b200.model import StafModel
+    from alphanesgpu_b200.params import ModelShape
+    pos, box, tipos = synth.water_frames("water96", [1000, 1001])
+    maps = dict(map_rad_afs={0: [3, 2], 1: [1, 4]}, map_ang_afs={0: list(channels), 1: list(channels[::-1])})
+    shape = ModelShape(nt=2, tipos=list(tipos), Fr=[5, 5], Fa=[sum(channels)] * 2, widths=[16, 1])
+    theta, emb = T.init_params(shape, maps, 3)
+    el, fl = synth.labels(2, shape.N)
+    kw = dict(pe=0.7, pf=1.3, pb=0.9, alpha_bound=5.0)
+    m = StafModel(shape, CFG, theta, emb, 2, dtype=_tdt(dtype), loss="huber", **kw)
+    _check_train_step(oracle, m, shape, pos, box, el, fl, theta, emb, dtype, "huber", kw, host_path=False)
+    m.close()
+
+
 def test_adam_matches_reference_formula():
     from alphanesgpu_b200.model import StafModel
     pos, box, tipos = synth.water_frames("water96", [1000])
