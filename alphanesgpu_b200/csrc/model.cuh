@@ -167,6 +167,14 @@ static inline int device_slot() {
   return (d >= 0 && d < MAX_DEVICES) ? d : 0;
 }
 
+// multiprocessors of the current device
+static inline int sm_count() {
+  int d = 0, n = 148;
+  cudaGetDevice(&d);
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, d);
+  return n;
+}
+
 // what a sweep launch needs besides the model: the records of this evaluation and the per-call buffers
 template <class T>
 struct SweepCall {

@@ -257,10 +257,10 @@ struct SweepArgs {
 
 // shared-memory layout of a sweep block (byte offsets)
 struct SweepSmem {
-  int row, spar, tab, xtra, acc, rsum, wch, red, etab, mbar, total;
+  int row, spar, tab, xtra, part, acc, rsum, wch, red, etab, mbar, total;
 };
 template <class T>
-static inline SweepSmem sweep_smem(const ModelDev& d, const SparLayout& sl, int nr, int mode) {
+static inline SweepSmem sweep_smem(const ModelDev& d, const SparLayout& sl, int nr, int mode, int nw) {
   SweepSmem L;
   int o = 0;
   auto take = [&](int bytes) { int r = o; o += (bytes + 15) & ~15; return r; };
@@ -269,7 +269,8 @@ static inline SweepSmem sweep_smem(const ModelDev& d, const SparLayout& sl, int 
   L.spar = take(sl.total);
   L.tab = take(TSTR * nr * 4 * es);
   L.xtra = take(mode == MODE_FORCE ? 3 * nr * es : (mode == MODE_FGRAD ? 4 * nr * es : 0));
-  L.acc = take((d.nt * d.Frmax + d.C * 3 * d.Famax + d.Famax) * es);
+  L.part = take(mode == MODE_FORCE && nw > 1 ? 3 * 32 * nw * es : 0);  // forces of the segments of an owner
+  L.acc = take(mode == MODE_FORCE ? 0 : (d.nt * d.Frmax + d.C * 3 * d.Famax + d.Famax) * es);
   L.rsum = take(d.nt * (d.Frmax > 0 ? d.Frmax : 1) * es);
   L.wch = take(mode == MODE_FORCE ? d.ncls * sl.maxp * 2 * es : 0);
   L.red = take(32 * es);  // group offsets
@@ -277,6 +278,16 @@ static inline SweepSmem sweep_smem(const ModelDev& d, const SparLayout& sl, int 
   L.mbar = take(16);
   L.total = o;
   return L;
+}
+
+// Barrier over the NW warps of a block, and an addition into shared memory that only one lane per warp makes.
+template <int NW>
+__device__ __forceinline__ void block_sync() {
+  if (NW == 1) __syncwarp(); else __syncthreads();
+}
+template <int NW, class T>
+__device__ __forceinline__ void acc_add(T* p, T v) {
+  if (NW == 1) *p += v; else atomicAdd(p, v);
 }
 
 // Sums NV per-lane values over the 32 lanes of a warp.  Every step halves the number of values a lane
@@ -303,13 +314,13 @@ __device__ __forceinline__ T multi_reduce(T (&v)[NV], int lane) {
   return r;
 }
 
-// Pairs of a class as a rectangle of rows x cols walked 32 positions at a time without divisions.  Two different
+// Pairs of a class as a rectangle of rows x cols walked LANES positions at a time without divisions.  Two different
 // species (SAME == false): rows = neighbours of ta, cols = neighbours of tb.  One species with n neighbours: the
 // strict upper triangle j < k folded into a rectangle - row r of the triangle (n-1-r entries) is followed by row
 // n-1-r (n even) or n-2-r (n odd), which together have n-1 (n) entries.
-template <bool SAME>
+template <bool SAME, int LANES>
 struct PairWalk {
-  int r, c, cols, q32, r32, nm1, odd;
+  int r, c, cols, qs, rs, nm1, odd;
   __device__ __forceinline__ void init(int na, int nb, int lane) {
     odd = na & 1;
     nm1 = na - 1;
@@ -317,8 +328,8 @@ struct PairWalk {
     if (cols < 1) cols = 1;
     r = lane / cols;
     c = lane - r * cols;
-    q32 = 32 / cols;
-    r32 = 32 - q32 * cols;
+    qs = LANES / cols;
+    rs = LANES - qs * cols;
   }
   __device__ __forceinline__ static int count(int na, int nb) { return SAME ? na * (na - 1) / 2 : na * nb; }
   __device__ __forceinline__ void get(int& j, int& k) const {
@@ -332,15 +343,15 @@ struct PairWalk {
     }
   }
   __device__ __forceinline__ void step() {
-    r += q32;
-    c += r32;
+    r += qs;
+    c += rs;
     if (c >= cols) { c -= cols; r++; }
   }
 };
 
 // ---- unordered pairs: fingerprints (AF), fingerprints + d(AF)/d(alpha) (AFV), backward of the forces (FGRAD).
 // Per-lane sums r[v][lp] (v = 0: fingerprint / gradnet, 1..3: alpha1, alpha2, beta terms) for NCHP channel pairs.
-template <class T, int MODE, int NCH, bool SAME, int NCHP = (NCH + 1) / 2>
+template <class T, int MODE, int NCH, bool SAME, int NW, int NCHP = (NCH + 1) / 2>
 __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __restrict__ U,
                                                 const typename Vec4<T>::type* __restrict__ V,
                                                 const typename Vec4<T>::type* __restrict__ dF,
@@ -358,8 +369,8 @@ __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __
   for (int lp = 0; lp < NCHP; lp++) r0[lp] = r1[lp] = r2[lp] = r3[lp] = mk2(T(0), T(0));
   const T2 one2 = mk2(T(1), T(1));
   constexpr bool ODD = sizeof(T) == 8 && (NCH & 1);
-  const int np = PairWalk<SAME>::count(na_, nb_);
-  PairWalk<SAME> pw;
+  const int np = PairWalk<SAME, 32 * NW>::count(na_, nb_);
+  PairWalk<SAME, 32 * NW> pw;
   pw.init(na_, nb_, lane);
   // beta*log2(e) of every channel pair stays in registers in the fingerprint modes
   T2 bsc[NCHP];
@@ -371,7 +382,7 @@ __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __
   // force-backward loop is too large for that (its unrolled body falls out of the instruction cache)
   constexpr int PAIR_UNROLL = (MODE == MODE_FGRAD) ? 1 : 2;
 #pragma unroll PAIR_UNROLL
-  for (int p = lane; p < np; p += 32) {
+  for (int p = lane; p < np; p += 32 * NW) {
     int jj, kk;
     pw.get(jj, kk);
     pw.step();
@@ -443,33 +454,37 @@ __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __
 // channel weights - and its force accumulator stay in registers for the whole segment, all lanes run the same
 // number of iterations, and the accumulators are flushed once per round (S lanes share an owner).  S in 1..4 is
 // chosen per class to fill the 32 lanes.  fo[k*3 + a]: force on neighbour k; (fix, fiy, fiz): on the centre.
-template <class T, int NCH, bool SAME, int NCHP = (NCH + 1) / 2>
+template <class T, int NCH, bool SAME, int NW, int NCHP = (NCH + 1) / 2>
 __device__ __forceinline__ void pairs_force(const typename Vec4<T>::type* __restrict__ U,
                                             const typename Vec4<T>::type* __restrict__ V,
                                             const typename Vec4<T>::type* __restrict__ tab4,
                                             const typename Vec4<T>::type* __restrict__ chq,
                                             const typename Vec4<T>::type* __restrict__ chr,
                                             const typename Vec2<T>::type* __restrict__ wch, const T* __restrict__ et,
-                                            int oo, int op, int no,
-                                            int npt, int lane, T* __restrict__ fo, T& fix, T& fiy, T& fiz) {
+                                            int oo, int op, int no, int npt, int lane, T* __restrict__ fo,
+                                            T* __restrict__ part, T& fix, T& fiy, T& fiz) {
   typedef typename Vec4<T>::type T4;
   typedef typename Vec2<T>::type T2;
   if (no <= 0 || npt <= 0) return;
   // segments per owner: fewest (iterations + 2) * rounds; the 2 stands for loading the owner and flushing
   int S = 1, seg = npt, best = 0x7fffffff;
 #pragma unroll
-  for (int s = 1; s <= 4; s++) {
-    const int sg = (npt + s - 1) / s, rounds = (no * s + 31) >> 5, cost = rounds * (sg + 2);
+  for (int s = 1; s <= (NW == 1 ? 4 : 16); s++) {
+    const int sg = (npt + s - 1) / s, rounds = (no * s + 32 * NW - 1) / (32 * NW), cost = rounds * (sg + 2);
     if (cost < best) { best = cost; S = s; seg = sg; }
   }
   constexpr int FORCE_UNROLL = sizeof(T) == 4 ? 2 : 1;  // two partners in flight where the registers allow it
   constexpr bool ODD = sizeof(T) == 8 && (NCH & 1);
   const int nseg = no * S;
   const T2 one2 = mk2(T(1), T(1));
-  for (int base = 0; base < nseg; base += 32) {
+  for (int base = 0; base < nseg; base += 32 * NW) {
     const int sidx = base + lane;
     const bool active = sidx < nseg;
-    const int ow = active ? ((S == 1) ? sidx : (S == 2) ? (sidx >> 1) : (S == 4) ? (sidx >> 2) : (sidx * 21846) >> 16) : 0;
+    int ow = 0;  // sidx / S (the reciprocal is exact for these ranges)
+    if (active) {
+      if (NW == 1) ow = (S == 1) ? sidx : (S == 2) ? (sidx >> 1) : (S == 4) ? (sidx >> 2) : (sidx * 21846) >> 16;
+      else ow = (sidx * ((65535 + S) / S)) >> 16;
+    }
     const int k0 = (sidx - ow * S) * seg;
     const int j = oo + ow;
     const T4 uj = U[j];
@@ -515,12 +530,31 @@ __device__ __forceinline__ void pairs_force(const typename Vec4<T>::type* __rest
         as += -cs * cjk + gfcj * (D * half * uk.w + BJ);
       }
     }
-    if (active) {
+    if (NW == 1) {
+      if (active) {
+        const T fx = ax + as * uj.x, fy = ay + as * uj.y, fz = az + as * uj.z;
+        atomicAdd(&fo[j * 3 + 0], fx);
+        atomicAdd(&fo[j * 3 + 1], fy);
+        atomicAdd(&fo[j * 3 + 2], fz);
+        fix -= fx; fiy -= fy; fiz -= fz;
+      }
+    } else {
       const T fx = ax + as * uj.x, fy = ay + as * uj.y, fz = az + as * uj.z;
-      atomicAdd(&fo[j * 3 + 0], fx);
-      atomicAdd(&fo[j * 3 + 1], fy);
-      atomicAdd(&fo[j * 3 + 2], fz);
-      fix -= fx; fiy -= fy; fiz -= fz;
+      if (active) { fix -= fx; fiy -= fy; fiz -= fz; }
+      // the segments of an owner lie on consecutive lanes: one thread per (owner, component) adds them up.  (A shared
+      // float atomic is a compare-and-swap loop: S lanes on one word cost S round trips, most of this function's time
+      // when four warps share an atom and S goes up to 16.  One warp, S <= 4, keeps the atomics: this form costs it
+      // registers, 5 % of a force sweep.)
+      part[lane * 3] = fx; part[lane * 3 + 1] = fy; part[lane * 3 + 2] = fz;
+      block_sync<NW>();
+      const int o0 = base / S, last = min(nseg - base, 32 * NW), cnt = (base + last - 1) / S + 1 - o0;
+      for (int q = lane; q < 3 * cnt; q += 32 * NW) {
+        const int o = o0 + q / 3, c = q % 3, l1 = min((o + 1) * S - base, last);
+        T f = T(0);
+        for (int l = max(o * S - base, 0); l < l1; l++) f += part[l * 3 + c];
+        fo[(oo + o) * 3 + c] += f;
+      }
+      block_sync<NW>();
     }
   }
 }
@@ -550,17 +584,18 @@ __device__ __forceinline__ void by_channels(int nch, Fn&& fn) {
   }
 }
 
-// One block of one warp per central atom.  VIR (force mode only) adds the virial; it is a template parameter so
+// One block of NW warps per central atom.  VIR (force mode only) adds the virial; it is a template parameter so
 // that the training step's force sweep does not carry its registers.
-template <class T, int MODE, bool VIR>
-__global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
+template <class T, int MODE, bool VIR, int NW>
+__global__ void __launch_bounds__(32 * NW, (SweepMinBlocks<MODE, sizeof(T)>::value + NW - 1) / NW)
     k_sweep(ModelDev md, SweepArgs<T> a, SweepSmem L) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   typedef typename Vec4<T>::type T4;
   typedef typename Vec2<T>::type T2;
   constexpr bool IS_AF = (MODE == MODE_AF || MODE == MODE_AFV);
   constexpr int ES = (int)sizeof(T);
-  const int lane = threadIdx.x;
+  constexpr int LANES = 32 * NW;
+  const int lane = NW == 1 ? (int)threadIdx.x : (int)(threadIdx.x & 31), tid = threadIdx.x;
   int t, b, i;
   if (!locate_atom(md, a.nf, 1, 0, t, b, i)) return;
   const int N = md.N, nr = a.nr, nt = md.nt;
@@ -581,6 +616,7 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
   const T4* rpar = reinterpret_cast<const T4*>(spb + sl.rpar);
   T4* tab4 = reinterpret_cast<T4*>(smem_raw + L.tab);
   T* xtra = reinterpret_cast<T*>(smem_raw + L.xtra);
+  T* part = reinterpret_cast<T*>(smem_raw + L.part);
   T* acc = reinterpret_cast<T*>(smem_raw + L.acc);
   T* rsum = reinterpret_cast<T*>(smem_raw + L.rsum);
   T2* wch_all = reinterpret_cast<T2*>(smem_raw + L.wch);
@@ -595,9 +631,9 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
 
   // The neighbour record is at least two kernels old (it belongs to the neighbour kernel of this batch), and so is
   // the parameter block except in the fingerprint sweep, which directly follows k_prep.
-  if (lane == 0) mbar_init(bar, 2);
-  __syncwarp();
-  if (lane == 0) {
+  if (tid == 0) mbar_init(bar, 2);
+  block_sync<NW>();
+  if (tid == 0) {
     mbar_expect_tx(bar, (unsigned)a.row_stride);
     bulk_g2s(smem_addr(rowp), a.rows + gi * (size_t)a.row_stride, (unsigned)a.row_stride, bar);
     if (!IS_AF) {
@@ -606,10 +642,12 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
     }
   }
   if (MODE != MODE_FORCE)
-    for (int q = lane; q < NACC; q += 32) acc[q] = T(0);
-  if (ES == 8 && lane < 16) et[lane] = (T)EXP16_TABLE[lane];
+    for (int q = tid; q < NACC; q += LANES) acc[q] = T(0);
+  if (NW > 1 && MODE != MODE_FORCE)
+    for (int q = tid; q < nt * Frmax; q += LANES) rsum[q] = T(0);
+  if (ES == 8 && tid < 16) et[tid] = (T)EXP16_TABLE[tid];
   chain_wait();
-  if (IS_AF && lane == 0) {
+  if (IS_AF && tid == 0) {
     mbar_expect_tx(bar, (unsigned)sl.total);
     bulk_g2s(smem_addr(spb), a.spar + (size_t)t * a.spar_stride, (unsigned)sl.total, bar);
   }
@@ -640,20 +678,20 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
         const double v = warp_sum(a.vacc[((size_t)b * 9 + q) * VIR_SLOTS + lane]);
         if (lane == q) w = v;
       }
-      if (lane < 9) {
+      if (tid < 9) {
         const T e = (T)w - a.vlab[b * 9 + lane];
         wbs[lane] = a.vscale * (hub ? (e > T(1) ? T(1) : (e < T(-1) ? T(-1) : e)) : T(2) * e);
       }
     }
   }
   if (!mbar_wait(bar, 0)) {
-    if (lane == 0) set_status(a.status, STAFB_ERR_STAGE_TIMEOUT);
+    if (tid == 0) set_status(a.status, STAFB_ERR_STAGE_TIMEOUT);
     return;
   }
   int n = hdr[0];
   if (n > nr) n = nr;
   // first entry of every species' group (kept in shared memory like the counts, not in registers)
-  if (lane == 0) {
+  if (tid == 0) {
     int o = 0;
     for (int q = 0; q < STAFB_MAX_TYPES; q++) {
       off[q] = o;
@@ -661,11 +699,11 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
     }
     off[STAFB_MAX_TYPES] = o;
   }
-  __syncwarp();
+  block_sync<NW>();
   if (MODE == MODE_FGRAD) {
     // dF_k = Fbar_k - Fbar_i and its projection on the unit vector
     T4* dF = reinterpret_cast<T4*>(xtra);
-    for (int k = lane; k < n; k += 32) {
+    for (int k = tid; k < n; k += LANES) {
       const int id = ids[k];
       const T4 u = U[k];
       T4 d;
@@ -686,7 +724,7 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
   if (MODE == MODE_FORCE) {
     // channel weights 0.25 * e3 * netderiv of every (class, channel pair); the 0.5 of E = 0.5 sum e and the 0.5 of
     // the symmetrised pair sum
-    for (int idx = lane; idx < md.ncls * sl.maxp; idx += 32) {
+    for (int idx = tid; idx < md.ncls * sl.maxp; idx += LANES) {
       const int s = idx / sl.maxp, pr = idx - s * sl.maxp;
       T2 w = mk2(T(0), T(0));
       if (2 * pr < nact_s[s]) {
@@ -697,13 +735,13 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
       wch_all[idx] = w;
     }
   }
-  __syncwarp();
+  block_sync<NW>();
 
   T fix = T(0), fiy = T(0), fiz = T(0);  // FORCE: force on the central atom
   // ------------------------------------------------------------------ radial part
   if (MODE == MODE_FORCE) {
     // g_k = 0.5 * sum_c netderiv_c e2 e^{alpha d}(1 + alpha d) * dd/dr * u_k  (force/rad/reforce.cu.cc:45-136)
-    for (int k = lane; k < nr; k += 32) {
+    for (int k = tid; k < nr; k += LANES) {
       T gx = T(0), gy = T(0), gz = T(0);
       if (k < n) {
         int tk = 0;
@@ -726,7 +764,8 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
   } else {
     // one thread per (neighbour species q, channel c) walks that species' neighbours, so the sums over
     // neighbours need no cross-lane reduction; the per-species partial sums of a channel are combined
-    // through rsum[].  AF, AFV: fingerprints; FGRAD: gradnet; all but AF: alpha2b terms.
+    // through rsum[] (several warps: each takes every NW-th neighbour).  AF, AFV: fingerprints; FGRAD: gradnet; all but
+    // AF: alpha2b terms.
     const int nqc = nt * Fr;
     for (int L0 = 0; L0 < nqc; L0 += 32) {
       const int Lq = L0 + lane;
@@ -736,10 +775,10 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
         T gn = T(0), ga = T(0);
         if (rp.z != T(0)) {
           const T als = rp.x, al = rp.y;
-          const int r0_ = off[q], r1_ = off[q + 1];
+          const int r0_ = off[q] + (NW == 1 ? 0 : tid >> 5), r1_ = off[q + 1];
           const T4* dF = reinterpret_cast<const T4*>(xtra);
 #pragma unroll 4
-          for (int r = r0_; r < r1_; r++) {
+          for (int r = r0_; r < r1_; r += NW) {
             const T4 v = V[r];
             const T dk = v.z;
             const T ex = Ex<T>::f(als * dk, et);
@@ -755,18 +794,23 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
           gn *= rp.z;
           ga *= (MODE == MODE_FGRAD ? chrow[c] : T(1)) * rp.z;
         }
-        rsum[q * Frmax + c] = gn;
-        if (MODE != MODE_AF) acc[ACC_A2 + q * Frmax + c] = ga;
+        if (NW == 1) {
+          rsum[q * Frmax + c] = gn;
+          if (MODE != MODE_AF) acc[ACC_A2 + q * Frmax + c] = ga;
+        } else {
+          atomicAdd(&rsum[q * Frmax + c], gn);
+          if (MODE != MODE_AF) atomicAdd(&acc[ACC_A2 + q * Frmax + c], ga);
+        }
       }
     }
-    __syncwarp();
-    for (int c = lane; c < Fr; c += 32) {
+    block_sync<NW>();
+    for (int c = tid; c < Fr; c += LANES) {
       T v = T(0);
       for (int q = 0; q < nt; q++) v += rsum[q * Frmax + c];
       a.out[gi * Fmax + c] = v;
     }
   }
-  __syncwarp();
+  block_sync<NW>();
 
   // ------------------------------------------------------------------ angular part
   for (int ta = 0; ta < nt; ta++) {
@@ -786,7 +830,7 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
         // tables exp(a1*fc_k), exp(a2*fc_k) of the neighbours of the two species, all channel pairs of a
         // neighbour in flight together
         const int nu = same ? na_ : na_ + nb_;
-        for (int r = lane; r < nu; r += 32) {
+        for (int r = tid; r < nu; r += LANES) {
           const int k = (r < na_) ? oa + r : ob + (r - na_);
           const T fck = U[k].w * Ex<T>::scale();
           const T2 f2 = mk2(fck, fck);
@@ -801,7 +845,7 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
             }
           }
         }
-        __syncwarp();
+        block_sync<NW>();
         if (MODE == MODE_FORCE) {
           const T2* wch = wch_all + s * sl.maxp + p0;
           const int npass = same ? 1 : 2;
@@ -812,9 +856,9 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
             auto go = [&](auto tag) {
               constexpr int NCH = decltype(tag)::value;
               if (same)
-                pairs_force<T, NCH, true>(U, V, tab4, chq, chr, wch, et, oo, op, no, npt, lane, xtra, fix, fiy, fiz);
+                pairs_force<T, NCH, true, NW>(U, V, tab4, chq, chr, wch, et, oo, op, no, npt, tid, xtra, part, fix, fiy, fiz);
               else
-                pairs_force<T, NCH, false>(U, V, tab4, chq, chr, wch, et, oo, op, no, npt, lane, xtra, fix, fiy, fiz);
+                pairs_force<T, NCH, false, NW>(U, V, tab4, chq, chr, wch, et, oo, op, no, npt, tid, xtra, part, fix, fiy, fiz);
             };
             by_channels<T>(nch, go);
           }
@@ -830,9 +874,11 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
             constexpr int NCH = decltype(nch_tag)::value, NCHP = (NCH + 1) / 2;
             T2 r0[NCHP], r1[NCHP], r2[NCHP], r3[NCHP];
             if (same)
-              pairs_unordered<T, MODE, NCH, true>(U, V, dF, tab4, nr, chq, chr, et, oa, ob, na_, nb_, lane, r0, r1, r2, r3);
+              pairs_unordered<T, MODE, NCH, true, NW>(U, V, dF, tab4, nr, chq, chr, et, oa, ob, na_, nb_, tid, r0, r1, r2,
+                                                      r3);
             else
-              pairs_unordered<T, MODE, NCH, false>(U, V, dF, tab4, nr, chq, chr, et, oa, ob, na_, nb_, lane, r0, r1, r2, r3);
+              pairs_unordered<T, MODE, NCH, false, NW>(U, V, dF, tab4, nr, chq, chr, et, oa, ob, na_, nb_, tid, r0, r1, r2,
+                                                       r3);
             if (MODE == MODE_AF) {
               constexpr int NV = NCHP == 1 ? 2 : (NCHP == 2 ? 4 : 8);
               T v[NV];
@@ -867,31 +913,31 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
               const int c = actc[s * Famax + slot];
               const T2 ee = che_all[s * sl.maxp + p0 + lp];
               const T cf = T(0.5) * (h ? ee.y : ee.x);
-              if (v == 0) acc[ACC_GN + c] += cf * tot;
+              if (v == 0) acc_add<NW>(&acc[ACC_GN + c], cf * tot);
               else if (MODE != MODE_AF) {
                 const T hn = MODE == MODE_FGRAD ? cf * chrow[Fr + c] : cf;
-                acc[ACC_A3 + (s * Famax + c) * 3 + (v - 1)] += hn * tot;
+                acc_add<NW>(&acc[ACC_A3 + (s * Famax + c) * 3 + (v - 1)], hn * tot);
               }
             }
           }
         }
-        __syncwarp();  // the next chunk rewrites the tables
+        block_sync<NW>();  // the next chunk rewrites the tables
       }
     }
   }
-  __syncwarp();
+  block_sync<NW>();
 
   // ------------------------------------------------------------------ write-back
   if (IS_AF) {
-    for (int c = lane; c < Fa; c += 32) a.out[gi * Fmax + Fr + c] = acc[ACC_GN + c];
-    for (int c = Fr + Fa + lane; c < Fmax; c += 32) a.out[gi * Fmax + c] = T(0);
+    for (int c = tid; c < Fa; c += LANES) a.out[gi * Fmax + Fr + c] = acc[ACC_GN + c];
+    for (int c = Fr + Fa + tid; c < Fmax; c += LANES) a.out[gi * Fmax + c] = T(0);
     if (MODE == MODE_AFV) {
       T* vr = a.vout + gi * a.nv;
-      for (int q = lane; q < a.nv; q += 32) vr[q] = acc[q];
+      for (int q = tid; q < a.nv; q += LANES) vr[q] = acc[q];
     }
   } else if (MODE == MODE_FORCE) {
     T* fbo = a.out + (size_t)b * a.nall * 3;
-    for (int q = lane; q < 3 * n; q += 32) atomicAdd(fbo + (size_t)ids[q / 3] * 3 + (q % 3), xtra[q]);
+    for (int q = tid; q < 3 * n; q += LANES) atomicAdd(fbo + (size_t)ids[q / 3] * 3 + (q % 3), xtra[q]);
     fix = warp_sum(fix); fiy = warp_sum(fiy); fiz = warp_sum(fiz);
     if (lane == 0) {
       atomicAdd(fbo + (size_t)i * 3 + 0, fix);
@@ -905,7 +951,7 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
 #pragma unroll 1
       for (int c = 0; c < 3; c++) {
         T w0 = T(0), w1 = T(0), w2 = T(0);
-        for (int k = lane; k < n; k += 32) {
+        for (int k = tid; k < n; k += LANES) {
           const T4 u = U[k];
           const T g = xtra[k * 3 + c] / V[k].x;  // g_a * |r|
           w0 -= g * u.x; w1 -= g * u.y; w2 -= g * u.z;
@@ -920,16 +966,16 @@ __global__ void __launch_bounds__(32, SweepMinBlocks<MODE, sizeof(T)>::value)
       }
     }
   } else {  // FGRAD
-    for (int c = lane; c < Fa; c += 32) a.out[gi * Fmax + Fr + c] = acc[ACC_GN + c];
-    for (int c = Fr + Fa + lane; c < Fmax; c += 32) a.out[gi * Fmax + c] = T(0);
+    for (int c = tid; c < Fa; c += LANES) a.out[gi * Fmax + Fr + c] = acc[ACC_GN + c];
+    for (int c = Fr + Fa + tid; c < Fmax; c += LANES) a.out[gi * Fmax + c] = T(0);
     if (a.grad) {
       T* g2 = a.grad + md.off_a2[t];
-      for (int q = lane; q < nt * Fr; q += 32) {
+      for (int q = tid; q < nt * Fr; q += LANES) {
         const T v = acc[ACC_A2 + (q / Fr) * Frmax + (q % Fr)];
         if (v != T(0)) atomicAdd(g2 + q, v);
       }
       T* g3 = a.grad + md.off_a3[t];
-      for (int q = lane; q < md.C * 3 * Fa; q += 32) {
+      for (int q = tid; q < md.C * 3 * Fa; q += LANES) {
         const int sc = q / 3, comp = q - sc * 3, s = sc / Fa, c = sc - s * Fa;
         const T v = acc[ACC_A3 + (s * Famax + c) * 3 + comp];
         if (v != T(0)) atomicAdd(g3 + q, v);

@@ -1,20 +1,20 @@
 // Launches of the sweeps (sweep.cuh), instantiated for REAL by sweep_f32.cu and sweep_f64.cu.
 #include "model.cuh"
 
-template <class T, int MODE>
-int launch_sweep(stafb_model* m, cudaStream_t s, const SweepCall<T>& call) {
+template <class T, int MODE, int NW>
+static int launch_sweep_nw(stafb_model* m, cudaStream_t s, const SweepCall<T>& call) {
   const ModelDev& d = m->md;
   const int nr = m->ctx->nr;
-  const SweepSmem L = sweep_smem<T>(d, m->sl, nr, MODE);
+  const SweepSmem L = sweep_smem<T>(d, m->sl, nr, MODE, NW);
   const size_t sm = (size_t)L.total;
   if (sm > m->smem_limit) return STAFB_ERR_CAPACITY;
-  static bool attr_dev[MAX_DEVICES] = {false};  // per instantiation (T, MODE) and device
+  static bool attr_dev[MAX_DEVICES] = {false};  // per instantiation (T, MODE, NW) and device
   bool& attr_done = attr_dev[device_slot()];
   if (sm > 48 * 1024 && !attr_done) {
-    STAFB_CUDA_OK(cudaFuncSetAttribute(k_sweep<T, MODE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    STAFB_CUDA_OK(cudaFuncSetAttribute(k_sweep<T, MODE, false, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)m->smem_limit));
     if (MODE == MODE_FORCE)
-      STAFB_CUDA_OK(cudaFuncSetAttribute(k_sweep<T, MODE, MODE == MODE_FORCE>,
+      STAFB_CUDA_OK(cudaFuncSetAttribute(k_sweep<T, MODE, MODE == MODE_FORCE, NW>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m->smem_limit));
     attr_done = true;
   }
@@ -31,11 +31,22 @@ int launch_sweep(stafb_model* m, cudaStream_t s, const SweepCall<T>& call) {
   a.vacc = call.vacc; a.vlab = call.vlab; a.vscale = call.vscale;
   const int blocks = call.nf * d.N;
   if (MODE == MODE_FORCE && call.vir)
-    STAFB_CUDA_OK(launch_chained(k_sweep<T, MODE, MODE == MODE_FORCE>, blocks, 32, sm, s, d, a, L));
+    STAFB_CUDA_OK(launch_chained(k_sweep<T, MODE, MODE == MODE_FORCE, NW>, blocks, 32 * NW, sm, s, d, a, L));
   else
-    STAFB_CUDA_OK(launch_chained(k_sweep<T, MODE, false>, blocks, 32, sm, s, d, a, L));
+    STAFB_CUDA_OK(launch_chained(k_sweep<T, MODE, false, NW>, blocks, 32 * NW, sm, s, d, a, L));
   m->ctx->launches++;
   return STAFB_OK;
+}
+
+template <class T, int MODE>
+int launch_sweep(stafb_model* m, cudaStream_t s, const SweepCall<T>& call) {
+  // Four warps per atom while that still leaves the chip room: a warp alone takes 10-14 us for its atom whatever the
+  // others do, and up to about three atoms per SM (two in double precision) the SMs are nearly empty.  Train step of
+  // 96 / 300 / 450 atoms: fp32 97 -> 88, 103 -> 97, 110 -> 105 us, fp64 133 -> 112, 141 -> 140, 154 -> 154 us; at 768
+  // atoms one warp per atom is the faster form (119 against 141 us).
+  static const int few = (sizeof(T) == 4 ? 3 : 2) * sm_count();
+  if (call.nf * m->md.N <= few) return launch_sweep_nw<T, MODE, 4>(m, s, call);
+  return launch_sweep_nw<T, MODE, 1>(m, s, call);
 }
 
 template int launch_sweep<REAL, MODE_AF>(stafb_model*, cudaStream_t, const SweepCall<REAL>&);
