@@ -28,6 +28,8 @@ __device__ __forceinline__ float r_cos(float x) { return cosf(x); }
 __device__ __forceinline__ double r_cos(double x) { return cos(x); }
 __device__ __forceinline__ float r_sin(float x) { return sinf(x); }
 __device__ __forceinline__ double r_sin(double x) { return sin(x); }
+__device__ __forceinline__ void r_sincos(float x, float* s, float* c) { sincosf(x, s, c); }
+__device__ __forceinline__ void r_sincos(double x, double* s, double* c) { sincos(x, s, c); }
 __device__ __forceinline__ float r_sqrt(float x) { return sqrtf(x); }
 __device__ __forceinline__ double r_sqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float r_pow(float x, float y) { return powf(x, y); }
@@ -164,13 +166,14 @@ struct stafb_ctx {
   int* cell_of;       // [max_batch, n_max]
   int* cell_count;    // [max_batch, cell_cap]
   int* cell_start;    // [max_batch, cell_cap+1]
-  int* cell_cursor;   // [max_batch, cell_cap]
-  int* cells_raw;     // [max_batch, n_max]
-  int* cells_sorted;  // [max_batch, n_max]
+  int* cell_cursor;   // [max_batch, cell_cap] arrival slots of the atoms inside their cells
+  int* cells_raw;     // [max_batch, n_max] atoms by cell in arrival order
+  void* cxyz;         // T[max_batch, n_max, 4] atoms by cell in ascending index: fractional coordinates, index
   void* geom;         // T[max_batch, n_max, nr, 4]: MIC vector r_i - r_j and its norm, sorted order
   void* gsc;          // T[max_batch, n_max, nr, 2]: d(raddescr)/dr and d(des3bsupp)/dr
   int* status_d;
-  int* status_h;  // pinned
+  int* status_h;  // pinned, written by the device: statuses handed over by k_loss (inference) or k_take_status
+  int status_fresh;  // the last launches on this context ended with such a hand-over
   int launches;
   // optional per-phase timing of the fused path (CUDA events on the launching stream)
   int timing;

@@ -98,7 +98,8 @@ __global__ void __launch_bounds__(256)
            const T* __restrict__ theta, T pe, T pf, T pb, T bound, int loss_kind, T* __restrict__ ebar,
            T* __restrict__ grad, double* __restrict__ losses, int* status, int* status_main,
            const double* __restrict__ vacc, T* __restrict__ virial_out, double* __restrict__ mirror,
-           double* __restrict__ epart, unsigned* __restrict__ ecount, const T* __restrict__ v_label, T pv) {
+           double* __restrict__ epart, unsigned* __restrict__ ecount, const T* __restrict__ v_label, T pv,
+           int* __restrict__ status_h) {
   __shared__ double red[9];
   __shared__ int last_s;
   const int N = md.N;
@@ -157,6 +158,10 @@ __global__ void __launch_bounds__(256)
       if (train) {
         atomicAdd(losses + 1, (double)le / nf);
         ebar[blk] = pe * de / T(nf) * T(0.5) / (per_atom ? T(N) : T(1));
+      } else if (status_h) {
+        // an inference evaluation ends here: its status goes straight to the host's word (stafb_status)
+        const int v = atomicExch(status, 0);
+        if (v) *status_h = v;
       }
     }
   } else if (blk < nf * eb + fb) {
@@ -566,9 +571,10 @@ static int run_fused(stafb_ctx* c, stafb_model* m, cudaStream_t s, const T* pos,
                                  (T*)m->ebar, grad, m->losses_d, cg->status_d, c->status_d, vacc, virial_out,
                                  train ? m->mirror_next : (double*)nullptr, m->epart,
                                  reinterpret_cast<unsigned*>(m->epart + (size_t)c->max_batch * LOSS_EB_MAX), v_label,
-                                 (T)pv));
+                                 (T)pv, train ? (int*)nullptr : c->status_h));
     m->mirror_next = nullptr;
     c->launches++;
+    c->status_fresh = train ? 0 : 1;
   }
   mark();  // loss
   if (train) {
@@ -608,7 +614,8 @@ static int run_mlp_only(stafb_ctx* c, stafb_model* m, cudaStream_t s, const T* a
                                m->losses_d, c->status_d, c->status_d, (const double*)nullptr, (T*)nullptr,
                                (double*)nullptr, m->epart,
                                reinterpret_cast<unsigned*>(m->epart + (size_t)c->max_batch * LOSS_EB_MAX),
-                               (const T*)nullptr, T(0));
+                               (const T*)nullptr, T(0), (int*)nullptr);
+  c->status_fresh = 0;
   c->launches++;
   STAFB_CUDA_OK(cudaGetLastError());
   return STAFB_OK;

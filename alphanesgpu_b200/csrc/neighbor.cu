@@ -61,13 +61,207 @@ __device__ void frame_geometry(const T* __restrict__ B, int N, T cutoff, int cel
   g.sz = T(1.) / (T)cz;
 }
 
-// Frame geometry, fractional coordinates (celle_gpu.cu.cc:11-28) and the cell of every atom
-// (celle_gpu.cu.cc:176-201) in one launch: grid (blocks over atoms, frames); every block derives its
+// An atom in cell order: fractional coordinates and index, what the neighbour search reads of a candidate in one load.
+template <class T>
+__device__ __forceinline__ typename Vec4<T>::type cell_entry(T fx, T fy, T fz, int i);
+template <>
+__device__ __forceinline__ float4 cell_entry<float>(float fx, float fy, float fz, int i) {
+  return make_float4(fx, fy, fz, __int_as_float(i));
+}
+template <>
+__device__ __forceinline__ double4 cell_entry<double>(double fx, double fy, double fz, int i) {
+  double4 v;
+  v.x = fx; v.y = fy; v.z = fz; v.w = __longlong_as_double((long long)i);
+  return v;
+}
+__device__ __forceinline__ int entry_index(const float4& v) { return __float_as_int(v.w); }
+__device__ __forceinline__ int entry_index(const double4& v) { return (int)__double_as_longlong(v.w); }
+
+// Fractional coordinates (celle_gpu.cu.cc:11-28) and cell (celle_gpu.cu.cc:176-201) of one atom.
+template <class T>
+__device__ __forceinline__ int place_atom(const FrameGeom<T>& g, const T* __restrict__ p, T& fx, T& fy, T& fz) {
+  const T px = p[0], py = p[1], pz = p[2];
+  fx = (g.inv[0] * px + g.inv[1] * py + g.inv[2] * pz);
+  fy = (g.inv[3] * py + g.inv[4] * pz);
+  fz = (g.inv[5] * pz);
+  int cx = (int)r_floor(fx / g.sx);
+  cx = cx % g.nx;
+  if (cx < 0) cx += g.nx;
+  int cy = (int)r_floor(fy / g.sy);
+  cy = cy % g.ny;
+  if (cy < 0) cy += g.ny;
+  int cz = (int)r_floor(fz / g.sz);
+  cz = cz % g.nz;
+  if (cz < 0) cz += g.nz;
+  return cx + cy * g.nx + cz * (g.nx * g.ny);
+}
+
+// Rank of atom i among the members of its cell, src[s0, s1): the reference's slot order is the atomicAdd arrival order
+// (celle_gpu.cu.cc:197-200), restated as ascending atom index.
+__device__ __forceinline__ int cell_rank(const int* src, int s0, int s1, int i) {
+  int r = 0;
+  for (int f = s0; f < s1; f++) r += (src[f] < i);
+  return r;
+}
+
+// Exclusive scan of one value per thread over the block (warps <= 32); part: 33 ints of shared memory.  Returns the
+// exclusive prefix, total in `tot`.
+__device__ __forceinline__ int block_scan(int v, int* part, int& tot) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  int x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) part[w] = x;
+  __syncthreads();
+  int off = 0, all = 0;
+  for (int q = 0; q < nw; q++) {
+    const int pq = part[q];
+    off += q < w ? pq : 0;
+    all += pq;
+  }
+  __syncthreads();
+  tot = all;
+  return off + x - v;
+}
+
+// Frame geometry, fractional coordinates, cell counts, their scan and the atoms in cell order (ascending index inside
+// a cell) of one frame by one block, all bookkeeping in shared memory: up to CELLS_SMALL_MAX atoms.  Every atom is one
+// thread's in all passes: it takes its arrival slot from the counter, leaves its index there, and then ranks itself
+// among its cell's members (11 on average in liquid water), so no pass walks the frame.  Bound by the latency of its
+// four dependent passes and the barriers between them, hence no more threads than atoms.
+// Dynamic shared memory: (cell_cap + 1 + 2 N) ints.
+constexpr int CELLS_SMALL_MAX = 2048;
+template <class T>
+__global__ void __launch_bounds__(1024)
+    k_cell_lists_small(const T* __restrict__ pos, const T* __restrict__ box, int N, T cutoff, int cell_cap, int mpc,
+                       FrameGeom<T>* __restrict__ fg, T* __restrict__ frac, int* __restrict__ cell_of,
+                       int* __restrict__ cell_start, typename Vec4<T>::type* __restrict__ cxyz,
+                       int* __restrict__ status) {
+  extern __shared__ int sm_i[];
+  __shared__ FrameGeom<T> gs;
+  __shared__ int part[33];
+  int* cnt = sm_i;                 // [cell_cap + 1] counts, then exclusive starts
+  int* raw = sm_i + cell_cap + 1;  // [N] atoms in arrival order
+  int* slot = raw + N;             // [N] arrival slot of an atom
+  const int b = blockIdx.x, tid = threadIdx.x;
+  chain_wait();
+  if (tid == 0) {
+    frame_geometry<T>(box + 6 * b, N, cutoff, cell_cap, gs, status);
+    fg[b] = gs;
+  }
+  __syncthreads();
+  const FrameGeom<T>& g = gs;
+  const int ncell = g.ncell;
+  for (int c = tid; c < ncell; c += blockDim.x) cnt[c] = 0;
+  __syncthreads();
+  T* fr = frac + (size_t)b * N * 3;
+  int* co = cell_of + (size_t)b * N;
+  for (int i = tid; i < N; i += blockDim.x) {
+    T fx, fy, fz;
+    const int c = place_atom<T>(g, pos + ((size_t)b * N + i) * 3, fx, fy, fz);
+    fr[3 * i] = fx; fr[3 * i + 1] = fy; fr[3 * i + 2] = fz;
+    co[i] = c;
+    slot[i] = atomicAdd(&cnt[c], 1);
+  }
+  __syncthreads();
+  int* st = cell_start + (size_t)b * (cell_cap + 1);
+  int carry = 0;
+  for (int base = 0; base < ncell; base += blockDim.x) {
+    const int c = base + tid, v = (c < ncell) ? cnt[c] : 0;
+    if (v > mpc) set_status(status, STAFB_ERR_CELL_OVERFLOW);
+    int tot;
+    const int x = carry + block_scan(v, part, tot);
+    if (c < ncell) cnt[c] = st[c] = x;
+    carry += tot;
+  }
+  if (tid == 0) cnt[ncell] = st[ncell] = N;
+  __syncthreads();
+  for (int i = tid; i < N; i += blockDim.x) raw[cnt[co[i]] + slot[i]] = i;
+  __syncthreads();
+  for (int i = tid; i < N; i += blockDim.x) {
+    const int c = co[i], s0 = cnt[c];
+    cxyz[(size_t)b * N + s0 + cell_rank(raw, s0, cnt[c + 1], i)] = cell_entry<T>(fr[3 * i], fr[3 * i + 1], fr[3 * i + 2], i);
+  }
+}
+
+// The same for frames of up to CELLS_CLUSTER_MAX atoms by a cluster of eight blocks: counters and lists in global
+// memory (they stay in L2), a cluster barrier between the passes.  24,576 atoms: one launch of 9 us where a memset
+// and four kernels took 33 us, nearly all of it launch gaps and one wave each of a few loads.
+constexpr int CELLS_CLUSTER = 8;
+constexpr int CELLS_CLUSTER_MAX = 65536;
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+template <class T>
+__global__ void __cluster_dims__(CELLS_CLUSTER, 1, 1) __launch_bounds__(1024)
+    k_cell_lists_cluster(const T* __restrict__ pos, const T* __restrict__ box, int N, T cutoff, int cell_cap, int mpc,
+                         FrameGeom<T>* __restrict__ fg, T* __restrict__ frac, int* __restrict__ cell_of,
+                         int* __restrict__ cell_count, int* __restrict__ cell_start, int* __restrict__ slot_all,
+                         int* __restrict__ raw_all, typename Vec4<T>::type* __restrict__ cxyz, int* __restrict__ status) {
+  __shared__ FrameGeom<T> gs;
+  __shared__ int part[33];
+  const int b = blockIdx.x / CELLS_CLUSTER, rank = blockIdx.x % CELLS_CLUSTER;
+  const int tid = threadIdx.x, gt = rank * 1024 + tid, GT = CELLS_CLUSTER * 1024;
+  chain_wait();
+  if (tid == 0) {
+    frame_geometry<T>(box + 6 * b, N, cutoff, cell_cap, gs, status);
+    if (rank == 0) fg[b] = gs;
+  }
+  __syncthreads();
+  const FrameGeom<T>& g = gs;
+  const int ncell = g.ncell;
+  int* cnt = cell_count + (size_t)b * cell_cap;
+  int* slot = slot_all + (size_t)b * cell_cap;
+  int* st = cell_start + (size_t)b * (cell_cap + 1);
+  int* raw = raw_all + (size_t)b * N;
+  int* co = cell_of + (size_t)b * N;
+  T* fr = frac + (size_t)b * N * 3;
+  for (int c = gt; c < ncell; c += GT) cnt[c] = 0;
+  cluster_barrier();
+  for (int i = gt; i < N; i += GT) {
+    T fx, fy, fz;
+    const int c = place_atom<T>(g, pos + ((size_t)b * N + i) * 3, fx, fy, fz);
+    fr[3 * i] = fx; fr[3 * i + 1] = fy; fr[3 * i + 2] = fz;
+    co[i] = c;
+    slot[i] = atomicAdd(cnt + c, 1);
+  }
+  cluster_barrier();
+  // every block scans the counts of all cells below its share first (a strided sum), then its share
+  const int per = (ncell + CELLS_CLUSTER - 1) / CELLS_CLUSTER, c0 = min(rank * per, ncell), c1 = min(c0 + per, ncell);
+  int below = 0;
+  for (int c = tid; c < c0; c += 1024) below += __ldcg(cnt + c);
+  int carry;
+  block_scan(below, part, carry);
+  for (int base = c0; base < c1; base += 1024) {
+    const int c = base + tid, v = (c < c1) ? __ldcg(cnt + c) : 0;
+    if (v > mpc) set_status(status, STAFB_ERR_CELL_OVERFLOW);
+    int tot;
+    const int x = carry + block_scan(v, part, tot);
+    if (c < c1) st[c] = x;
+    carry += tot;
+  }
+  if (gt == 0) st[ncell] = N;
+  cluster_barrier();
+  for (int i = gt; i < N; i += GT) raw[__ldcg(st + co[i]) + slot[i]] = i;
+  cluster_barrier();
+  for (int i = gt; i < N; i += GT) {
+    const int c = co[i], s0 = __ldcg(st + c), s1 = __ldcg(st + c + 1);
+    int r = 0;
+    for (int f = s0; f < s1; f++) r += (__ldcg(raw + f) < i);
+    cxyz[(size_t)b * N + s0 + r] = cell_entry<T>(fr[3 * i], fr[3 * i + 1], fr[3 * i + 2], i);
+  }
+}
+
+// Larger frames: the same passes as kernels over all atoms.  grid (blocks over atoms, frames); every block derives its
 // frame's geometry again (a few dozen flops) instead of waiting for a separate set-up launch.
 template <class T>
 __global__ void k_cells(const T* __restrict__ pos, const T* __restrict__ box, int nf, int N, T cutoff, int cell_cap,
                         FrameGeom<T>* __restrict__ fg, T* __restrict__ frac, int* __restrict__ cell_of,
-                        int* __restrict__ cell_count, int* __restrict__ status) {
+                        int* __restrict__ cell_count, int* __restrict__ slot, int* __restrict__ status) {
   __shared__ FrameGeom<T> gs;
   const int b = blockIdx.y;
   chain_wait();
@@ -78,217 +272,56 @@ __global__ void k_cells(const T* __restrict__ pos, const T* __restrict__ box, in
   __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const FrameGeom<T>& g = gs;
   const size_t t = (size_t)b * N + i;
-  T px = pos[t * 3 + 0], py = pos[t * 3 + 1], pz = pos[t * 3 + 2];
-  T fx = (g.inv[0] * px + g.inv[1] * py + g.inv[2] * pz);
-  T fy = (g.inv[3] * py + g.inv[4] * pz);
-  T fz = (g.inv[5] * pz);
-  frac[t * 3 + 0] = fx;
-  frac[t * 3 + 1] = fy;
-  frac[t * 3 + 2] = fz;
-  int cx = (int)r_floor(fx / g.sx);
-  cx = cx % g.nx;
-  if (cx < 0) cx += g.nx;
-  int cy = (int)r_floor(fy / g.sy);
-  cy = cy % g.ny;
-  if (cy < 0) cy += g.ny;
-  int cz = (int)r_floor(fz / g.sz);
-  cz = cz % g.nz;
-  if (cz < 0) cz += g.nz;
-  int c = cx + cy * g.nx + cz * (g.nx * g.ny);
+  T fx, fy, fz;
+  const int c = place_atom<T>(gs, pos + t * 3, fx, fy, fz);
+  frac[t * 3] = fx; frac[t * 3 + 1] = fy; frac[t * 3 + 2] = fz;
   cell_of[t] = c;
-  atomicAdd(cell_count + (size_t)b * cell_cap + c, 1);
-}
-
-// Members of every cell in ascending atom index, gathered directly by one warp per cell that walks
-// the frame's atoms 32 at a time (used for small systems; replaces the fill + sort pair).
-template <class T>
-__global__ void k_gather_cells(const FrameGeom<T>* __restrict__ fg, int nf, int N, const int* __restrict__ cell_of,
-                               const int* __restrict__ cell_start, int* __restrict__ cells_sorted, int cell_cap) {
-  chain_wait();
-  int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  int b = gw / cell_cap, c = gw - b * cell_cap;
-  if (b >= nf || c >= fg[b].ncell) return;
-  const int* co = cell_of + (size_t)b * N;
-  int* dst = cells_sorted + (size_t)b * N + cell_start[(size_t)b * (cell_cap + 1) + c];
-  const unsigned lt = (1u << lane) - 1u;
-  int cnt = 0;
-  for (int j0 = 0; j0 < N; j0 += 32) {
-    const int j = j0 + lane;
-    const bool p = (j < N) && (co[j] == c);
-    const unsigned bal = __ballot_sync(0xffffffffu, p);
-    if (p) dst[cnt + __popc(bal & lt)] = j;
-    cnt += __popc(bal);
-  }
-}
-
-// Small systems: frame geometry, fractional coordinates, cell of every atom, per-cell counts, their
-// exclusive scan and the members of every cell in ascending atom index - one block per frame, all
-// bookkeeping in shared memory (k_cells + k_scan + k_gather_cells in one launch, no counter memset).
-// Dynamic shared memory: (cell_cap + 1 + N) ints.
-template <class T>
-__global__ void __launch_bounds__(1024)
-    k_cell_lists_small(const T* __restrict__ pos, const T* __restrict__ box, int N, T cutoff, int cell_cap, int mpc,
-                       FrameGeom<T>* __restrict__ fg, T* __restrict__ frac, int* __restrict__ cell_of,
-                       int* __restrict__ cell_start, int* __restrict__ cells_sorted, int* __restrict__ status) {
-  extern __shared__ int sm_i[];
-  __shared__ FrameGeom<T> gs;
-  __shared__ int part[32];
-  __shared__ int carry;
-  int* cnt = sm_i;                  // [cell_cap + 1] counts, then exclusive starts
-  int* cof = sm_i + cell_cap + 1;   // [N] cell of every atom
-  const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
-  if (tid == 0) {
-    frame_geometry<T>(box + 6 * b, N, cutoff, cell_cap, gs, status);
-    fg[b] = gs;
-    carry = 0;
-  }
-  for (int c = tid; c <= cell_cap; c += blockDim.x) cnt[c] = 0;
-  __syncthreads();
-  const FrameGeom<T>& g = gs;
-  for (int i = tid; i < N; i += blockDim.x) {
-    const size_t t = (size_t)b * N + i;
-    T px = pos[t * 3 + 0], py = pos[t * 3 + 1], pz = pos[t * 3 + 2];
-    T fx = (g.inv[0] * px + g.inv[1] * py + g.inv[2] * pz);
-    T fy = (g.inv[3] * py + g.inv[4] * pz);
-    T fz = (g.inv[5] * pz);
-    frac[t * 3 + 0] = fx;
-    frac[t * 3 + 1] = fy;
-    frac[t * 3 + 2] = fz;
-    int cx = (int)r_floor(fx / g.sx);
-    cx = cx % g.nx;
-    if (cx < 0) cx += g.nx;
-    int cy = (int)r_floor(fy / g.sy);
-    cy = cy % g.ny;
-    if (cy < 0) cy += g.ny;
-    int cz = (int)r_floor(fz / g.sz);
-    cz = cz % g.nz;
-    if (cz < 0) cz += g.nz;
-    const int c = cx + cy * g.nx + cz * (g.nx * g.ny);
-    cell_of[t] = c;
-    cof[i] = c;
-    atomicAdd(&cnt[c], 1);
-  }
-  __syncthreads();
-  const int ncell = g.ncell;
-  int* st = cell_start + (size_t)b * (cell_cap + 1);
-  for (int base = 0; base < ncell; base += blockDim.x) {
-    const int c = base + tid;
-    const int v = (c < ncell) ? cnt[c] : 0;
-    if (v > mpc) set_status(status, STAFB_ERR_CELL_OVERFLOW);
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) part[w] = x;
-    __syncthreads();
-    int off = carry;
-    for (int q = 0; q < w; q++) off += part[q];
-    if (c < ncell) {
-      cnt[c] = off + x - v;
-      st[c] = off + x - v;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      int tot = 0;
-      for (int q = 0; q < nw; q++) tot += part[q];
-      carry += tot;
-    }
-    __syncthreads();
-  }
-  if (tid == 0) st[ncell] = carry;
-  // members in ascending atom index: one warp per cell walks the frame's atoms 32 at a time
-  const unsigned lt = (1u << lane) - 1u;
-  int* dstb = cells_sorted + (size_t)b * N;
-  for (int c = w; c < ncell; c += nw) {
-    int* dst = dstb + cnt[c];
-    int k = 0;
-    for (int j0 = 0; j0 < N; j0 += 32) {
-      const int j = j0 + lane;
-      const bool p = (j < N) && (cof[j] == c);
-      const unsigned bal = __ballot_sync(0xffffffffu, p);
-      if (p) dst[k + __popc(bal & lt)] = j;
-      k += __popc(bal);
-    }
-  }
+  slot[(size_t)b * cell_cap + i] = atomicAdd(cell_count + (size_t)b * cell_cap + c, 1);
 }
 
 // Exclusive scan of the per-cell counts of one frame (one block per frame).
 template <class T>
 __global__ void k_scan(const FrameGeom<T>* __restrict__ fg, const int* __restrict__ cell_count,
-                       int* __restrict__ cell_start, int* __restrict__ cell_cursor, int cell_cap, int mpc,
-                       int* __restrict__ status) {
-  __shared__ int part[32];
-  __shared__ int carry;
+                       int* __restrict__ cell_start, int cell_cap, int mpc, int* __restrict__ status) {
+  __shared__ int part[33];
   chain_wait();
   const int b = blockIdx.x, ncell = fg[b].ncell;
   const int* cnt = cell_count + (size_t)b * cell_cap;
   int* st = cell_start + (size_t)b * (cell_cap + 1);
-  int* cur = cell_cursor + (size_t)b * cell_cap;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  int carry = 0;
   for (int base = 0; base < ncell; base += blockDim.x) {
-    int c = base + threadIdx.x;
-    int v = (c < ncell) ? cnt[c] : 0;
+    const int c = base + threadIdx.x, v = (c < ncell) ? cnt[c] : 0;
     if (v > mpc) set_status(status, STAFB_ERR_CELL_OVERFLOW);
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) part[w] = x;
-    __syncthreads();
-    int off = carry;
-    for (int q = 0; q < w; q++) off += part[q];
-    if (c < ncell) {
-      st[c] = off + x - v;
-      cur[c] = 0;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int tot = 0;
-      for (int q = 0; q < nw; q++) tot += part[q];
-      carry += tot;
-    }
-    __syncthreads();
+    int tot;
+    const int x = carry + block_scan(v, part, tot);
+    if (c < ncell) st[c] = x;
+    carry += tot;
   }
   if (threadIdx.x == 0) st[ncell] = carry;
 }
 
 __global__ void k_fill(int nf, int N, const int* __restrict__ cell_of, const int* __restrict__ cell_start,
-                       int* __restrict__ cell_cursor, int* __restrict__ cells_raw, int cell_cap) {
+                       const int* __restrict__ slot, int* __restrict__ raw, int cell_cap) {
   chain_wait();
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nf * N) return;
-  int b = t / N, i = t - b * N;
-  int c = cell_of[t];
-  int slot = atomicAdd(cell_cursor + (size_t)b * cell_cap + c, 1);
-  cells_raw[(size_t)b * N + cell_start[(size_t)b * (cell_cap + 1) + c] + slot] = i;
+  const int b = t / N, i = t - b * N;
+  raw[(size_t)b * N + cell_start[(size_t)b * (cell_cap + 1) + cell_of[t]] + slot[(size_t)b * cell_cap + i]] = i;
 }
 
-// Orders every cell's members by atom index (one warp per cell): the reference's slot order
-// is the atomicAdd arrival order (celle_gpu.cu.cc:197-200), restated as ascending index.
 template <class T>
-__global__ void k_sort_cells(const FrameGeom<T>* __restrict__ fg, int nf, int N, const int* __restrict__ cell_start,
-                             const int* __restrict__ cells_raw, int* __restrict__ cells_sorted, int cell_cap) {
+__global__ void k_order_cells(int nf, int N, const int* __restrict__ cell_of, const int* __restrict__ cell_start,
+                              const int* __restrict__ raw, const T* __restrict__ frac,
+                              typename Vec4<T>::type* __restrict__ cxyz, int cell_cap) {
   chain_wait();
-  int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  int b = gw / cell_cap, c = gw - b * cell_cap;
-  if (b >= nf || c >= fg[b].ncell) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nf * N) return;
+  const int b = t / N, i = t - b * N;
   const int* st = cell_start + (size_t)b * (cell_cap + 1);
-  int s0 = st[c], s1 = st[c + 1];
-  const int* src = cells_raw + (size_t)b * N;
-  int* dst = cells_sorted + (size_t)b * N;
-  for (int e = s0 + lane; e < s1; e += 32) {
-    int me = src[e], r = 0;
-    for (int f = s0; f < s1; f++) r += (src[f] < me);
-    dst[s0 + r] = me;
-  }
+  const int c = cell_of[t], s0 = st[c];
+  const int r = cell_rank(raw + (size_t)b * N, s0, st[c + 1], i);
+  cxyz[(size_t)b * N + s0 + r] = cell_entry<T>(frac[(size_t)t * 3], frac[(size_t)t * 3 + 1], frac[(size_t)t * 3 + 2], i);
 }
 
 template <class T>
@@ -314,7 +347,8 @@ struct SlotVals {
 // descriptor, angular-support cutoff, their gradients, the neighbour id and the compact geometry the
 // angular-descriptor kernel reads.  Slots past the neighbour count (valid == false) are zero-filled.  Every
 // output pointer may be null; `sv` always receives the slot's values for the record of the fused sweeps.
-template <class T>
+// OPS == false: only those values are wanted, and the gradient vectors (six divisions) are not formed.
+template <class T, bool OPS>
 __device__ __forceinline__ void radial_slot(const CoreCoef<T>& cc, bool valid, int j, T vx, T vy, T vz, size_t base,
                                             int k, int nr, T* __restrict__ raddescr, T* __restrict__ des3bsupp,
                                             int* __restrict__ intmap2b, T* __restrict__ der2b,
@@ -325,14 +359,12 @@ __device__ __forceinline__ void radial_slot(const CoreCoef<T>& cc, bool valid, i
   T dn = T(0), s2 = T(0), s3 = T(0);
   if (valid) {
     dn = r_sqrt(vx * vx + vy * vy + vz * vz);
+    T sa, ca;
+    r_sincos(PI * dn / cc.Ra, &sa, &ca);
     if (dn < cc.Ra) {
       nang++;
-      d3 = T(0.5) * (r_cos(PI * dn / cc.Ra) + T(1));
-      const T pre = T(-0.5) * r_sin(PI * dn / cc.Ra) * PI / cc.Ra;
-      s3 = pre;
-      g3x = pre * vx / dn;
-      g3y = pre * vy / dn;
-      g3z = pre * vz / dn;
+      d3 = T(0.5) * (ca + T(1));
+      s3 = T(-0.5) * sa * PI / cc.Ra;
     }
     if (dn < cc.Rs) {
       // A/r^1 + B/r^-30 + C with the powers by repeated multiplication (the reference calls pow;
@@ -340,43 +372,46 @@ __device__ __forceinline__ void radial_slot(const CoreCoef<T>& cc, bool valid, i
       const T r2 = dn * dn, r4 = r2 * r2, r8 = r4 * r4, r16 = r8 * r8;
       const T r28 = r16 * r8 * r4, r29 = r28 * dn, r30 = r28 * r2;
       rd = cc.A / dn + cc.B * r30 + cc.C;
-      const T pre = (-cc.pa * cc.A / r2 - cc.pb * cc.B * r29);
-      s2 = pre;
-      g2x = pre * vx / dn;
-      g2y = pre * vy / dn;
-      g2z = pre * vz / dn;
+      s2 = (-cc.pa * cc.A / r2 - cc.pb * cc.B * r29);
     } else {
-      rd = T(0.5) * (r_cos(PI * dn / cc.Rc) + T(1));
-      const T pre = T(-0.5) * r_sin(PI * dn / cc.Rc) * PI / cc.Rc;
-      s2 = pre;
-      g2x = pre * vx / dn;
-      g2y = pre * vy / dn;
-      g2z = pre * vz / dn;
+      if (cc.Ra != cc.Rc) r_sincos(PI * dn / cc.Rc, &sa, &ca);
+      rd = T(0.5) * (ca + T(1));
+      s2 = T(-0.5) * sa * PI / cc.Rc;
+    }
+    if (OPS) {
+      g3x = s3 * vx / dn;
+      g3y = s3 * vy / dn;
+      g3z = s3 * vz / dn;
+      g2x = s2 * vx / dn;
+      g2y = s2 * vy / dn;
+      g2z = s2 * vz / dn;
     }
   }
-  if (raddescr) raddescr[base * nr + k] = rd;
-  if (des3bsupp) des3bsupp[base * nr + k] = d3;
-  if (der2b) {
-    der2b[(base * 3 + 0) * nr + k] = g2x;
-    der2b[(base * 3 + 1) * nr + k] = g2y;
-    der2b[(base * 3 + 2) * nr + k] = g2z;
-  }
-  if (der3bsupp) {
-    der3bsupp[(base * 3 + 0) * nr + k] = g3x;
-    der3bsupp[(base * 3 + 1) * nr + k] = g3y;
-    der3bsupp[(base * 3 + 2) * nr + k] = g3z;
-  }
-  if (intmap2b) intmap2b[base * (nr + 1) + 1 + k] = valid ? j : 0;
-  if (geom) {
-    typename Vec4<T>::type q;
-    q.x = vx; q.y = vy; q.z = vz; q.w = dn;
-    reinterpret_cast<typename Vec4<T>::type*>(geom)[base * nr + k] = q;
-  }
-  if (gsc) {
-    // scalar radial derivatives: der2b = s2 * v/|v|, der3bsupp = s3 * v/|v|
-    typename Vec2<T>::type q;
-    q.x = s2; q.y = s3;
-    reinterpret_cast<typename Vec2<T>::type*>(gsc)[base * nr + k] = q;
+  if (OPS) {
+    if (raddescr) raddescr[base * nr + k] = rd;
+    if (des3bsupp) des3bsupp[base * nr + k] = d3;
+    if (der2b) {
+      der2b[(base * 3 + 0) * nr + k] = g2x;
+      der2b[(base * 3 + 1) * nr + k] = g2y;
+      der2b[(base * 3 + 2) * nr + k] = g2z;
+    }
+    if (der3bsupp) {
+      der3bsupp[(base * 3 + 0) * nr + k] = g3x;
+      der3bsupp[(base * 3 + 1) * nr + k] = g3y;
+      der3bsupp[(base * 3 + 2) * nr + k] = g3z;
+    }
+    if (intmap2b) intmap2b[base * (nr + 1) + 1 + k] = valid ? j : 0;
+    if (geom) {
+      typename Vec4<T>::type q;
+      q.x = vx; q.y = vy; q.z = vz; q.w = dn;
+      reinterpret_cast<typename Vec4<T>::type*>(geom)[base * nr + k] = q;
+    }
+    if (gsc) {
+      // scalar radial derivatives: der2b = s2 * v/|v|, der3bsupp = s3 * v/|v|
+      typename Vec2<T>::type q;
+      q.x = s2; q.y = s3;
+      reinterpret_cast<typename Vec2<T>::type*>(gsc)[base * nr + k] = q;
+    }
   }
   const T inv = valid ? T(1) / dn : T(0);
   sv.ux = vx * inv; sv.uy = vy * inv; sv.uz = vz * inv; sv.fc = d3;
@@ -463,113 +498,137 @@ __device__ __forceinline__ void record_header(const RowSink& sk, size_t row, int
   }
 }
 
+// Shared memory of one warp of k_nl_radial: nr4 keys (nr rounded up to four, then a key of padding), two index rows
+// and the candidate list.
+constexpr int NL_CAND = 384;  // candidates listed at a time (27 cells hold about 300 atoms in liquid water)
+template <class T>
+__host__ __device__ inline int nl_warp_bytes(int nr) {
+  const int nr4 = (nr + 3) & ~3;
+  return nr4 * (int)sizeof(T) + 2 * nr4 * 4 + NL_CAND * 4;
+}
+
 // One warp per central atom: candidate discovery over the 27 neighbour cells in the
 // reference's visiting order (x outer, y, z inner, offsets -1,0,1: celle_gpu.cu.cc:61-82),
 // stable sort by dist2 (celle_gpu.cu.cc:128-152), then the radial descriptor row
-// (reforce.cu.cc:17-110).
-template <class T, int WARPS>
+// (reforce.cu.cc:17-110).  Bound by instruction issue at large sizes: 3,000 warp instructions per atom when every
+// candidate found its cell by bisection and its position through an index, the sort compared keys one by one with
+// their tie rule and the record path formed the operators' gradient vectors too; about half of that now.
+template <class T, int WARPS, bool OPS>
 __global__ void __launch_bounds__(WARPS * 32)
     k_nl_radial(int nf, int N, int ncen, int nr, CoreCoef<T> cc, const FrameGeom<T>* __restrict__ fg,
                 const T* __restrict__ frac, const int* __restrict__ cell_of, const int* __restrict__ cell_start,
-                const int* __restrict__ cells_sorted, int cell_cap, T* __restrict__ raddescr,
+                const typename Vec4<T>::type* __restrict__ cxyz, int cell_cap, T* __restrict__ raddescr,
                 T* __restrict__ des3bsupp, int* __restrict__ intmap2b, T* __restrict__ der2b,
                 T* __restrict__ der3bsupp, int* __restrict__ numtriplet, T* __restrict__ geom, T* __restrict__ gsc,
                 int na, int* __restrict__ status, RowSink sink) {
-  extern __shared__ unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  typedef typename Vec4<T>::type T4;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gi = blockIdx.x * WARPS + warp;  // row index: the centres are the first ncen atoms of each frame
   if (gi >= nf * ncen) return;
   chain_wait();  // the cell lists come from the kernel just before this one
-  const int b = gi / ncen, i = gi - b * ncen;
-  // per-warp rows: d2a[nr] d2b[nr] (T) then ja[nr] jb[nr] (int)
-  T* d2a = reinterpret_cast<T*>(smem_raw) + (size_t)warp * 2 * nr;
-  T* d2b = d2a + nr;
-  int* ja = reinterpret_cast<int*>(reinterpret_cast<T*>(smem_raw) + (size_t)WARPS * 2 * nr) + (size_t)warp * 2 * nr;
-  int* jb = ja + nr;
+  const int b = gi / ncen, i = gi - b * ncen, nr4 = (nr + 3) & ~3;
+  T* d2a = reinterpret_cast<T*>(smem_raw + (size_t)warp * nl_warp_bytes<T>(nr));  // [nr4] squared distances
+  int* ja = reinterpret_cast<int*>(d2a + nr4);  // [nr4] neighbours in order of discovery
+  int* jb = ja + nr4;                           // [nr4] sorted
+  int* cand = jb + nr4;                         // [NL_CAND] candidates' places in the cell-ordered atoms
 
   const FrameGeom<T> g = fg[b];
   const T* fr = frac + (size_t)b * N * 3;
+  const T4* cx4 = cxyz + (size_t)b * N;
   const T pix = fr[3 * i], piy = fr[3 * i + 1], piz = fr[3 * i + 2];
   const int ci = cell_of[(size_t)b * N + i];
   const int cz = ci / (g.nx * g.ny), rem = ci - cz * (g.nx * g.ny), cy = rem / g.nx, cx = rem - cy * g.nx;
   const int* cst = cell_start + (size_t)b * (cell_cap + 1);
-  const int* cl = cells_sorted + (size_t)b * N;
   const T cut2 = cc.Rc * cc.Rc;
   const unsigned lt = (1u << lane) - 1u;
-  // The 27 neighbour cells in the reference's visiting order, flattened into one candidate list so
-  // that all 32 lanes work on every pass: lane q < 27 owns cell q, an inclusive scan gives each cell's
-  // offset in the list, and a candidate finds its cell by bisection.
-  int* cbeg = reinterpret_cast<int*>(reinterpret_cast<int*>(reinterpret_cast<T*>(smem_raw) + (size_t)WARPS * 2 * nr) +
-                                     (size_t)WARPS * 2 * nr) + warp * 64;  // [32] cell starts, [32] list offsets
-  int* coff = cbeg + 32;
-  {
-    int s0 = 0, cn = 0;
-    if (lane < 27) {
-      const int di = lane / 9 - 1, dj = (lane / 3) % 3 - 1, dk = lane % 3 - 1;
-      int bi = cx + di, bj = cy + dj, bk = cz + dk;
-      if (bi < 0) bi = g.nx - 1; else if (bi == g.nx) bi = 0;
-      if (bj < 0) bj = g.ny - 1; else if (bj == g.ny) bj = 0;
-      if (bk < 0) bk = g.nz - 1; else if (bk == g.nz) bk = 0;
-      const int c = bi + bj * g.nx + bk * g.nx * g.ny;
-      s0 = cst[c];
-      cn = cst[c + 1] - s0;
-    }
-    int x = cn;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    cbeg[lane] = s0;
-    coff[lane] = x - cn;  // exclusive offset; lanes >= 27 hold the total
+  // The 27 neighbour cells in the reference's visiting order: lane q < 27 owns cell q and an inclusive scan gives the
+  // place of its members in the list of candidates, which the lanes write NL_CAND at a time.
+  int s0 = 0, cn = 0;
+  if (lane < 27) {
+    const int di = lane / 9 - 1, dj = (lane / 3) % 3 - 1, dk = lane % 3 - 1;
+    int bi = cx + di, bj = cy + dj, bk = cz + dk;
+    if (bi < 0) bi = g.nx - 1; else if (bi == g.nx) bi = 0;
+    if (bj < 0) bj = g.ny - 1; else if (bj == g.ny) bj = 0;
+    if (bk < 0) bk = g.nz - 1; else if (bk == g.nz) bk = 0;
+    const int c = bi + bj * g.nx + bk * g.nx * g.ny;
+    s0 = cst[c];
+    cn = cst[c + 1] - s0;
   }
-  __syncwarp();
-  const int M = coff[27];
-  int count = 0;
-  for (int e0 = 0; e0 < M; e0 += 32) {
-    const int e = e0 + lane;
-    bool pred = false;
-    int j = -1;
-    T dist2 = T(0);
-    if (e < M) {
-      int q = 0;
+  int x = cn;
 #pragma unroll
-      for (int st = 16; st > 0; st >>= 1)
-        if (q + st < 27 && coff[q + st] <= e) q += st;
-      j = cl[cbeg[q] + (e - coff[q])];
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  const int M = __shfl_sync(0xffffffffu, x, 31), coff = x - cn;
+  int count = 0;
+  for (int w0 = 0; w0 < M; w0 += NL_CAND) {
+    __syncwarp();
+    const int q0 = max(w0 - coff, 0), q1 = min(cn, w0 + NL_CAND - coff);
+    for (int q = q0; q < q1; q++) cand[coff + q - w0] = s0 + q;
+    __syncwarp();
+    const int wn = min(M - w0, NL_CAND);
+    T4 v;
+    if (lane < wn) v = cx4[cand[lane]];
+    for (int e0 = 0; e0 < wn; e0 += 32) {
+      const int e = e0 + lane;
+      const T4 u = v;
+      if (e + 32 < wn) v = cx4[cand[e + 32]];  // the next candidate is on its way while this one is tested
+      const int j = entry_index(u);
       T dx, dy, dz;
-      mic_vec(g, fr[3 * j], fr[3 * j + 1], fr[3 * j + 2], pix, piy, piz, dx, dy, dz);
-      dist2 = dx * dx + dy * dy + dz * dz;
-      pred = (dist2 < cut2) && (j != i);
+      mic_vec(g, u.x, u.y, u.z, pix, piy, piz, dx, dy, dz);
+      const T dist2 = dx * dx + dy * dy + dz * dz;
+      const bool pred = (e < wn) && (dist2 < cut2) && (j != i);
+      const unsigned bal = __ballot_sync(0xffffffffu, pred);
+      const int slot = count + __popc(bal & lt);
+      if (pred && slot < nr) {
+        d2a[slot] = dist2;
+        ja[slot] = j;
+      }
+      count += __popc(bal);
     }
-    const unsigned bal = __ballot_sync(0xffffffffu, pred);
-    const int slot = count + __popc(bal & lt);
-    if (pred && slot < nr) {
-      d2a[slot] = dist2;
-      ja[slot] = j;
-    }
-    count += __popc(bal);
   }
   if (count > nr && lane == 0) set_status(status, STAFB_ERR_RADIAL_OVERFLOW);
   const int n = count < nr ? count : nr;
+  if (n + lane < nr4 && lane < 4) d2a[n + lane] = T(3e38);
+  for (int k = lane; k < n; k += 32) jb[k] = -1;
   __syncwarp();
-  // stable rank sort: position = #{f : d2[f] < d2[e] or (equal and f < e)}
-  for (int e = lane; e < n; e += 32) {
-    const T key = d2a[e];
-    int r = 0;
-    for (int f = 0; f < n; f++) {
-      const T kf = d2a[f];
-      r += (kf < key) || (kf == key && f < e);
+  // Rank sort, two keys per lane against four keys per load: position = #{f : d2[f] < d2[e]}.  Equal distances collide
+  // in one place and leave another empty; then (rare) the ranks are formed again with the stable rule
+  // #{f : d2[f] < d2[e] or (equal and f < e)}.
+  for (int e0 = 0; e0 < n; e0 += 64) {
+    const int ea = e0 + lane, eb = ea + 32;
+    const T ka = ea < n ? d2a[ea] : T(0), kb = eb < n ? d2a[eb] : T(0);
+    int ra = 0, rb = 0;
+    for (int f = 0; f < n; f += 4) {
+      const T4 kf = *reinterpret_cast<const T4*>(d2a + f);
+      ra += (kf.x < ka) + (kf.y < ka) + (kf.z < ka) + (kf.w < ka);
+      rb += (kf.x < kb) + (kf.y < kb) + (kf.z < kb) + (kf.w < kb);
     }
-    d2b[r] = key;
-    jb[r] = ja[e];
+    if (ea < n) jb[ra] = ja[ea];
+    if (eb < n) jb[rb] = ja[eb];
+  }
+  __syncwarp();
+  bool hole = false;
+  for (int k = lane; k < n; k += 32) hole |= jb[k] < 0;
+  if (__any_sync(0xffffffffu, hole)) {
+    for (int e = lane; e < n; e += 32) {
+      const T key = d2a[e];
+      int r = 0;
+      for (int f = 0; f < n; f++) {
+        const T kf = d2a[f];
+        r += (kf < key) || (kf == key && f < e);
+      }
+      jb[r] = ja[e];
+    }
   }
   __syncwarp();
   const size_t base = (size_t)gi;
   int cnt[STAFB_MAX_TYPES];
   if (sink.rows) group_by_species(sink, jb, n, lane, ja, cnt);  // ja[] is free after the sort
   int nang = 0;
-  for (int k = lane; k < nr; k += 32) {
+  for (int k = lane; k < (OPS ? nr : n); k += 32) {
     T vx = T(0), vy = T(0), vz = T(0);
     int j = 0;
     if (k < n) {
@@ -577,15 +636,15 @@ __global__ void __launch_bounds__(WARPS * 32)
       mic_vec(g, pix, piy, piz, fr[3 * j], fr[3 * j + 1], fr[3 * j + 2], vx, vy, vz);
     }
     SlotVals<T> sv;
-    radial_slot<T>(cc, k < n, j, vx, vy, vz, base, k, nr, raddescr, des3bsupp, intmap2b, der2b, der3bsupp, geom, gsc,
-                   nang, sv);
+    radial_slot<T, OPS>(cc, k < n, j, vx, vy, vz, base, k, nr, raddescr, des3bsupp, intmap2b, der2b, der3bsupp, geom,
+                        gsc, nang, sv);
     if (sink.rows && k < n) record_slot<T>(sink, base, nr, ja[k] & 0xffff, j, sv);
   }
   nang = warp_sum(nang);
   if (sink.rows) record_header(sink, base, nr, (int)sizeof(T), ja, n, nang, cnt, lane);
   if (lane == 0) {
-    if (intmap2b) intmap2b[base * (nr + 1)] = n;
-    if (numtriplet) numtriplet[base] = nang;
+    if (OPS && intmap2b) intmap2b[base * (nr + 1)] = n;
+    if (OPS && numtriplet) numtriplet[base] = nang;
     if ((long long)nang * (nang - 1) / 2 > na) set_status(status, STAFB_ERR_ANGULAR_OVERFLOW);
   }
 }
@@ -639,7 +698,7 @@ __global__ void __launch_bounds__(WARPS * 32)
   for (int k = lane; k < n; k += 32) {
     const int j = ids[k];
     SlotVals<T> sv;
-    radial_slot<T>(cc, true, j, pix - pos[3 * j], piy - pos[3 * j + 1], piz - pos[3 * j + 2], base, k, nr,
+    radial_slot<T, false>(cc, true, j, pix - pos[3 * j], piy - pos[3 * j + 1], piz - pos[3 * j + 2], base, k, nr,
                    (T*)nullptr, (T*)nullptr, (int*)nullptr, (T*)nullptr, (T*)nullptr, (T*)nullptr, (T*)nullptr, nang,
                    sv);
     record_slot<T>(sink, base, nr, spos[k] & 0xffff, j, sv);
@@ -724,6 +783,7 @@ int launch_descriptors(stafb_ctx* c, cudaStream_t s, const T* pos, const T* box,
   if (nf > c->max_batch || N > c->n_max) return STAFB_ERR_CAPACITY;
   if (ncen < 0) ncen = N;  // every atom is a centre unless the caller restricts the rows to the first ncen
   if (ncen > N) return STAFB_ERR_INVALID;
+  c->status_fresh = 0;
   const int nr = c->nr, na = c->na, cap = c->cell_cap;
   FrameGeom<T>* fg = reinterpret_cast<FrameGeom<T>*>(c->fgeom);
   T* frac = reinterpret_cast<T*>(c->frac);
@@ -742,40 +802,41 @@ int launch_descriptors(stafb_ctx* c, cudaStream_t s, const T* pos, const T* box,
   cc.Rc = (T)c->Rc; cc.Rs = (T)c->Rs; cc.Ra = (T)c->Ra;
   cc.A = (T)c->coef[0]; cc.B = (T)c->coef[1]; cc.C = (T)c->coef[2]; cc.pa = (T)c->coef[3]; cc.pb = (T)c->coef[4];
   const int tot = nf * N;
-  const size_t small_sm = sizeof(int) * ((size_t)cap + 1 + N);
-  if (small_sm <= 48 * 1024 && N <= 2048) {
-    k_cell_lists_small<T><<<nf, 1024, small_sm, s>>>(pos, box, N, cc.Rc, cap, mpc, fg, frac, c->cell_of, c->cell_start,
-                                                    c->cells_sorted, c->status_d);
+  typedef typename Vec4<T>::type T4;
+  T4* cxyz = reinterpret_cast<T4*>(c->cxyz);
+  const size_t small_sm = sizeof(int) * ((size_t)cap + 1 + 2 * N);
+  if (small_sm <= 48 * 1024 && N <= CELLS_SMALL_MAX) {
+    const int threads = N >= 1024 ? 1024 : ((N + 31) & ~31);
+    STAFB_CUDA_OK(launch_chained(k_cell_lists_small<T>, nf, threads, small_sm, s, pos, box, N, cc.Rc, cap, mpc, fg, frac,
+                                 c->cell_of, c->cell_start, cxyz, c->status_d));
+    c->launches += 1;
+  } else if (N <= CELLS_CLUSTER_MAX) {
+    STAFB_CUDA_OK(launch_chained(k_cell_lists_cluster<T>, nf * CELLS_CLUSTER, 1024, 0, s, pos, box, N, cc.Rc, cap, mpc,
+                                 fg, frac, c->cell_of, c->cell_count, c->cell_start, c->cell_cursor, c->cells_raw, cxyz,
+                                 c->status_d));
     c->launches += 1;
   } else {
     STAFB_CUDA_OK(cudaMemsetAsync(c->cell_count, 0, sizeof(int) * (size_t)nf * cap, s));
     // each of these needs all of its predecessor's output: chained launches only save the launch gaps
     STAFB_CUDA_OK(launch_chained(k_cells<T>, dim3((N + 255) / 256, nf), 256, 0, s, pos, box, nf, N, cc.Rc, cap, fg,
-                                 frac, c->cell_of, c->cell_count, c->status_d));
+                                 frac, c->cell_of, c->cell_count, c->cell_cursor, c->status_d));
     STAFB_CUDA_OK(launch_chained(k_scan<T>, nf, 1024, 0, s, (const FrameGeom<T>*)fg, (const int*)c->cell_count,
-                                 c->cell_start, c->cell_cursor, cap, mpc, c->status_d));
-    const long long warps = (long long)nf * cap;
-    if (N <= 4096) {
-      STAFB_CUDA_OK(launch_chained(k_gather_cells<T>, (unsigned)((warps * 32 + 255) / 256), 256, 0, s,
-                                   (const FrameGeom<T>*)fg, nf, N, (const int*)c->cell_of, (const int*)c->cell_start,
-                                   c->cells_sorted, cap));
-      c->launches += 4;
-    } else {
-      STAFB_CUDA_OK(launch_chained(k_fill, (tot + 255) / 256, 256, 0, s, nf, N, (const int*)c->cell_of,
-                                   (const int*)c->cell_start, c->cell_cursor, c->cells_raw, cap));
-      STAFB_CUDA_OK(launch_chained(k_sort_cells<T>, (unsigned)((warps * 32 + 255) / 256), 256, 0, s,
-                                   (const FrameGeom<T>*)fg, nf, N, (const int*)c->cell_start, (const int*)c->cells_raw,
-                                   c->cells_sorted, cap));
-      c->launches += 5;
-    }
+                                 c->cell_start, cap, mpc, c->status_d));
+    STAFB_CUDA_OK(launch_chained(k_fill, (tot + 255) / 256, 256, 0, s, nf, N, (const int*)c->cell_of,
+                                 (const int*)c->cell_start, (const int*)c->cell_cursor, c->cells_raw, cap));
+    STAFB_CUDA_OK(launch_chained(k_order_cells<T>, (tot + 255) / 256, 256, 0, s, nf, N, (const int*)c->cell_of,
+                                 (const int*)c->cell_start, (const int*)c->cells_raw, (const T*)frac, cxyz, cap));
+    c->launches += 5;
   }
   {
     constexpr int W = 4;
-    size_t sm = (size_t)W * 2 * nr * (sizeof(T) + sizeof(int)) + (size_t)W * 64 * sizeof(int);
+    const size_t sm = (size_t)W * nl_warp_bytes<T>(nr);
     const int rows = nf * ncen;
-    STAFB_CUDA_OK(launch_chained(k_nl_radial<T, W>, (rows + W - 1) / W, W * 32, sm, s, nf, N, ncen, nr, cc, fg, frac,
-                                 c->cell_of, c->cell_start, c->cells_sorted, cap, raddescr, des3bsupp, intmap2b, der2b,
-                                 der3bsupp, numtriplet, geom, gsc, na, c->status_d, sk));
+    // the operators' outputs or the records of the fused sweeps alone
+    auto kern = raddescr || intmap2b ? k_nl_radial<T, W, true> : k_nl_radial<T, W, false>;
+    STAFB_CUDA_OK(launch_chained(kern, (rows + W - 1) / W, W * 32, sm, s, nf, N, ncen, nr, cc, fg, frac, c->cell_of,
+                                 c->cell_start, cxyz, cap, raddescr, des3bsupp, intmap2b, der2b, der3bsupp, numtriplet,
+                                 geom, gsc, na, c->status_d, sk));
   }
   c->launches += 1;
   if (want_angular) {
@@ -799,6 +860,7 @@ int launch_rows_from_list(stafb_ctx* c, cudaStream_t s, const T* pos, int ncen, 
                           const int* with, const RowSink* sink) {
   if (ncen <= 0 || nall < ncen || !howmany || !with || !sink || !sink->rows) return STAFB_ERR_INVALID;
   if (nall > c->n_max) return STAFB_ERR_CAPACITY;
+  c->status_fresh = 0;
   CoreCoef<T> cc;
   cc.Rc = (T)c->Rc; cc.Rs = (T)c->Rs; cc.Ra = (T)c->Ra;
   cc.A = (T)c->coef[0]; cc.B = (T)c->coef[1]; cc.C = (T)c->coef[2]; cc.pa = (T)c->coef[3]; cc.pb = (T)c->coef[4];
@@ -845,8 +907,8 @@ constexpr size_t NA_OFF_COUNT = NA_OFF_CELLOF + al256(sizeof(int) * NOALLOC_MAX_
 constexpr size_t NA_OFF_START = NA_OFF_COUNT + al256(sizeof(int) * NOALLOC_MAX_CELLS);
 constexpr size_t NA_OFF_CURSOR = NA_OFF_START + al256(sizeof(int) * (NOALLOC_MAX_CELLS + NOALLOC_MAX_FRAMES));
 constexpr size_t NA_OFF_RAW = NA_OFF_CURSOR + al256(sizeof(int) * NOALLOC_MAX_CELLS);
-constexpr size_t NA_OFF_SORTED = NA_OFF_RAW + al256(sizeof(int) * NOALLOC_MAX_ATOMS);
-constexpr size_t NA_OFF_GEOM = NA_OFF_SORTED + al256(sizeof(int) * NOALLOC_MAX_ATOMS);
+constexpr size_t NA_OFF_CXYZ = NA_OFF_RAW + al256(sizeof(int) * NOALLOC_MAX_ATOMS);
+constexpr size_t NA_OFF_GEOM = NA_OFF_CXYZ + al256(sizeof(double) * 4 * NOALLOC_MAX_ATOMS);
 constexpr size_t NA_OFF_GSC = NA_OFF_GEOM + al256(sizeof(double) * 4 * NOALLOC_MAX_ATOMS * NOALLOC_MAX_NR);
 constexpr size_t NA_OFF_STATUS = NA_OFF_GSC + al256(sizeof(double) * 2 * NOALLOC_MAX_ATOMS * NOALLOC_MAX_NR);
 constexpr size_t NA_TOTAL = NA_OFF_STATUS + 256;
@@ -908,7 +970,7 @@ extern "C" int stafb_compute_descriptors_light_noalloc(int dtype, double radial_
   c.cell_start = reinterpret_cast<int*>(base + NA_OFF_START);
   c.cell_cursor = reinterpret_cast<int*>(base + NA_OFF_CURSOR);
   c.cells_raw = reinterpret_cast<int*>(base + NA_OFF_RAW);
-  c.cells_sorted = reinterpret_cast<int*>(base + NA_OFF_SORTED);
+  c.cxyz = base + NA_OFF_CXYZ;
   c.geom = base + NA_OFF_GEOM;
   c.gsc = base + NA_OFF_GSC;
   c.status_d = reinterpret_cast<int*>(base + NA_OFF_STATUS);
