@@ -95,9 +95,10 @@ extern "C" int stafb_create(stafb_ctx** out, int dtype, double Rc, double Rs, do
   STAFB_CUDA_OK(cudaMalloc(&c->frac, es * B * Nn * 3));
   STAFB_CUDA_OK(cudaMalloc((void**)&c->cell_of, sizeof(int) * B * Nn));
   STAFB_CUDA_OK(cudaMalloc((void**)&c->cell_count, sizeof(int) * B * c->cell_cap));
-  STAFB_CUDA_OK(cudaMalloc((void**)&c->cell_start, sizeof(int) * B * (c->cell_cap + 1)));
-  STAFB_CUDA_OK(cudaMalloc((void**)&c->cell_cursor, sizeof(int) * B * c->cell_cap));
-  STAFB_CUDA_OK(cudaMalloc((void**)&c->cells_raw, sizeof(int) * B * Nn));
+  STAFB_CUDA_OK(cudaMemset(c->cell_count, 0, sizeof(int) * B * c->cell_cap));
+  STAFB_CUDA_OK(cudaMalloc(&c->cell_range, sizeof(int2) * B * c->cell_cap));
+  STAFB_CUDA_OK(cudaMalloc((void**)&c->cell_slot, sizeof(int) * B * Nn));
+  STAFB_CUDA_OK(cudaMalloc((void**)&c->cell_total, sizeof(int) * B));
   STAFB_CUDA_OK(cudaMalloc(&c->cxyz, es * B * Nn * 4));
   STAFB_CUDA_OK(cudaMalloc(&c->geom, es * B * Nn * nr * 4));
   STAFB_CUDA_OK(cudaMalloc(&c->gsc, es * B * Nn * nr * 2));
@@ -115,7 +116,7 @@ extern "C" void stafb_destroy(stafb_ctx* c) {
   cudaGetDevice(&cur);
   cudaSetDevice(c->device);
   cudaFree(c->fgeom); cudaFree(c->frac); cudaFree(c->cell_of); cudaFree(c->cell_count);
-  cudaFree(c->cell_start); cudaFree(c->cell_cursor); cudaFree(c->cells_raw); cudaFree(c->cxyz);
+  cudaFree(c->cell_range); cudaFree(c->cell_slot); cudaFree(c->cell_total); cudaFree(c->cxyz);
   cudaFree(c->geom); cudaFree(c->gsc); cudaFree(c->status_d);
   cudaFreeHost(c->status_h);
   for (int q = 0; q < 16; q++)

@@ -164,11 +164,11 @@ struct stafb_ctx {
   void* fgeom;        // FrameGeom<T>[max_batch]
   void* frac;         // T[max_batch, n_max, 3]
   int* cell_of;       // [max_batch, n_max]
-  int* cell_count;    // [max_batch, cell_cap]
-  int* cell_start;    // [max_batch, cell_cap+1]
-  int* cell_cursor;   // [max_batch, cell_cap] arrival slots of the atoms inside their cells
-  int* cells_raw;     // [max_batch, n_max] atoms by cell in arrival order
-  void* cxyz;         // T[max_batch, n_max, 4] atoms by cell in ascending index: fractional coordinates, index
+  int* cell_count;    // [max_batch, cell_cap] zero between calls
+  void* cell_range;   // int2[max_batch, cell_cap] first place and number of a cell's members in cxyz
+  int* cell_slot;     // [max_batch, n_max] arrival slots of the atoms inside their cells
+  int* cell_total;    // [max_batch]
+  void* cxyz;         // T[max_batch, n_max, 4] atoms by cell: fractional coordinates, index
   void* geom;         // T[max_batch, n_max, nr, 4]: MIC vector r_i - r_j and its norm, sorted order
   void* gsc;          // T[max_batch, n_max, nr, 2]: d(raddescr)/dr and d(des3bsupp)/dr
   int* status_d;

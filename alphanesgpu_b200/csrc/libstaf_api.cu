@@ -37,7 +37,7 @@ struct StafModel {
   // Per-call staging.  The caller's arrays are copied as they are, in the caller's order, into pinned memory that the
   // device reads and writes directly (k_stage_in, k_stage_list, k_stage_out: conversion, permutation to slot order
   // and the slot numbers of the neighbours all happen there), so there are no copy-engine transfers:
-  //   xin_h : x[3*nall] | box[6]        list_h : howmany[nlocal] | rows[nlocal][nr]
+  //   xin_h : x[3*nall] | box[6]        list_h : entries in all | howmany[nlocal] | rows, packed
   //   fout_h: f[3*nall] | energy | virial[9] | bad list entry + 1 (0: none)
   // Device blocks in the computing precision and in slot order (stage_layout):
   //   in_d  : pos[3*cap] | box[6] | type_map[cap] | howmany[cap] | with[cap*nr]
@@ -45,6 +45,7 @@ struct StafModel {
   char *in_d, *out_d;
   double *xin_h, *fout_h;
   int *list_h, *tmap_h;
+  int* list_d;  // device copy of list_h
   int* slot_d;  // to_slot on the device
   size_t in_bytes, out_bytes;
   cudaStream_t stream;
@@ -136,7 +137,7 @@ static void release_device(StafModel* m) {
   if (m->ctx) stafb_destroy(m->ctx);
   m->model = nullptr;
   m->ctx = nullptr;
-  void* dv[] = {m->theta_d, m->emb_d, m->in_d, m->out_d, m->slot_d};
+  void* dv[] = {m->theta_d, m->emb_d, m->in_d, m->out_d, m->slot_d, m->list_d};
   for (void* q : dv) if (q) cudaFree(q);
   void* hv[] = {m->xin_h, m->fout_h, m->list_h, m->tmap_h};
   for (void* q : hv) if (q) cudaFreeHost(q);
@@ -144,7 +145,7 @@ static void release_device(StafModel* m) {
   m->in_d = m->out_d = nullptr;
   m->xin_h = m->fout_h = nullptr;
   m->list_h = m->tmap_h = nullptr;
-  m->slot_d = nullptr;
+  m->slot_d = m->list_d = nullptr;
   m->type_prev.clear();
   m->nlocal_prev = -1;
   m->cap_n = 0;
@@ -164,7 +165,7 @@ extern "C" StafModel* staf_load(const char* model_dir, const StafOptions* opt) {
   m->in_d = m->out_d = nullptr;
   m->xin_h = m->fout_h = nullptr;
   m->list_h = m->tmap_h = nullptr;
-  m->slot_d = nullptr;
+  m->slot_d = m->list_d = nullptr;
   m->nlocal_prev = -1;
   m->type_prev_null = 0;
   m->stream = nullptr;
@@ -303,9 +304,18 @@ static int ensure_device(StafModel* m, int nall, const std::vector<int>& tipos) 
 
 // Caller order, double -> slot order, computing precision (positions and box), and back (forces, energy, virial).
 // xin and fout are pinned host memory: every word crosses PCIe once, in full lines.
+// list_h (null: none): the packed neighbour rows, brought over as they are by the blocks behind those of the atoms,
+// 16 bytes per thread.  (k_stage_list reading them in place took 82 us for 2,997 rows of 150 bytes: partial lines.)
 template <class T>
 __global__ void k_stage_in(int nall, const double* __restrict__ xin, const int* __restrict__ slot, T* __restrict__ pos,
-                           T* __restrict__ box) {
+                           T* __restrict__ box, int atom_blocks, const int4* __restrict__ list_h, int4* __restrict__ list_d) {
+  if ((int)blockIdx.x >= atom_blocks) {
+    const int words = (list_h[0].x + 3) >> 2;  // list_h[0].x: ints in all, this one included
+    for (int q = (blockIdx.x - atom_blocks) * blockDim.x + threadIdx.x; q < words;
+         q += (gridDim.x - atom_blocks) * blockDim.x)
+      list_d[q] = list_h[q];
+    return;
+  }
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q < 3 * nall) {
     const int i = q / 3, c = q - 3 * i;
@@ -326,16 +336,15 @@ __global__ void k_stage_out(int nall, const T* __restrict__ force, const T* __re
 }
 
 // The caller's neighbour rows -> slot order and slot numbers (staf_api.cpp:304-347), one warp per centre.  An entry
-// outside [0, nall) is reported in *bad (entry + 1) and becomes -1.  how / rows: pinned host memory.  On the host this
-// was 38 random reads per atom, 100 of the 390 us of a 2,997-atom call.
-__global__ void k_stage_list(int nlocal, int nall, int nr, const int* __restrict__ how, const int* __restrict__ rows,
-                             const int* __restrict__ slot, int* __restrict__ how_d, int* __restrict__ with_d,
-                             double* __restrict__ bad) {
+// outside [0, nall) is reported in *bad (entry + 1) and becomes -1.  list: number of ints | per centre the end of its
+// row | rows.  On the host this was 38 random reads per atom, 100 of the 390 us of a 2,997-atom call.
+__global__ void k_stage_list(int nlocal, int nall, int nr, const int* __restrict__ list, const int* __restrict__ slot,
+                             int* __restrict__ how_d, int* __restrict__ with_d, double* __restrict__ bad) {
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= nlocal) return;
-  const int n = how[i], sl = slot[i];
+  const int beg = i == 0 ? 1 + nlocal : list[i], n = list[1 + i] - beg, sl = slot[i];
   for (int k = lane; k < n; k += 32) {
-    const int j = rows[(size_t)i * nr + k];
+    const int j = list[beg + k];
     const bool ok = j >= 0 && j < nall;
     if (!ok) *bad = (double)j + (j >= 0 ? 1.0 : 0.0);
     with_d[(size_t)sl * nr + k] = ok ? slot[j] : -1;
@@ -397,25 +406,30 @@ static int compute_impl(StafModel* m, int nlocal, int nghost, const double* x, c
   double* bad = m->fout_h + 3 * (size_t)nall + 10;
   *bad = 0.0;
   if (howmany) {
-    if (!m->list_h &&
-        cudaMallocHost((void**)&m->list_h, sizeof(int) * (size_t)m->cap_n * (size_t)(1 + nr)) != cudaSuccess)
+    const size_t ints = (size_t)m->cap_n * (size_t)(1 + nr) + 4;
+    if (!m->list_h && (cudaMallocHost((void**)&m->list_h, sizeof(int) * ints) != cudaSuccess ||
+                       cudaMalloc((void**)&m->list_d, sizeof(int) * ints) != cudaSuccess))
       return -14;
-    int *how_h = m->list_h, *rows_h = m->list_h + m->cap_n;
+    int o = 1 + nlocal;
     for (int i = 0; i < nlocal; i++) {
       int nn = howmany[i];
       if (nn < 0) nn = 0;
       if (nn > nr) nn = nr;
       if (nn > maxneigh) nn = maxneigh;
-      how_h[i] = nn;
-      memcpy(rows_h + (size_t)i * nr, with + (size_t)i * maxneigh, sizeof(int) * (size_t)nn);
+      memcpy(m->list_h + o, with + (size_t)i * maxneigh, sizeof(int) * (size_t)nn);
+      o += nn;
+      m->list_h[1 + i] = o;
     }
+    m->list_h[0] = o;
   }
   const int nb = (3 * nall + 255) / 256;
   auto enqueue = [&]() -> int {
-    k_stage_in<T><<<nb, 256, 0, s>>>(nall, m->xin_h, m->slot_d, reinterpret_cast<T*>(m->in_d + L.pos),
-                                     reinterpret_cast<T*>(m->in_d + L.box));
+    const int lb = howmany ? (nlocal * (1 + nr) / 4 + 255) / 256 : 0;
+    k_stage_in<T><<<nb + lb, 256, 0, s>>>(nall, m->xin_h, m->slot_d, reinterpret_cast<T*>(m->in_d + L.pos),
+                                          reinterpret_cast<T*>(m->in_d + L.box), nb,
+                                          reinterpret_cast<const int4*>(m->list_h), reinterpret_cast<int4*>(m->list_d));
     if (howmany)
-      k_stage_list<<<(nlocal + 7) / 8, 256, 0, s>>>(nlocal, nall, nr, m->list_h, m->list_h + m->cap_n, m->slot_d,
+      k_stage_list<<<(nlocal + 7) / 8, 256, 0, s>>>(nlocal, nall, nr, m->list_d, m->slot_d,
                                                     reinterpret_cast<int*>(m->in_d + L.how),
                                                     reinterpret_cast<int*>(m->in_d + L.with), bad);
     const int rc = stafb_energy_force_domain(

@@ -11,6 +11,7 @@
 // cutoff tests must round in expression order, because neighbour sets and neighbour ORDER
 // are compared bit-exactly.
 #include <string.h>
+#include <type_traits>
 #include "common.cuh"
 
 namespace stafb {
@@ -96,61 +97,47 @@ __device__ __forceinline__ int place_atom(const FrameGeom<T>& g, const T* __rest
   return cx + cy * g.nx + cz * (g.nx * g.ny);
 }
 
-// Rank of atom i among the members of its cell, src[s0, s1): the reference's slot order is the atomicAdd arrival order
-// (celle_gpu.cu.cc:197-200), restated as ascending atom index.
-__device__ __forceinline__ int cell_rank(const int* src, int s0, int s1, int i) {
-  int r = 0;
-  for (int f = s0; f < s1; f++) r += (src[f] < i);
-  return r;
-}
-
-// Exclusive scan of one value per thread over the block (warps <= 32); part: 33 ints of shared memory.  Returns the
-// exclusive prefix, total in `tot`.
-__device__ __forceinline__ int block_scan(int v, int* part, int& tot) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  int x = v;
+// Places for the members of the cells of one frame: a warp's cells share one atomic add on *total.  Which cell comes
+// first is left to chance; a cell's members are consecutive, and that is all that the search needs.
+__device__ __forceinline__ int cell_places(int count, int* total) {
+  const int lane = threadIdx.x & 31;
+  int x = count;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const int y = __shfl_up_sync(0xffffffffu, x, o);
     if (lane >= o) x += y;
   }
-  if (lane == 31) part[w] = x;
-  __syncthreads();
-  int off = 0, all = 0;
-  for (int q = 0; q < nw; q++) {
-    const int pq = part[q];
-    off += q < w ? pq : 0;
-    all += pq;
-  }
-  __syncthreads();
-  tot = all;
-  return off + x - v;
+  int base = 0;
+  if (lane == 31) base = atomicAdd(total, x);
+  return __shfl_sync(0xffffffffu, base, 31) + x - count;
 }
 
-// Frame geometry, fractional coordinates, cell counts, their scan and the atoms in cell order (ascending index inside
-// a cell) of one frame by one block, all bookkeeping in shared memory: up to CELLS_SMALL_MAX atoms.  Every atom is one
-// thread's in all passes: it takes its arrival slot from the counter, leaves its index there, and then ranks itself
-// among its cell's members (11 on average in liquid water), so no pass walks the frame.  Bound by the latency of its
-// four dependent passes and the barriers between them, hence no more threads than atoms.
-// Dynamic shared memory: (cell_cap + 1 + 2 N) ints.
+// The cell lists: where a cell's members lie (cell_range: first, number) among the atoms in cell order (cxyz).  Inside
+// a cell the members lie in the order in which they arrived; the reference's order there is its atomicAdd arrival
+// (celle_gpu.cu.cc:197-200), restated as ascending index - which the search restores where it matters, between
+// neighbours at bit-equal distance.  So no pass orders the members, and no scan orders the cells: three short passes
+// (count, places, fill), each bound by the latency of one or two dependent loads.
+//
+// One block per frame with all bookkeeping in shared memory, no more threads than atoms: up to CELLS_SMALL_MAX atoms.
+// Dynamic shared memory: (cell_cap + N) ints.
 constexpr int CELLS_SMALL_MAX = 2048;
 template <class T>
 __global__ void __launch_bounds__(1024)
     k_cell_lists_small(const T* __restrict__ pos, const T* __restrict__ box, int N, T cutoff, int cell_cap, int mpc,
                        FrameGeom<T>* __restrict__ fg, T* __restrict__ frac, int* __restrict__ cell_of,
-                       int* __restrict__ cell_start, typename Vec4<T>::type* __restrict__ cxyz,
+                       int2* __restrict__ cell_range, typename Vec4<T>::type* __restrict__ cxyz,
                        int* __restrict__ status) {
   extern __shared__ int sm_i[];
   __shared__ FrameGeom<T> gs;
-  __shared__ int part[33];
-  int* cnt = sm_i;                 // [cell_cap + 1] counts, then exclusive starts
-  int* raw = sm_i + cell_cap + 1;  // [N] atoms in arrival order
-  int* slot = raw + N;             // [N] arrival slot of an atom
+  __shared__ int total;
+  int* cnt = sm_i;              // [cell_cap] counts, then first places
+  int* slot = sm_i + cell_cap;  // [N] arrival slot of an atom
   const int b = blockIdx.x, tid = threadIdx.x;
   chain_wait();
   if (tid == 0) {
     frame_geometry<T>(box + 6 * b, N, cutoff, cell_cap, gs, status);
     fg[b] = gs;
+    total = 0;
   }
   __syncthreads();
   const FrameGeom<T>& g = gs;
@@ -167,107 +154,37 @@ __global__ void __launch_bounds__(1024)
     slot[i] = atomicAdd(&cnt[c], 1);
   }
   __syncthreads();
-  int* st = cell_start + (size_t)b * (cell_cap + 1);
-  int carry = 0;
   for (int base = 0; base < ncell; base += blockDim.x) {
     const int c = base + tid, v = (c < ncell) ? cnt[c] : 0;
     if (v > mpc) set_status(status, STAFB_ERR_CELL_OVERFLOW);
-    int tot;
-    const int x = carry + block_scan(v, part, tot);
-    if (c < ncell) cnt[c] = st[c] = x;
-    carry += tot;
+    const int x = cell_places(v, &total);
+    if (c < ncell) {
+      cnt[c] = x;
+      cell_range[(size_t)b * cell_cap + c] = make_int2(x, v);
+    }
   }
-  if (tid == 0) cnt[ncell] = st[ncell] = N;
   __syncthreads();
-  for (int i = tid; i < N; i += blockDim.x) raw[cnt[co[i]] + slot[i]] = i;
-  __syncthreads();
-  for (int i = tid; i < N; i += blockDim.x) {
-    const int c = co[i], s0 = cnt[c];
-    cxyz[(size_t)b * N + s0 + cell_rank(raw, s0, cnt[c + 1], i)] = cell_entry<T>(fr[3 * i], fr[3 * i + 1], fr[3 * i + 2], i);
-  }
+  for (int i = tid; i < N; i += blockDim.x)
+    cxyz[(size_t)b * N + cnt[co[i]] + slot[i]] = cell_entry<T>(fr[3 * i], fr[3 * i + 1], fr[3 * i + 2], i);
 }
 
-// The same for frames of up to CELLS_CLUSTER_MAX atoms by a cluster of eight blocks: counters and lists in global
-// memory (they stay in L2), a cluster barrier between the passes.  24,576 atoms: one launch of 9 us where a memset
-// and four kernels took 33 us, nearly all of it launch gaps and one wave each of a few loads.
-constexpr int CELLS_CLUSTER = 8;
-constexpr int CELLS_CLUSTER_MAX = 65536;
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-template <class T>
-__global__ void __cluster_dims__(CELLS_CLUSTER, 1, 1) __launch_bounds__(1024)
-    k_cell_lists_cluster(const T* __restrict__ pos, const T* __restrict__ box, int N, T cutoff, int cell_cap, int mpc,
-                         FrameGeom<T>* __restrict__ fg, T* __restrict__ frac, int* __restrict__ cell_of,
-                         int* __restrict__ cell_count, int* __restrict__ cell_start, int* __restrict__ slot_all,
-                         int* __restrict__ raw_all, typename Vec4<T>::type* __restrict__ cxyz, int* __restrict__ status) {
-  __shared__ FrameGeom<T> gs;
-  __shared__ int part[33];
-  const int b = blockIdx.x / CELLS_CLUSTER, rank = blockIdx.x % CELLS_CLUSTER;
-  const int tid = threadIdx.x, gt = rank * 1024 + tid, GT = CELLS_CLUSTER * 1024;
-  chain_wait();
-  if (tid == 0) {
-    frame_geometry<T>(box + 6 * b, N, cutoff, cell_cap, gs, status);
-    if (rank == 0) fg[b] = gs;
-  }
-  __syncthreads();
-  const FrameGeom<T>& g = gs;
-  const int ncell = g.ncell;
-  int* cnt = cell_count + (size_t)b * cell_cap;
-  int* slot = slot_all + (size_t)b * cell_cap;
-  int* st = cell_start + (size_t)b * (cell_cap + 1);
-  int* raw = raw_all + (size_t)b * N;
-  int* co = cell_of + (size_t)b * N;
-  T* fr = frac + (size_t)b * N * 3;
-  for (int c = gt; c < ncell; c += GT) cnt[c] = 0;
-  cluster_barrier();
-  for (int i = gt; i < N; i += GT) {
-    T fx, fy, fz;
-    const int c = place_atom<T>(g, pos + ((size_t)b * N + i) * 3, fx, fy, fz);
-    fr[3 * i] = fx; fr[3 * i + 1] = fy; fr[3 * i + 2] = fz;
-    co[i] = c;
-    slot[i] = atomicAdd(cnt + c, 1);
-  }
-  cluster_barrier();
-  // every block scans the counts of all cells below its share first (a strided sum), then its share
-  const int per = (ncell + CELLS_CLUSTER - 1) / CELLS_CLUSTER, c0 = min(rank * per, ncell), c1 = min(c0 + per, ncell);
-  int below = 0;
-  for (int c = tid; c < c0; c += 1024) below += __ldcg(cnt + c);
-  int carry;
-  block_scan(below, part, carry);
-  for (int base = c0; base < c1; base += 1024) {
-    const int c = base + tid, v = (c < c1) ? __ldcg(cnt + c) : 0;
-    if (v > mpc) set_status(status, STAFB_ERR_CELL_OVERFLOW);
-    int tot;
-    const int x = carry + block_scan(v, part, tot);
-    if (c < c1) st[c] = x;
-    carry += tot;
-  }
-  if (gt == 0) st[ncell] = N;
-  cluster_barrier();
-  for (int i = gt; i < N; i += GT) raw[__ldcg(st + co[i]) + slot[i]] = i;
-  cluster_barrier();
-  for (int i = gt; i < N; i += GT) {
-    const int c = co[i], s0 = __ldcg(st + c), s1 = __ldcg(st + c + 1);
-    int r = 0;
-    for (int f = s0; f < s1; f++) r += (__ldcg(raw + f) < i);
-    cxyz[(size_t)b * N + s0 + r] = cell_entry<T>(fr[3 * i], fr[3 * i + 1], fr[3 * i + 2], i);
-  }
-}
-
-// Larger frames: the same passes as kernels over all atoms.  grid (blocks over atoms, frames); every block derives its
-// frame's geometry again (a few dozen flops) instead of waiting for a separate set-up launch.
+// Larger frames: the same passes as kernels over all atoms (all cells).  grid (blocks, frames); every block derives its
+// frame's geometry again (a few dozen flops) instead of waiting for a separate set-up launch.  The counters are zero
+// on entry: k_cell_places, which reads them last, clears them for the next call.
 template <class T>
 __global__ void k_cells(const T* __restrict__ pos, const T* __restrict__ box, int nf, int N, T cutoff, int cell_cap,
                         FrameGeom<T>* __restrict__ fg, T* __restrict__ frac, int* __restrict__ cell_of,
-                        int* __restrict__ cell_count, int* __restrict__ slot, int* __restrict__ status) {
+                        int* __restrict__ cell_count, int* __restrict__ slot, int* __restrict__ total,
+                        int* __restrict__ status) {
   __shared__ FrameGeom<T> gs;
   const int b = blockIdx.y;
   chain_wait();
   if (threadIdx.x == 0) {
     frame_geometry<T>(box + 6 * b, N, cutoff, cell_cap, gs, status);
-    if (blockIdx.x == 0) fg[b] = gs;
+    if (blockIdx.x == 0) {
+      fg[b] = gs;
+      total[b] = 0;
+    }
   }
   __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -277,51 +194,38 @@ __global__ void k_cells(const T* __restrict__ pos, const T* __restrict__ box, in
   const int c = place_atom<T>(gs, pos + t * 3, fx, fy, fz);
   frac[t * 3] = fx; frac[t * 3 + 1] = fy; frac[t * 3 + 2] = fz;
   cell_of[t] = c;
-  slot[(size_t)b * cell_cap + i] = atomicAdd(cell_count + (size_t)b * cell_cap + c, 1);
+  slot[t] = atomicAdd(cell_count + (size_t)b * cell_cap + c, 1);
 }
 
-// Exclusive scan of the per-cell counts of one frame (one block per frame).
 template <class T>
-__global__ void k_scan(const FrameGeom<T>* __restrict__ fg, const int* __restrict__ cell_count,
-                       int* __restrict__ cell_start, int cell_cap, int mpc, int* __restrict__ status) {
-  __shared__ int part[33];
+__global__ void k_cell_places(const FrameGeom<T>* __restrict__ fg, int* __restrict__ cell_count,
+                              int2* __restrict__ cell_range, int* __restrict__ total, int cell_cap, int mpc,
+                              int* __restrict__ status) {
   chain_wait();
-  const int b = blockIdx.x, ncell = fg[b].ncell;
-  const int* cnt = cell_count + (size_t)b * cell_cap;
-  int* st = cell_start + (size_t)b * (cell_cap + 1);
-  int carry = 0;
-  for (int base = 0; base < ncell; base += blockDim.x) {
-    const int c = base + threadIdx.x, v = (c < ncell) ? cnt[c] : 0;
+  const int b = blockIdx.y, ncell = fg[b].ncell;
+  for (int base = blockIdx.x * blockDim.x; base < ncell; base += gridDim.x * blockDim.x) {
+    const int c = base + threadIdx.x;
+    int* cnt = cell_count + (size_t)b * cell_cap + c;
+    const int v = (c < ncell) ? *cnt : 0;
     if (v > mpc) set_status(status, STAFB_ERR_CELL_OVERFLOW);
-    int tot;
-    const int x = carry + block_scan(v, part, tot);
-    if (c < ncell) st[c] = x;
-    carry += tot;
+    const int x = cell_places(v, total + b);
+    if (c < ncell) {
+      cell_range[(size_t)b * cell_cap + c] = make_int2(x, v);
+      *cnt = 0;
+    }
   }
-  if (threadIdx.x == 0) st[ncell] = carry;
-}
-
-__global__ void k_fill(int nf, int N, const int* __restrict__ cell_of, const int* __restrict__ cell_start,
-                       const int* __restrict__ slot, int* __restrict__ raw, int cell_cap) {
-  chain_wait();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nf * N) return;
-  const int b = t / N, i = t - b * N;
-  raw[(size_t)b * N + cell_start[(size_t)b * (cell_cap + 1) + cell_of[t]] + slot[(size_t)b * cell_cap + i]] = i;
 }
 
 template <class T>
-__global__ void k_order_cells(int nf, int N, const int* __restrict__ cell_of, const int* __restrict__ cell_start,
-                              const int* __restrict__ raw, const T* __restrict__ frac,
-                              typename Vec4<T>::type* __restrict__ cxyz, int cell_cap) {
+__global__ void k_fill(int nf, int N, const int* __restrict__ cell_of, const int2* __restrict__ cell_range,
+                       const int* __restrict__ slot, const T* __restrict__ frac,
+                       typename Vec4<T>::type* __restrict__ cxyz, int cell_cap) {
   chain_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nf * N) return;
   const int b = t / N, i = t - b * N;
-  const int* st = cell_start + (size_t)b * (cell_cap + 1);
-  const int c = cell_of[t], s0 = st[c];
-  const int r = cell_rank(raw + (size_t)b * N, s0, st[c + 1], i);
-  cxyz[(size_t)b * N + s0 + r] = cell_entry<T>(frac[(size_t)t * 3], frac[(size_t)t * 3 + 1], frac[(size_t)t * 3 + 2], i);
+  const int p = cell_range[(size_t)b * cell_cap + cell_of[t]].x + slot[t];
+  cxyz[(size_t)b * N + p] = cell_entry<T>(frac[(size_t)t * 3], frac[(size_t)t * 3 + 1], frac[(size_t)t * 3 + 2], i);
 }
 
 template <class T>
@@ -498,6 +402,16 @@ __device__ __forceinline__ void record_header(const RowSink& sk, size_t row, int
   }
 }
 
+// Whether neighbour j was discovered before neighbour i: cells[27] in visiting order, ascending index inside a cell.
+static __device__ __noinline__ int discovered_before(int j, int i, const int* __restrict__ cell_of,
+                                                     const int* cells) {
+  const int cj = cell_of[j], ci = cell_of[i];
+  if (cj == ci) return j < i;
+  int q = 0;
+  while (q < 26 && cells[q] != cj && cells[q] != ci) q++;
+  return cells[q] == cj;
+}
+
 // Shared memory of one warp of k_nl_radial: nr4 keys (nr rounded up to four, then a key of padding), two index rows
 // and the candidate list.
 constexpr int NL_CAND = 384;  // candidates listed at a time (27 cells hold about 300 atoms in liquid water)
@@ -516,7 +430,7 @@ __host__ __device__ inline int nl_warp_bytes(int nr) {
 template <class T, int WARPS, bool OPS>
 __global__ void __launch_bounds__(WARPS * 32)
     k_nl_radial(int nf, int N, int ncen, int nr, CoreCoef<T> cc, const FrameGeom<T>* __restrict__ fg,
-                const T* __restrict__ frac, const int* __restrict__ cell_of, const int* __restrict__ cell_start,
+                const T* __restrict__ frac, const int* __restrict__ cell_of, const int2* __restrict__ cell_range,
                 const typename Vec4<T>::type* __restrict__ cxyz, int cell_cap, T* __restrict__ raddescr,
                 T* __restrict__ des3bsupp, int* __restrict__ intmap2b, T* __restrict__ der2b,
                 T* __restrict__ der3bsupp, int* __restrict__ numtriplet, T* __restrict__ geom, T* __restrict__ gsc,
@@ -539,21 +453,22 @@ __global__ void __launch_bounds__(WARPS * 32)
   const T pix = fr[3 * i], piy = fr[3 * i + 1], piz = fr[3 * i + 2];
   const int ci = cell_of[(size_t)b * N + i];
   const int cz = ci / (g.nx * g.ny), rem = ci - cz * (g.nx * g.ny), cy = rem / g.nx, cx = rem - cy * g.nx;
-  const int* cst = cell_start + (size_t)b * (cell_cap + 1);
+  const int2* crg = cell_range + (size_t)b * cell_cap;
   const T cut2 = cc.Rc * cc.Rc;
   const unsigned lt = (1u << lane) - 1u;
   // The 27 neighbour cells in the reference's visiting order: lane q < 27 owns cell q and an inclusive scan gives the
   // place of its members in the list of candidates, which the lanes write NL_CAND at a time.
-  int s0 = 0, cn = 0;
+  int s0 = 0, cn = 0, mycell = -1;
   if (lane < 27) {
     const int di = lane / 9 - 1, dj = (lane / 3) % 3 - 1, dk = lane % 3 - 1;
     int bi = cx + di, bj = cy + dj, bk = cz + dk;
     if (bi < 0) bi = g.nx - 1; else if (bi == g.nx) bi = 0;
     if (bj < 0) bj = g.ny - 1; else if (bj == g.ny) bj = 0;
     if (bk < 0) bk = g.nz - 1; else if (bk == g.nz) bk = 0;
-    const int c = bi + bj * g.nx + bk * g.nx * g.ny;
-    s0 = cst[c];
-    cn = cst[c + 1] - s0;
+    mycell = bi + bj * g.nx + bk * g.nx * g.ny;
+    const int2 rg = crg[mycell];
+    s0 = rg.x;
+    cn = rg.y;
   }
   int x = cn;
 #pragma unroll
@@ -594,34 +509,37 @@ __global__ void __launch_bounds__(WARPS * 32)
   if (n + lane < nr4 && lane < 4) d2a[n + lane] = T(3e38);
   for (int k = lane; k < n; k += 32) jb[k] = -1;
   __syncwarp();
-  // Rank sort, two keys per lane against four keys per load: position = #{f : d2[f] < d2[e]}.  Equal distances collide
-  // in one place and leave another empty; then (rare) the ranks are formed again with the stable rule
-  // #{f : d2[f] < d2[e] or (equal and f < e)}.
-  for (int e0 = 0; e0 < n; e0 += 64) {
-    const int ea = e0 + lane, eb = ea + 32;
-    const T ka = ea < n ? d2a[ea] : T(0), kb = eb < n ? d2a[eb] : T(0);
-    int ra = 0, rb = 0;
-    for (int f = 0; f < n; f += 4) {
-      const T4 kf = *reinterpret_cast<const T4*>(d2a + f);
-      ra += (kf.x < ka) + (kf.y < ka) + (kf.z < ka) + (kf.w < ka);
-      rb += (kf.x < kb) + (kf.y < kb) + (kf.z < kb) + (kf.w < kb);
+  // Rank sort, two keys per lane against four keys per load: position = #{f : d2[f] < d2[e]}.  Equal distances (the two
+  // hydrogens of a rigid molecule, often) collide in one place and leave another empty.  Then the keys are walked once
+  // more for equal ones, which are ordered as they were discovered: by cell, in ascending index inside a cell.
+  auto rank_sort = [&](auto ties) {
+    for (int e0 = 0; e0 < n; e0 += 64) {
+      const int ea = e0 + lane, eb = ea + 32;
+      const T ka = ea < n ? d2a[ea] : T(0), kb = eb < n ? d2a[eb] : T(0);
+      int ra = 0, rb = 0;
+      for (int f = 0; f < n; f += 4) {
+        const T4 kf = *reinterpret_cast<const T4*>(d2a + f);
+        ra += (kf.x < ka) + (kf.y < ka) + (kf.z < ka) + (kf.w < ka);
+        rb += (kf.x < kb) + (kf.y < kb) + (kf.z < kb) + (kf.w < kb);
+      }
+      if (decltype(ties)::value)
+        for (int f = 0; f < n; f++) {
+          const T kf = d2a[f];
+          if (kf == ka && f != ea) ra += discovered_before(ja[f], ja[ea], cell_of + (size_t)b * N, cand);
+          if (kf == kb && f != eb) rb += discovered_before(ja[f], ja[eb], cell_of + (size_t)b * N, cand);
+        }
+      if (ea < n) jb[ra] = ja[ea];
+      if (eb < n) jb[rb] = ja[eb];
     }
-    if (ea < n) jb[ra] = ja[ea];
-    if (eb < n) jb[rb] = ja[eb];
-  }
+  };
+  rank_sort(std::false_type());
   __syncwarp();
   bool hole = false;
   for (int k = lane; k < n; k += 32) hole |= jb[k] < 0;
   if (__any_sync(0xffffffffu, hole)) {
-    for (int e = lane; e < n; e += 32) {
-      const T key = d2a[e];
-      int r = 0;
-      for (int f = 0; f < n; f++) {
-        const T kf = d2a[f];
-        r += (kf < key) || (kf == key && f < e);
-      }
-      jb[r] = ja[e];
-    }
+    cand[lane] = mycell;  // the 27 cells in visiting order
+    __syncwarp();
+    rank_sort(std::true_type());
   }
   __syncwarp();
   const size_t base = (size_t)gi;
@@ -804,29 +722,23 @@ int launch_descriptors(stafb_ctx* c, cudaStream_t s, const T* pos, const T* box,
   const int tot = nf * N;
   typedef typename Vec4<T>::type T4;
   T4* cxyz = reinterpret_cast<T4*>(c->cxyz);
-  const size_t small_sm = sizeof(int) * ((size_t)cap + 1 + 2 * N);
+  int2* crange = reinterpret_cast<int2*>(c->cell_range);
+  const size_t small_sm = sizeof(int) * ((size_t)cap + N);
   if (small_sm <= 48 * 1024 && N <= CELLS_SMALL_MAX) {
     const int threads = N >= 1024 ? 1024 : ((N + 31) & ~31);
     STAFB_CUDA_OK(launch_chained(k_cell_lists_small<T>, nf, threads, small_sm, s, pos, box, N, cc.Rc, cap, mpc, fg, frac,
-                                 c->cell_of, c->cell_start, cxyz, c->status_d));
-    c->launches += 1;
-  } else if (N <= CELLS_CLUSTER_MAX) {
-    STAFB_CUDA_OK(launch_chained(k_cell_lists_cluster<T>, nf * CELLS_CLUSTER, 1024, 0, s, pos, box, N, cc.Rc, cap, mpc,
-                                 fg, frac, c->cell_of, c->cell_count, c->cell_start, c->cell_cursor, c->cells_raw, cxyz,
-                                 c->status_d));
+                                 c->cell_of, crange, cxyz, c->status_d));
     c->launches += 1;
   } else {
-    STAFB_CUDA_OK(cudaMemsetAsync(c->cell_count, 0, sizeof(int) * (size_t)nf * cap, s));
     // each of these needs all of its predecessor's output: chained launches only save the launch gaps
     STAFB_CUDA_OK(launch_chained(k_cells<T>, dim3((N + 255) / 256, nf), 256, 0, s, pos, box, nf, N, cc.Rc, cap, fg,
-                                 frac, c->cell_of, c->cell_count, c->cell_cursor, c->status_d));
-    STAFB_CUDA_OK(launch_chained(k_scan<T>, nf, 1024, 0, s, (const FrameGeom<T>*)fg, (const int*)c->cell_count,
-                                 c->cell_start, cap, mpc, c->status_d));
-    STAFB_CUDA_OK(launch_chained(k_fill, (tot + 255) / 256, 256, 0, s, nf, N, (const int*)c->cell_of,
-                                 (const int*)c->cell_start, (const int*)c->cell_cursor, c->cells_raw, cap));
-    STAFB_CUDA_OK(launch_chained(k_order_cells<T>, (tot + 255) / 256, 256, 0, s, nf, N, (const int*)c->cell_of,
-                                 (const int*)c->cell_start, (const int*)c->cells_raw, (const T*)frac, cxyz, cap));
-    c->launches += 5;
+                                 frac, c->cell_of, c->cell_count, c->cell_slot, c->cell_total, c->status_d));
+    // a liquid has an atom in every tenth of a cutoff's cube or so; emptier frames make a block loop
+    STAFB_CUDA_OK(launch_chained(k_cell_places<T>, dim3((N / 8 + 255) / 256, nf), 256, 0, s, (const FrameGeom<T>*)fg,
+                                 c->cell_count, crange, c->cell_total, cap, mpc, c->status_d));
+    STAFB_CUDA_OK(launch_chained(k_fill<T>, (tot + 255) / 256, 256, 0, s, nf, N, (const int*)c->cell_of,
+                                 (const int2*)crange, (const int*)c->cell_slot, (const T*)frac, cxyz, cap));
+    c->launches += 3;
   }
   {
     constexpr int W = 4;
@@ -835,7 +747,7 @@ int launch_descriptors(stafb_ctx* c, cudaStream_t s, const T* pos, const T* box,
     // the operators' outputs or the records of the fused sweeps alone
     auto kern = raddescr || intmap2b ? k_nl_radial<T, W, true> : k_nl_radial<T, W, false>;
     STAFB_CUDA_OK(launch_chained(kern, (rows + W - 1) / W, W * 32, sm, s, nf, N, ncen, nr, cc, fg, frac, c->cell_of,
-                                 c->cell_start, cxyz, cap, raddescr, des3bsupp, intmap2b, der2b, der3bsupp, numtriplet,
+                                 (const int2*)crange, cxyz, cap, raddescr, des3bsupp, intmap2b, der2b, der3bsupp, numtriplet,
                                  geom, gsc, na, c->status_d, sk));
   }
   c->launches += 1;
@@ -904,10 +816,10 @@ constexpr size_t NA_OFF_FGEOM = 0;
 constexpr size_t NA_OFF_FRAC = NA_OFF_FGEOM + al256(sizeof(stafb::FrameGeom<double>) * NOALLOC_MAX_FRAMES);
 constexpr size_t NA_OFF_CELLOF = NA_OFF_FRAC + al256(sizeof(double) * 3 * NOALLOC_MAX_ATOMS);
 constexpr size_t NA_OFF_COUNT = NA_OFF_CELLOF + al256(sizeof(int) * NOALLOC_MAX_ATOMS);
-constexpr size_t NA_OFF_START = NA_OFF_COUNT + al256(sizeof(int) * NOALLOC_MAX_CELLS);
-constexpr size_t NA_OFF_CURSOR = NA_OFF_START + al256(sizeof(int) * (NOALLOC_MAX_CELLS + NOALLOC_MAX_FRAMES));
-constexpr size_t NA_OFF_RAW = NA_OFF_CURSOR + al256(sizeof(int) * NOALLOC_MAX_CELLS);
-constexpr size_t NA_OFF_CXYZ = NA_OFF_RAW + al256(sizeof(int) * NOALLOC_MAX_ATOMS);
+constexpr size_t NA_OFF_RANGE = NA_OFF_COUNT + al256(sizeof(int) * NOALLOC_MAX_CELLS);
+constexpr size_t NA_OFF_SLOT = NA_OFF_RANGE + al256(sizeof(int) * 2 * NOALLOC_MAX_CELLS);
+constexpr size_t NA_OFF_TOTAL = NA_OFF_SLOT + al256(sizeof(int) * NOALLOC_MAX_ATOMS);
+constexpr size_t NA_OFF_CXYZ = NA_OFF_TOTAL + al256(sizeof(int) * NOALLOC_MAX_FRAMES);
 constexpr size_t NA_OFF_GEOM = NA_OFF_CXYZ + al256(sizeof(double) * 4 * NOALLOC_MAX_ATOMS);
 constexpr size_t NA_OFF_GSC = NA_OFF_GEOM + al256(sizeof(double) * 4 * NOALLOC_MAX_ATOMS * NOALLOC_MAX_NR);
 constexpr size_t NA_OFF_STATUS = NA_OFF_GSC + al256(sizeof(double) * 2 * NOALLOC_MAX_ATOMS * NOALLOC_MAX_NR);
@@ -967,15 +879,15 @@ extern "C" int stafb_compute_descriptors_light_noalloc(int dtype, double radial_
   c.frac = base + NA_OFF_FRAC;
   c.cell_of = reinterpret_cast<int*>(base + NA_OFF_CELLOF);
   c.cell_count = reinterpret_cast<int*>(base + NA_OFF_COUNT);
-  c.cell_start = reinterpret_cast<int*>(base + NA_OFF_START);
-  c.cell_cursor = reinterpret_cast<int*>(base + NA_OFF_CURSOR);
-  c.cells_raw = reinterpret_cast<int*>(base + NA_OFF_RAW);
+  c.cell_range = base + NA_OFF_RANGE;
+  c.cell_slot = reinterpret_cast<int*>(base + NA_OFF_SLOT);
+  c.cell_total = reinterpret_cast<int*>(base + NA_OFF_TOTAL);
   c.cxyz = base + NA_OFF_CXYZ;
   c.geom = base + NA_OFF_GEOM;
   c.gsc = base + NA_OFF_GSC;
   c.status_d = reinterpret_cast<int*>(base + NA_OFF_STATUS);
-  // the shared array keeps the previous call's contents: clear the status word here (the cell
-  // counters are cleared by the descriptor launch sequence itself)
+  // the shared array keeps the previous call's contents: clear the status word here (frames of this size count their
+  // cells in shared memory)
   STAFB_CUDA_OK(cudaMemsetAsync(c.status_d, 0, sizeof(int), s));
   int rc;
   if (dtype == STAFB_F32)

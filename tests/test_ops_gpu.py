@@ -68,6 +68,22 @@ def test_compute_descriptors_light(ops, oracle, frame0, case, dtype):
     print("tie groups:", groups)
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [6, 13])
+def test_equal_distances_keep_the_order_of_discovery(ops, oracle, n, dtype):
+    """A perfect cubic lattice (216 and 2,197 atoms: the one-block and the multi-kernel cell lists), where every
+    neighbour shell is at one distance: the order inside a shell is cell by cell, ascending index in a cell."""
+    L, rng = 3.0 * n, np.random.default_rng(n)
+    x = (np.stack(np.meshgrid(*[np.arange(n)] * 3, indexing="ij"), -1).reshape(-1, 3) * 3.0)[rng.permutation(n ** 3)]
+    pos, box = x.reshape(1, -1).astype(dtype), np.array([[L, 0, 0, L, 0, L]], dtype)
+    _ctx(ops, dtype, n ** 3, 1)
+    ref = oracle.descriptors(CFG["Rc"], CFG["Rs"], CFG["Ra"], CFG["nr"], CFG["na"], pos, box, dtype)
+    assert ref["status"] == 0 and ref["intmap2b"][..., 0].min() == 18
+    for _ in range(3):
+        out = ops.compute_descriptors_light(_t(pos), _t(box), with_angular=False)
+        assert np.array_equal(out[3].cpu().numpy(), ref["intmap2b"])
+
+
 def _species_slices(d, shape, t):
     s, Nl = shape.shift(t), shape.tipos[t]
     return {k: np.ascontiguousarray(v[:, s:s + Nl]) for k, v in d.items() if isinstance(v, np.ndarray) and v.ndim >= 2}
