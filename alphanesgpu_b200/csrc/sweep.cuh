@@ -146,7 +146,7 @@ template <> struct SweepMinBlocks<MODE_FGRAD, 8> { static constexpr int value = 
 //   [0, 32)  int nact[8]            active channels (squared embedding != 0) of class s = ta + tb
 //   actc     uchar [ncls][Famax]    their channel numbers, compacted
 //   chq      T4 [ncls][maxp]        channel pair (2p, 2p+1) of the compacted list: alpha1 x2, alpha2 x2
-//   chr      T4 [ncls][maxp]        beta x2, beta*log2(e) x2
+//   chr      T2 [ncls][maxp]        beta x2
 //   che      T2 [ncls][maxp]        squared embedding x2 (an odd count is padded with an all-zero channel)
 //   rpar     T4 [nt][Frmax]         radial channels: alpha2b*log2(e), alpha2b, squared embedding, 0
 struct SparLayout {
@@ -160,7 +160,7 @@ static inline SparLayout spar_layout(const ModelDev& d) {
   L.maxp = (d.Famax + 1) / 2 > 0 ? (d.Famax + 1) / 2 : 1;
   L.actc = take(d.ncls * (d.Famax > 0 ? d.Famax : 1));
   L.chq = take(d.ncls * L.maxp * 4 * (int)sizeof(T));
-  L.chr = take(d.ncls * L.maxp * 4 * (int)sizeof(T));
+  L.chr = take(d.ncls * L.maxp * 2 * (int)sizeof(T));
   L.che = take(d.ncls * L.maxp * 2 * (int)sizeof(T));
   L.rpar = take(d.nt * (d.Frmax > 0 ? d.Frmax : 1) * 4 * (int)sizeof(T));
   L.total = o;
@@ -179,10 +179,9 @@ __device__ __forceinline__ void spar_fill_class(const ModelDev& md, const SparLa
   const T* e3 = emb + md.off_emb[t] + nt * Fr + (size_t)s * Fa;
   unsigned char* actc = blk + sl.actc + s * md.Famax;
   T* chq = reinterpret_cast<T*>(blk + sl.chq) + (size_t)s * sl.maxp * 4;
-  T* chr = reinterpret_cast<T*>(blk + sl.chr) + (size_t)s * sl.maxp * 4;
+  T* chr = reinterpret_cast<T*>(blk + sl.chr) + (size_t)s * sl.maxp * 2;
   T* che = reinterpret_cast<T*>(blk + sl.che) + (size_t)s * sl.maxp * 2;
   const unsigned lt = (1u << lane) - 1u;
-  const T SC = Ex<T>::scale();
   int nact = 0;
   for (int c0 = 0; c0 < Fa; c0 += 32) {
     const int c = c0 + lane;
@@ -194,7 +193,7 @@ __device__ __forceinline__ void spar_fill_class(const ModelDev& md, const SparLa
       const T al1 = a3[3 * c], al2 = a3[3 * c + 1], be = a3[3 * c + 2];
       actc[slot] = (unsigned char)c;
       chq[pr * 4 + h] = al1; chq[pr * 4 + 2 + h] = al2;
-      chr[pr * 4 + h] = be;  chr[pr * 4 + 2 + h] = be * SC;
+      chr[pr * 2 + h] = be;
       che[pr * 2 + h] = ee;
     }
     nact += __popc(bal);
@@ -204,7 +203,7 @@ __device__ __forceinline__ void spar_fill_class(const ModelDev& md, const SparLa
     if (nact & 1) {  // the partner of the last channel: a channel that contributes nothing
       const int pr = nact >> 1;
       chq[pr * 4 + 1] = T(0); chq[pr * 4 + 3] = T(0);
-      chr[pr * 4 + 1] = T(0); chr[pr * 4 + 3] = T(0);
+      chr[pr * 2 + 1] = T(0);
       che[pr * 2 + 1] = T(0);
     }
   }
@@ -357,7 +356,7 @@ __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __
                                                 const typename Vec4<T>::type* __restrict__ dF,
                                                 const typename Vec4<T>::type* __restrict__ tab4, int nr,
                                                 const typename Vec4<T>::type* __restrict__ chq,
-                                                const typename Vec4<T>::type* __restrict__ chr, const T* __restrict__ et,
+                                                const typename Vec2<T>::type* __restrict__ chr, const T* __restrict__ et,
                                                 int oa, int ob,
                                                 int na_, int nb_, int lane,
                                                 typename Vec2<T>::type (&r0)[NCHP], typename Vec2<T>::type (&r1)[NCHP],
@@ -372,11 +371,11 @@ __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __
   const int np = PairWalk<SAME, 32 * NW>::count(na_, nb_);
   PairWalk<SAME, 32 * NW> pw;
   pw.init(na_, nb_, lane);
-  // beta*log2(e) of every channel pair stays in registers in the fingerprint modes
+  // beta of every channel pair stays in registers in the fingerprint modes
   T2 bsc[NCHP];
   if (MODE != MODE_FGRAD) {
 #pragma unroll
-    for (int lp = 0; lp < NCHP; lp++) { const T4 cr = chr[lp]; bsc[lp] = mk2(cr.z, cr.w); }
+    for (int lp = 0; lp < NCHP; lp++) bsc[lp] = chr[lp];
   }
   // pairs in flight per lane: two hide the shared-memory and exponential latencies of the fingerprint loops; the
   // force-backward loop is too large for that (its unrolled body falls out of the instruction cache)
@@ -392,7 +391,8 @@ __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __
     const T cs = uj.x * uk.x + uj.y * uk.y + uj.z * uk.z;
     const T half = T(0.5) * cs + T(0.5);
     const T tt = half * fcj * fck;
-    const T2 tt2 = mk2(tt, tt), fcj2 = mk2(fcj, fcj), fck2 = mk2(fck, fck);
+    const T ts = tt * Ex<T>::scale();  // exp(beta t) as 2^(beta ts) in fp32
+    const T2 tt2 = mk2(tt, tt), ts2 = mk2(ts, ts), fcj2 = mk2(fcj, fcj), fck2 = mk2(fck, fck);
     if (MODE != MODE_FGRAD) {
 #pragma unroll
       for (int lp = 0; lp < NCHP; lp++) {
@@ -400,7 +400,7 @@ __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __
         const T4 A = tab4[j * TSTR + lp], B = tab4[k * TSTR + lp];
         const T2 S1 = p_mul(mk2(A.z, A.w), mk2(B.x, B.y), h);  // exp(a2*sj + a1*sk)
         const T2 S2 = p_mul(mk2(A.x, A.y), mk2(B.z, B.w), h);  // exp(a1*sj + a2*sk)
-        const T2 cm = p_mul(p_ex(p_mul(bsc[lp], tt2, h), et, h), tt2, h);  // t*exp(beta*t)
+        const T2 cm = p_mul(p_ex(p_mul(bsc[lp], ts2, h), et, h), tt2, h);  // t*exp(beta*t)
         const T2 ss = p_add(S1, S2, h);
         r0[lp] = p_fma(cm, ss, r0[lp], h);  // the channel coefficient is applied after the reduction
         if (MODE == MODE_AFV) {
@@ -418,7 +418,7 @@ __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __
       // its derivatives:  d/da1 = Z1 (sj H1 + t Pj/2) + Z2 (sk H2 + t Pk/2),  d/da2 with sj, sk and Pj, Pk
       // exchanged inside each bracket,  d/dbeta = t [Z1 (H1 + Q/2) + Z2 (H2 + Q/2)]
       // (STAF/src/grad_force/ang/reforce.cu.cc:47-231).
-      const T4 pj = V[j], pk = V[k];
+      const T2 pj = *reinterpret_cast<const T2*>(V + j), pk = *reinterpret_cast<const T2*>(V + k);  // 1/r, dfc/dr
       const T hf = T(0.5) * fcj * fck;
       const T ajk = hf * pj.x, akj = hf * pk.x;
       const T bjk = -cs * ajk + half * pj.y * fck;
@@ -433,12 +433,13 @@ __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __
 #pragma unroll
       for (int lp = 0; lp < NCHP; lp++) {
         const bool h = ODD && lp == NCHP - 1;
-        const T4 A = tab4[j * TSTR + lp], B = tab4[k * TSTR + lp], cq = chq[lp], cr = chr[lp];
+        const T4 A = tab4[j * TSTR + lp], B = tab4[k * TSTR + lp], cq = chq[lp];
+        const T2 be = chr[lp];
         const T2 al1 = mk2(cq.x, cq.y), al2 = mk2(cq.z, cq.w);
-        const T2 E = p_ex(p_mul(mk2(cr.z, cr.w), tt2, h), et, h);
+        const T2 E = p_ex(p_mul(be, ts2, h), et, h);
         const T2 Z1 = p_mul(E, p_mul(mk2(A.x, A.y), mk2(B.z, B.w), h), h);
         const T2 Z2 = p_mul(E, p_mul(mk2(A.z, A.w), mk2(B.x, B.y), h), h);
-        const T2 gQ = p_mul(p_fma(mk2(cr.x, cr.y), tt2, one2, h), Qh2, h);
+        const T2 gQ = p_mul(p_fma(be, tt2, one2, h), Qh2, h);
         const T2 H1 = p_fma(al1, Pj2, p_fma(al2, Pk2, gQ, h), h), H2 = p_fma(al1, Pk2, p_fma(al2, Pj2, gQ, h), h);
         r0[lp] = p_fma(Z1, H1, p_fma(Z2, H2, r0[lp], h), h);
         r1[lp] = p_fma(Z1, p_fma(fcj2, H1, Pj2, h), p_fma(Z2, p_fma(fck2, H2, Pk2, h), r1[lp], h), h);
@@ -459,7 +460,7 @@ __device__ __forceinline__ void pairs_force(const typename Vec4<T>::type* __rest
                                             const typename Vec4<T>::type* __restrict__ V,
                                             const typename Vec4<T>::type* __restrict__ tab4,
                                             const typename Vec4<T>::type* __restrict__ chq,
-                                            const typename Vec4<T>::type* __restrict__ chr,
+                                            const typename Vec2<T>::type* __restrict__ chr,
                                             const typename Vec2<T>::type* __restrict__ wch, const T* __restrict__ et,
                                             int oo, int op, int no, int npt, int lane, T* __restrict__ fo,
                                             T* __restrict__ part, T& fix, T& fiy, T& fiz) {
@@ -511,16 +512,18 @@ __device__ __forceinline__ void pairs_force(const typename Vec4<T>::type* __rest
         const T cs = uj.x * uk.x + uj.y * uk.y + uj.z * uk.z;
         const T half = T(0.5) * cs + T(0.5);
         const T tt = half * uj.w * uk.w;
-        const T2 tt2 = mk2(tt, tt);
+        const T ts = tt * Ex<T>::scale();
+        const T2 tt2 = mk2(tt, tt), ts2 = mk2(ts, ts);
         T2 D2 = mk2(T(0), T(0)), BJ2 = mk2(T(0), T(0));
 #pragma unroll
         for (int lp = 0; lp < NCHP; lp++) {
-          const T4 B = tab4[k * TSTR + lp], cr = chr[lp];
+          const T4 B = tab4[k * TSTR + lp];
+          const T2 be = chr[lp];
           const T2 A1k = mk2(B.x, B.y), A2k = mk2(B.z, B.w);
           const bool h = ODD && lp == NCHP - 1;
-          const T2 Ex2 = p_ex(p_mul(mk2(cr.z, cr.w), tt2, h), et, h);
+          const T2 Ex2 = p_ex(p_mul(be, ts2, h), et, h);
           const T2 sum = p_fma(a1w[lp], A2k, p_mul(a2w[lp], A1k, h), h);                // w (S2 + S1)
-          D2 = p_fma(p_mul(p_fma(mk2(cr.x, cr.y), tt2, one2, h), Ex2, h), sum, D2, h);  // w e^{bt} (1 + bt) (S1 + S2)
+          D2 = p_fma(p_mul(p_fma(be, tt2, one2, h), Ex2, h), sum, D2, h);  // w e^{bt} (1 + bt) (S1 + S2)
           BJ2 = p_fma(Ex2, p_fma(b1w[lp], A2k, p_mul(b2w[lp], A1k, h), h), BJ2, h);     // w e^{bt} (a1 S2 + a2 S1)
         }
         const T D = D2.x + D2.y, BJ = (BJ2.x + BJ2.y) * tt;
@@ -611,7 +614,7 @@ __global__ void __launch_bounds__(32 * NW, (SweepMinBlocks<MODE, sizeof(T)>::val
   const int* nact_s = reinterpret_cast<const int*>(spb);
   const unsigned char* actc = spb + sl.actc;
   const T4* chq_all = reinterpret_cast<const T4*>(spb + sl.chq);
-  const T4* chr_all = reinterpret_cast<const T4*>(spb + sl.chr);
+  const T2* chr_all = reinterpret_cast<const T2*>(spb + sl.chr);
   const T2* che_all = reinterpret_cast<const T2*>(spb + sl.che);
   const T4* rpar = reinterpret_cast<const T4*>(spb + sl.rpar);
   T4* tab4 = reinterpret_cast<T4*>(smem_raw + L.tab);
@@ -826,7 +829,7 @@ __global__ void __launch_bounds__(32 * NW, (SweepMinBlocks<MODE, sizeof(T)>::val
         const int nchp = (npair - p0) < MAXP ? (npair - p0) : MAXP;
         const int nch = sizeof(T) == 4 ? 2 * nchp : ((nact - 2 * p0) < 2 * MAXP ? (nact - 2 * p0) : 2 * MAXP);
         const T4* chq = chq_all + s * sl.maxp + p0;
-        const T4* chr = chr_all + s * sl.maxp + p0;
+        const T2* chr = chr_all + s * sl.maxp + p0;
         // tables exp(a1*fc_k), exp(a2*fc_k) of the neighbours of the two species, all channel pairs of a
         // neighbour in flight together
         const int nu = same ? na_ : na_ + nb_;
