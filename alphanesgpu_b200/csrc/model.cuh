@@ -66,6 +66,7 @@ static inline int species_blocks(const ModelDev& md, int nf, int W) {
   return s;
 }
 
+#include "devmath.cuh"
 #include "sweep.cuh"
 
 // ---------------------------------------------------------------------------- MLP head

@@ -7,12 +7,44 @@
 // one write per output element (per-atom outputs) or one atomic per block (parameter
 // gradients) instead of one global atomic per (neighbour, channel).  Channel/class pairs whose
 // squared embedding is exactly zero are skipped (they contribute exactly zero).
+//
+// Angular operators.  The neighbours are grouped by species, so that the triplets of a species-pair class are a
+// rectangle (or a triangle) of group members with one parameter row, and the triplet's slot in the caller's tensors
+// follows from the two sorted positions.  exp(a1 sj + a2 sk) is a product of table entries exp(a1 s), exp(a2 s) per
+// (neighbour, channel), which leaves one exponential per (triplet, channel) instead of three; a chunk of channels
+// shares one pass over a class, and its sums one reduction at the end.  What bounds them is the latency of a block's
+// passes (staging, tables, triplets, reduction) at one block per atom: 768 atoms, fp32, all central species,
+// fingerprints 71 -> 25 us, their gradient 81 -> 28 us, forces 128 -> 41 us, gradient of the forces 92 -> 45 us (the
+// form before this one: three library exponentials per (triplet, channel), a block reduction per channel and class,
+// and shared-memory float atomics for the forces, whose 32 lanes met on one address).
 #include "common.cuh"
 
 namespace stafb {
 
+#include "devmath.cuh"
+
 constexpr int OPS_THREADS = 128;
 constexpr int OPS_WARPS = OPS_THREADS / 32;
+constexpr int ANG_THREADS = 256;
+constexpr int ANG_WARPS = ANG_THREADS / 32;
+constexpr int ANG_CH = 8;  // channels per pass at most
+
+__device__ __forceinline__ float op_exp(float x, const float*) { return expf(x); }
+__device__ __forceinline__ double op_exp(double x, const double* et) { return exp_table16(x, et); }
+
+// Zero-fills ahead of the operators that accumulate: two buffers, sizes in 4-byte words.  The operator behind it is
+// its programmatic dependent and stages its inputs meanwhile.
+__global__ void k_zero(int* __restrict__ a, size_t na, int* __restrict__ b, size_t nb) {
+  chain_wait();
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x, st = (size_t)gridDim.x * blockDim.x;
+  for (size_t q = t; q < na; q += st) a[q] = 0;
+  for (size_t q = t; q < nb; q += st) b[q] = 0;
+}
+static cudaError_t zero_two(cudaStream_t s, void* a, size_t na, void* b, size_t nb) {
+  const size_t w = (na > nb ? na : nb) / 4;
+  const int blocks = (int)((w + 255) / 256 < 1 ? 1 : ((w + 255) / 256 > 592 ? 592 : (w + 255) / 256));
+  return launch_chained(k_zero, blocks, 256, 0, s, (int*)a, na / 4, (int*)b, nb / 4);
+}
 
 // Extra inputs / outputs of the ...Virial and ...VirialGrad operators (null pointers: plain operator).
 template <class T>
@@ -46,94 +78,474 @@ __device__ __forceinline__ int species_shift(const int* tipos, const int* actual
   return s;
 }
 
-// ---------------------------------------------------------------- radial AF (ComputeSortProj)
-template <class T>
-__global__ void __launch_bounds__(OPS_THREADS)
-    k_af_rad(int natoms, int nr, int Fr, const T* __restrict__ rad, const int* __restrict__ im2,
-             const T* __restrict__ alpha2b, const T* __restrict__ e2, const int* __restrict__ type_map,
-             T* __restrict__ out) {
-  const int gi = blockIdx.x * OPS_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (gi >= natoms) return;
-  const size_t base = gi;
-  int n = im2[base * (nr + 1)];
-  if (n > nr) n = nr;
-  for (int c = 0; c < Fr; c++) {
-    T acc = T(0);
-    for (int j = lane; j < n; j += 32) {
-      const T d = rad[base * nr + j];
-      const int tj = type_map[im2[base * (nr + 1) + 1 + j]];
-      const T ch = e2[Fr * tj + c];
-      if (ch != T(0)) acc += d * (r_exp(alpha2b[Fr * tj + c] * d) * ch);
-    }
-    acc = warp_sum(acc);
-    if (lane == 0) out[base * Fr + c] = acc;
-  }
-}
-
-// Shared staging for the angular operators: species and cutoff value of the sorted
-// neighbours, and the (j,k) pair of every triplet slot packed in 16 bits.
-template <class T>
-struct AngStage {
-  int m, Tn;
-  int* tj;             // [nr]
-  T* ds;               // [nr]
-  unsigned short* jk;  // [na]
+// ---- radial operators that sum over neighbours.  One warp per atom: the neighbours grouped by species in shared
+// memory, one lane per (species, channel) walking its group, so that no sum crosses lanes.
+//   val[k]: descriptor of the k-th grouped neighbour; src[k]: its position in the row; off[q]: first of species q
+struct RadStage {
+  int* src;
+  int* off;  // [nt + 1]
 };
-
+__device__ __forceinline__ void rad_group(const RadStage& st, const int* __restrict__ row, int n, int nt,
+                                          const int* __restrict__ type_map, int lane) {
+  const unsigned lt = (1u << lane) - 1u;
+  int o = 0;
+  for (int q = 0; q < nt; q++) {
+    if (lane == 0) st.off[q] = o;
+    for (int k0 = 0; k0 < n; k0 += 32) {
+      const int k = k0 + lane;
+      const bool p = k < n && type_map[row[k]] == q;
+      const unsigned bal = __ballot_sync(0xffffffffu, p);
+      if (p) st.src[o + __popc(bal & lt)] = k;
+      o += __popc(bal);
+    }
+  }
+  if (lane == 0) st.off[nt] = o;
+  __syncwarp();
+}
+// bytes of shared memory per warp: two value rows, the source row, the offsets, a row per (species, channel)
 template <class T>
-__device__ __forceinline__ void ang_stage(AngStage<T>& st, size_t base, int nr, int na, const int* numtriplet,
-                                          const int* im2, const T* ds3, const int* type_map) {
-  int m = numtriplet[base];
-  if (m > nr) m = nr;
-  long long Tl = (long long)m * (m - 1) / 2;
-  st.m = m;
-  st.Tn = Tl < na ? (int)Tl : na;
-  for (int k = threadIdx.x; k < m; k += blockDim.x) {
-    st.tj[k] = type_map[im2[base * (nr + 1) + 1 + k]];
-    st.ds[k] = ds3[base * nr + k];
-  }
-  for (int nn = threadIdx.x; nn < st.Tn; nn += blockDim.x) {
-    int j, k;
-    unrank_pair(nn, m, j, k);
-    st.jk[nn] = (unsigned short)((j << 8) | k);
-  }
-  __syncthreads();
+static inline size_t rad_warp_bytes(int nr, int nt, int Fr) {
+  return ((size_t)sizeof(T) * (2 * nr + nt * Fr) + sizeof(int) * (nr + nt + 1) + 15) & ~(size_t)15;
+}
+template <class T>
+__device__ __forceinline__ void exp_table_load(T* et) {
+  if (sizeof(T) == 8 && threadIdx.x < 16) et[threadIdx.x] = (T)EXP16_TABLE[threadIdx.x];
+  if (sizeof(T) == 8) __syncthreads();
 }
 
-// ---------------------------------------------------------------- angular AF (ComputeSortProj3body)
+// MODE 0: fingerprints (ComputeSortProj); 1: their parameter gradient (ComputeTwoBodyParGrad); 2: backward of the
+// radial force (ComputeForceRadialGrad).
 template <class T>
-__global__ void __launch_bounds__(OPS_THREADS)
-    k_af_ang(int nr, int na, int Fa, int ncls, const T* __restrict__ ang, const T* __restrict__ ds3,
-             const int* __restrict__ im2, const T* __restrict__ alpha3b, const T* __restrict__ e3,
-             const int* __restrict__ type_map, const int* __restrict__ numtriplet, T* __restrict__ out) {
-  extern __shared__ unsigned char smem_raw[];
-  __shared__ T red[OPS_WARPS + 1];
-  AngStage<T> st;
-  st.ds = reinterpret_cast<T*>(smem_raw);
-  st.tj = reinterpret_cast<int*>(st.ds + nr);
-  st.jk = reinterpret_cast<unsigned short*>(st.tj + nr);
-  const size_t base = blockIdx.x;
-  ang_stage(st, base, nr, na, numtriplet, im2, ds3, type_map);
-  const T* t_row = ang + base * na;
-  for (int c = 0; c < Fa; c++) {
-    T acc = T(0);
-    for (int s = 0; s < ncls; s++) {
-      const T ch = e3[s * Fa + c];
-      if (ch == T(0)) continue;
-      const T a1 = alpha3b[(s * Fa + c) * 3], a2 = alpha3b[(s * Fa + c) * 3 + 1], be = alpha3b[(s * Fa + c) * 3 + 2];
-      for (int nn = threadIdx.x; nn < st.Tn; nn += OPS_THREADS) {
-        const int j = st.jk[nn] >> 8, k = st.jk[nn] & 255;
-        if (st.tj[j] + st.tj[k] != s) continue;
-        const T t = t_row[nn], dj = st.ds[j], dk = st.ds[k];
-        T sw = r_exp(a1 * dj + a2 * dk);
-        sw += r_exp(a2 * dj + a1 * dk);
-        sw *= r_exp(be * t);
-        acc += t * sw * ch / T(2.);
+struct RadArgs {
+  int natoms, Nl, N, nr, Fr, nt;
+  const T *rad, *alpha2b, *e2;
+  const int *im2, *type_map;
+  T* out;             // 0: two_body_afs; 2: gradnet
+  const T* prevgrad;  // 1: [natoms, Fr]; 2: force cotangent [nf, 3N]
+  T *g_alpha, *g_emb;
+  const T *netderiv, *der2b;
+  const int *tipos, *actual_type;
+};
+template <class T, int MODE>
+__global__ void __launch_bounds__(OPS_THREADS) k_rad_sums(RadArgs<T> a, size_t warp_bytes, VirArgs<T> va) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ T et[16];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nr = a.nr, Fr = a.Fr, nt = a.nt, nqc = nt * Fr;
+  T* val = reinterpret_cast<T*>(smem_raw + w * warp_bytes);  // [nr] descriptor
+  T* qv = val + nr;                                          // [nr] 2: projected force cotangent
+  T* rs = qv + nr;                                           // [nt*Fr]
+  RadStage st;
+  st.src = reinterpret_cast<int*>(rs + nqc);
+  st.off = st.src + nr;
+  exp_table_load(et);
+  chain_wait();
+  // a warp keeps the parameter sums of its lanes over all of its atoms and adds them to the gradient once
+  for (int L0 = 0; L0 < nqc; L0 += 32) {
+    const int L = L0 + lane, q = L < nqc ? L / Fr : 0, c = L < nqc ? L - q * Fr : 0;
+    const T al = L < nqc ? a.alpha2b[L] : T(0), ch = L < nqc ? a.e2[L] : T(0);
+    T ga = T(0), ge = T(0);
+    for (int gi = blockIdx.x * OPS_WARPS + w; gi < a.natoms; gi += gridDim.x * OPS_WARPS) {
+      const size_t base = gi;
+      const int* row = a.im2 + base * (nr + 1) + 1;
+      int n = a.im2[base * (nr + 1)];
+      if (n > nr) n = nr;
+      rad_group(st, row, n, nt, a.type_map, lane);
+      const int ng = st.off[nt];
+      int b = 0, ipar = 0;
+      T pix = T(0), piy = T(0), piz = T(0);
+      if (MODE == 2) {
+        b = gi / a.Nl;
+        ipar = gi - b * a.Nl + species_shift(a.tipos, a.actual_type);
+        const T* p = a.prevgrad + ((size_t)b * a.N + ipar) * 3;
+        pix = p[0]; piy = p[1]; piz = p[2];
+      }
+      for (int g = lane; g < ng; g += 32) {
+        const int k = st.src[g];
+        val[g] = a.rad[base * nr + k];
+        if (MODE == 2) {
+          // q = sum_a (Fbar_j - Fbar_i)_a * 0.5 * dd/dr_{i,a}
+          const int nj = row[k];
+          const T* pj = a.prevgrad + ((size_t)b * a.N + nj) * 3;
+          T wd[3] = {T(0), T(0), T(0)};
+          if (va.wbar) {  // the virial cotangent shifts the neighbour's force cotangent by -(Wbar r) (grad_force/rad/reforce.cu.cc:165-234)
+            T r[3];
+            mic_cart(va.pos + ((size_t)b * a.N + ipar) * 3, va.pos + ((size_t)b * a.N + nj) * 3, va.box + (size_t)b * 6, r);
+            const T* Wg = va.wbar + (size_t)b * 9;
+#pragma unroll
+            for (int x = 0; x < 3; x++) wd[x] = Wg[x * 3] * r[0] + Wg[x * 3 + 1] * r[1] + Wg[x * 3 + 2] * r[2];
+          }
+          const T* d2 = a.der2b + base * 3 * nr + k;
+          qv[g] = T(0.5) * ((pj[0] - pix - wd[0]) * d2[0] + (pj[1] - piy - wd[1]) * d2[nr] + (pj[2] - piz - wd[2]) * d2[2 * nr]);
+        }
+      }
+      __syncwarp();
+      if (L < nqc) {
+        T s0 = T(0), s1 = T(0), s2 = T(0);
+        for (int g = st.off[q]; g < st.off[q + 1]; g++) {
+          const T d = val[g], x = op_exp(al * d, et);
+          if (MODE == 0) s0 += d * (x * ch);
+          if (MODE == 1) {
+            s1 += d * d * (x * ch);
+            s2 += d * x;
+          }
+          if (MODE == 2) {
+            const T qq = qv[g], sds = x * (T(1.) + al * d);
+            s0 += qq * ch * sds;
+            s1 += qq * (ch * x * d * (T(2.) + al * d));
+            s2 += qq * sds;
+          }
+        }
+        if (MODE != 1) rs[L] = s0;
+        if (MODE != 0) {
+          const T f = MODE == 1 ? a.prevgrad[base * Fr + c] : a.netderiv[base * Fr + c];
+          ga += f * s1;
+          ge += f * s2;
+        }
+      }
+      __syncwarp();
+      if (MODE != 1 && L0 + 32 >= nqc) {  // every (species, channel) of this atom has been formed
+        for (int cc = lane; cc < Fr; cc += 32) {
+          T v = T(0);
+          for (int x = 0; x < nt; x++) v += rs[x * Fr + cc];
+          a.out[base * Fr + cc] = v;
+        }
+        __syncwarp();
       }
     }
-    acc = block_sum<T, OPS_WARPS>(acc, red);
-    if (threadIdx.x == 0) out[base * Fa + c] = acc;
+    if (MODE != 0 && L < nqc) {
+      if (ga != T(0)) atomicAdd(a.g_alpha + L, ga);
+      if (ge != T(0)) atomicAdd(a.g_emb + L, ge);
+    }
   }
+}
+
+// ---- angular operators: staging
+template <class T>
+struct AngArgs {
+  int Nl, N, nr, na, Fa, nt, ncls, chunk;  // chunk: channels per pass, <= ANG_CH
+  const T *ang, *ds3, *alpha3b, *e3;
+  const int *im2, *type_map, *numtriplet;
+  T* out;              // fingerprints / forces / gradnet
+  const T* prevgrad;   // gradient of the fingerprints: [.,Fa]; backward of the forces: force cotangent [nf,3N]
+  T* g_alpha3;
+  T* zero;             // written with zeros (the operator's third output), zero_n elements
+  int zero_n;
+  const T *netderiv, *der3bsupp, *der3b;
+  const int *tipos, *actual_type;
+};
+// shared memory: T4 par[ncls][chunk] | T2 tab[nt][chunk][nr] | T ds[nr] | T acc[Fa] | T red[C][warps][32] | extra |
+// int pos[nr] | int sp[nr] | int off[nt+1] | int nact[ncls] | ushort act[ncls][Fa]
+template <class T>
+struct AngSmem {
+  int par, tab, ds, acc, red, extra, pos, sp, off, nact, act, total;
+};
+template <class T>
+static inline AngSmem<T> ang_smem(int nr, int nt, int ncls, int Fa, int chunk, int nval, int extra) {
+  AngSmem<T> L;
+  int o = 0;
+  auto take = [&](int bytes) { int r = o; o += (bytes + 15) & ~15; return r; };
+  const int es = (int)sizeof(T);
+  L.par = take(ncls * chunk * 4 * es);
+  L.tab = take(nt * chunk * nr * 2 * es);
+  L.ds = take(nr * es);
+  L.acc = take(Fa * es);
+  L.red = take(nval ? nt * (nt + 1) / 2 * ANG_WARPS * nval * es : 0);
+  L.extra = take(extra * es);
+  L.pos = take(nr * 4);
+  L.sp = take(nr * 4);
+  L.off = take((nt + 1) * 4);
+  L.nact = take(ncls * 4);
+  L.act = take(ncls * Fa * 2);
+  L.total = o;
+  return L;
+}
+
+template <class T>
+struct AngStage {
+  typedef typename Vec4<T>::type T4;
+  typedef typename Vec2<T>::type T2;
+  int m, Tn;
+  T4* par;
+  T2* tab;
+  T *ds, *acc, *red, *extra;
+  int *pos, *sp, *off, *nact;
+  unsigned short* act;
+  const T* et;
+  __device__ __forceinline__ void carve(unsigned char* p, const AngSmem<T>& L) {
+    par = reinterpret_cast<T4*>(p + L.par);
+    tab = reinterpret_cast<T2*>(p + L.tab);
+    ds = reinterpret_cast<T*>(p + L.ds);
+    acc = reinterpret_cast<T*>(p + L.acc);
+    red = reinterpret_cast<T*>(p + L.red);
+    extra = reinterpret_cast<T*>(p + L.extra);
+    pos = reinterpret_cast<int*>(p + L.pos);
+    sp = reinterpret_cast<int*>(p + L.sp);
+    off = reinterpret_cast<int*>(p + L.off);
+    nact = reinterpret_cast<int*>(p + L.nact);
+    act = reinterpret_cast<unsigned short*>(p + L.act);
+  }
+  // Warp 0 groups the angular neighbours by species (pos[g]: sorted position of the g-th grouped one, sp[g] its
+  // species); the other warps list the channels of every class whose squared embedding is not zero.
+  __device__ __forceinline__ void init(const AngArgs<T>& a, size_t base) {
+    m = a.numtriplet[base];
+    if (m > a.nr) m = a.nr;
+    const long long Tl = (long long)m * (m - 1) / 2;
+    Tn = Tl < a.na ? (int)Tl : a.na;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    if (w == 0) {
+      const int* row = a.im2 + base * (a.nr + 1) + 1;
+      for (int k = lane; k < m; k += 32) {
+        sp[k] = a.type_map[row[k]];  // by position for now
+        ds[k] = a.ds3[base * a.nr + k];
+      }
+      __syncwarp();
+      int o = 0;
+      for (int q = 0; q < a.nt; q++) {
+        if (lane == 0) off[q] = o;
+        for (int k0 = 0; k0 < m; k0 += 32) {
+          const int k = k0 + lane;
+          const bool p = k < m && sp[k] == q;
+          const unsigned bal = __ballot_sync(0xffffffffu, p);
+          if (p) pos[o + __popc(bal & lt)] = k;
+          o += __popc(bal);
+        }
+      }
+      if (lane == 0) off[a.nt] = o;
+    } else {
+      for (int s = w - 1; s < a.ncls; s += ANG_WARPS - 1) {
+        int n = 0;
+        for (int c0 = 0; c0 < a.Fa; c0 += 32) {
+          const int c = c0 + lane;
+          const bool p = c < a.Fa && a.e3[(size_t)s * a.Fa + c] != T(0);
+          const unsigned bal = __ballot_sync(0xffffffffu, p);
+          if (p) act[s * a.Fa + n + __popc(bal & lt)] = (unsigned short)c;
+          n += __popc(bal);
+        }
+        if (lane == 0) nact[s] = n;
+      }
+    }
+    for (int c = threadIdx.x; c < a.Fa; c += ANG_THREADS) acc[c] = T(0);
+    __syncthreads();
+    for (int q = 0; q < a.nt; q++)  // species by group from now on
+      for (int g = off[q] + threadIdx.x; g < off[q + 1]; g += ANG_THREADS) sp[g] = q;
+  }
+  __device__ __forceinline__ int most_channels(const AngArgs<T>& a) const {
+    int n = 0;
+    for (int s = 0; s < a.ncls; s++) n = max(n, nact[s]);
+    return n;
+  }
+  // channels of class s in the pass that starts at channel p0
+  __device__ __forceinline__ int channels(const AngArgs<T>& a, int s, int p0) const {
+    return max(0, min(a.chunk, nact[s] - p0));
+  }
+  // parameters and tables of a pass; block barriers on both sides
+  __device__ __forceinline__ void tables(const AngArgs<T>& a, int p0) {
+    __syncthreads();
+    for (int q = threadIdx.x; q < a.ncls * a.chunk; q += ANG_THREADS) {
+      const int s = q / a.chunk, i = q - s * a.chunk;
+      T4 v;
+      v.x = v.y = v.z = v.w = T(0);
+      if (p0 + i < nact[s]) {
+        const int c = act[s * a.Fa + p0 + i];
+        const T* al = a.alpha3b + ((size_t)s * a.Fa + c) * 3;
+        v.x = al[0]; v.y = al[1]; v.z = al[2]; v.w = a.e3[(size_t)s * a.Fa + c];
+      }
+      par[q] = v;
+    }
+    __syncthreads();
+    const int ng = off[a.nt];
+    for (int q = threadIdx.x; q < a.nt * a.chunk * ng; q += ANG_THREADS) {
+      const int g = q % ng, qc = q / ng, i = qc % a.chunk, tq = qc / a.chunk, s = sp[g] + tq;
+      if (s < a.ncls && p0 + i < nact[s]) {
+        const T4 v = par[s * a.chunk + i];
+        const T d = ds[pos[g]];
+        T2 e;
+        e.x = op_exp(v.x * d, et);
+        e.y = op_exp(v.y * d, et);
+        tab[qc * a.nr + g] = e;
+      }
+    }
+    __syncthreads();
+  }
+  // slot of the triplet of sorted positions j < k
+  __device__ __forceinline__ int slot(int j, int k) const { return (j * (2 * m - j - 1)) / 2 + k - j - 1; }
+};
+
+// The p-th pair of class (ta, tb): grouped indices ga (species ta), gb (species tb).
+template <class T>
+__device__ __forceinline__ void class_pair(const AngStage<T>& st, int ta, int tb, int p, int& ga, int& gb) {
+  const int oa = st.off[ta], na_ = st.off[ta + 1] - oa, ob = st.off[tb], nb_ = st.off[tb + 1] - ob;
+  if (ta == tb) {
+    unrank_pair(p, na_, ga, gb);
+    ga += oa; gb += oa;
+  } else {
+    const int r = p / nb_;
+    ga = oa + r; gb = ob + p - r * nb_;
+  }
+}
+template <class T>
+__device__ __forceinline__ int class_pairs(const AngStage<T>& st, int ta, int tb) {
+  const int na_ = st.off[ta + 1] - st.off[ta], nb_ = st.off[tb + 1] - st.off[tb];
+  return ta == tb ? na_ * (na_ - 1) / 2 : na_ * nb_;
+}
+
+// Sums of NV values per thread over the block, left in red[warp][NV] for sum_warps() behind the next barrier.
+template <class T, int NV>
+__device__ __forceinline__ void leave_sums(T (&v)[NV], T* red) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  constexpr int SH = NV == 32 ? 0 : (NV == 16 ? 1 : 2);  // log2(32 / NV)
+  const T tot = multi_reduce<T, NV>(v, lane);
+  if ((lane & ((1 << SH) - 1)) == 0) red[w * NV + (lane >> SH)] = tot;
+}
+template <class T, int NV>
+__device__ __forceinline__ T sum_warps(const T* red, int i) {
+  T s = T(0);
+#pragma unroll
+  for (int w = 0; w < ANG_WARPS; w++) s += red[w * NV + i];
+  return s;
+}
+
+// MODE 0: fingerprints (ComputeSortProj3body); 1: their parameter gradient (ComputeSortProj3bodyGrad); 2: backward of
+// the angular force (ComputeForceTriplGrad).  Per triplet the force cotangent of 2 enters only through three scalars,
+//   Q  = sum_a (Fb_j-Fb_i)_a dt/d(ij)_a + (Fb_k-Fb_i)_a dt/d(ik)_a,
+//   Pj = sum_a (Fb_j-Fb_i)_a dfc_j,a,   Pk = sum_a (Fb_k-Fb_i)_a dfc_k,a,
+// and with Z1 = e^{bt} exp(a1 sj + a2 sk), Z2 with j, k exchanged, g = 1 + bt, H1 = g Q/2 + (t/2)(a1 Pj + a2 Pk), H2
+// with Pj, Pk exchanged, the channel's gradnet term is Z1 H1 + Z2 H2 and the parameter terms are its derivatives.
+template <class T, int MODE>
+__global__ void __launch_bounds__(ANG_THREADS) k_ang_sums(AngArgs<T> a, AngSmem<T> L, VirArgs<T> va) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ T et[16];
+  typedef typename Vec4<T>::type T4;
+  typedef typename Vec2<T>::type T2;
+  constexpr int PER = MODE == 0 ? 1 : (MODE == 1 ? 3 : 4), NV = MODE == 0 ? 8 : 32;
+  AngStage<T> st;
+  st.carve(smem_raw, L);
+  st.et = et;
+  exp_table_load(et);
+  // 1, 2: directly behind the zero fill of their outputs, so everything they read is at least two kernels old
+  if (MODE == 0) chain_wait();
+  const size_t base = blockIdx.x;
+  st.init(a, base);
+  T* dF = st.extra;           // 2: [nr][3] Fbar_k - Fbar_i
+  T* pn = st.extra + 3 * a.nr;  //    [nr] their projections on dfc
+  if (MODE == 2) {
+    const int b = (int)(base / a.Nl), ipar = (int)(base - (size_t)b * a.Nl) + species_shift(a.tipos, a.actual_type);
+    const T* pgb = a.prevgrad + (size_t)b * a.N * 3;
+    for (int k = threadIdx.x; k < st.m; k += ANG_THREADS) {
+      const int id = a.im2[base * (a.nr + 1) + 1 + k];
+      T wd[3] = {T(0), T(0), T(0)}, p = T(0);
+      if (va.wbar) {  // grad_force/ang/reforce.cu.cc:274-446
+        T r[3];
+        mic_cart(va.pos + ((size_t)b * a.N + ipar) * 3, va.pos + ((size_t)b * a.N + id) * 3, va.box + (size_t)b * 6, r);
+        const T* Wg = va.wbar + (size_t)b * 9;
+#pragma unroll
+        for (int x = 0; x < 3; x++) wd[x] = Wg[x * 3] * r[0] + Wg[x * 3 + 1] * r[1] + Wg[x * 3 + 2] * r[2];
+      }
+#pragma unroll
+      for (int x = 0; x < 3; x++) {
+        const T d = pgb[(size_t)id * 3 + x] - pgb[(size_t)ipar * 3 + x] - wd[x];
+        dF[k * 3 + x] = d;
+        p += d * a.der3bsupp[(base * 3 + x) * a.nr + k];
+      }
+      pn[k] = p;
+    }
+  }
+  const T* t_row = a.ang + base * a.na;
+  const T2* d3 = MODE == 2 ? reinterpret_cast<const T2*>(a.der3b) + base * 3 * a.na : nullptr;
+  const int most = st.most_channels(a);
+  for (int p0 = 0; p0 < most; p0 += a.chunk) {
+    st.tables(a, p0);
+    int ci = 0;
+    for (int ta = 0; ta < a.nt; ta++) {
+      for (int tb = ta; tb < a.nt; tb++, ci++) {
+        const int s = ta + tb;
+        if (s >= a.ncls) continue;
+        const int nch = st.channels(a, s, p0), np = class_pairs(st, ta, tb);
+        T v[NV];
+#pragma unroll
+        for (int x = 0; x < NV; x++) v[x] = T(0);
+        const T4* par = st.par + s * a.chunk;
+        const T2* tA = st.tab + (size_t)tb * a.chunk * a.nr;  // entries of the ta neighbours for partners of species tb
+        const T2* tB = st.tab + (size_t)ta * a.chunk * a.nr;
+        if (nch > 0)
+          for (int p = threadIdx.x; p < np; p += ANG_THREADS) {
+            int ga, gb;
+            class_pair(st, ta, tb, p, ga, gb);
+            const int ka = st.pos[ga], kb = st.pos[gb];
+            const int nn = st.slot(min(ka, kb), max(ka, kb));
+            if (nn >= st.Tn) continue;
+            const T t = t_row[nn], sa = st.ds[ka], sb = st.ds[kb];
+            T Qh = T(0), Pa = T(0), Pb = T(0);
+            if (MODE == 2) {
+              const int j = min(ka, kb), k = max(ka, kb);
+#pragma unroll
+              for (int x = 0; x < 3; x++) {
+                const T2 id = d3[(size_t)x * a.na + nn];
+                Qh += dF[j * 3 + x] * id.x + dF[k * 3 + x] * id.y;
+              }
+              Qh *= T(0.5);
+              Pa = T(0.5) * t * pn[ka];
+              Pb = T(0.5) * t * pn[kb];
+            }
+#pragma unroll
+            for (int c = 0; c < ANG_CH; c++) {
+              if (c >= nch) break;
+              const T4 pr = par[c];
+              const T2 A = tA[c * a.nr + ga], B = tB[c * a.nr + gb];
+              const T E = op_exp(pr.z * t, et);
+              const T Z1 = E * (A.x * B.y), Z2 = E * (A.y * B.x);
+              if (MODE == 0) v[c] += t * (Z1 + Z2);
+              if (MODE == 1) {
+                v[4 * c] += t * (Z1 * sa + Z2 * sb);
+                v[4 * c + 1] += t * (Z1 * sb + Z2 * sa);
+                v[4 * c + 2] += t * t * (Z1 + Z2);
+              }
+              if (MODE == 2) {
+                const T gQ = (T(1) + pr.z * t) * Qh;
+                const T H1 = gQ + pr.x * Pa + pr.y * Pb, H2 = gQ + pr.x * Pb + pr.y * Pa;
+                v[4 * c] += Z1 * H1 + Z2 * H2;
+                v[4 * c + 1] += Z1 * (sa * H1 + Pa) + Z2 * (sb * H2 + Pb);
+                v[4 * c + 2] += Z1 * (sb * H1 + Pb) + Z2 * (sa * H2 + Pa);
+                v[4 * c + 3] += t * (Z1 * (H1 + Qh) + Z2 * (H2 + Qh));
+              }
+            }
+          }
+        leave_sums<T, NV>(v, st.red + ci * ANG_WARPS * NV);
+      }
+    }
+    if (MODE != 0) chain_wait();
+    __syncthreads();
+    // totals: fingerprints and gradnet per channel in acc (a channel may belong to several classes), parameter
+    // gradients to global memory, one add per block
+    ci = 0;
+    for (int ta = 0; ta < a.nt; ta++) {
+      for (int tb = ta; tb < a.nt; tb++, ci++) {
+        const int s = ta + tb;
+        if (s >= a.ncls) continue;
+        const int nch = st.channels(a, s, p0);
+        const T* red = st.red + ci * ANG_WARPS * NV;
+        for (int x = threadIdx.x; x < nch * PER; x += ANG_THREADS) {
+          const int i = x / PER, k = x - i * PER, c = st.act[s * a.Fa + p0 + i];
+          const T f = T(0.5) * st.par[s * a.chunk + i].w * sum_warps<T, NV>(red, MODE == 0 ? i : 4 * i + k);
+          if (MODE == 0 || (MODE == 2 && k == 0)) st.acc[c] += f;  // one thread per channel of the class
+          else {
+            const T g = f * (MODE == 1 ? a.prevgrad[base * a.Fa + c] : a.netderiv[base * a.Fa + c]);
+            atomicAdd(a.g_alpha3 + ((size_t)s * a.Fa + c) * 3 + (MODE == 1 ? k : k - 1), g);
+          }
+        }
+        __syncthreads();
+      }
+    }
+  }
+  if (MODE != 0) chain_wait();
+  if (MODE != 1) {
+    __syncthreads();
+    for (int c = threadIdx.x; c < a.Fa; c += ANG_THREADS) a.out[base * a.Fa + c] = st.acc[c];
+  }
+  if (MODE != 0 && base == 0)
+    for (int c = threadIdx.x; c < a.zero_n; c += ANG_THREADS) a.zero[c] = T(0);
 }
 
 // ---------------------------------------------------------------- radial force (ComputeForceRadial)
@@ -146,6 +558,7 @@ __global__ void __launch_bounds__(OPS_THREADS)
                 VirArgs<T> va) {
   const int gi = blockIdx.x * OPS_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (gi >= natoms) return;
+  chain_wait();
   const int b = gi / Nl, par = gi - b * Nl;
   const int ipar = par + species_shift(tipos, actual_type);
   const size_t base = gi;
@@ -203,77 +616,108 @@ __global__ void __launch_bounds__(OPS_THREADS)
 }
 
 // ---------------------------------------------------------------- angular force (ComputeForceTripl)
+// Ordered pairs: four threads share a neighbour and walk its partners, so that the force on it stays in registers
+// until the end; every triplet is evaluated from both sides (one exponential per channel each).
+constexpr int ANG_TPO = 4;
 template <class T>
-__global__ void __launch_bounds__(OPS_THREADS)
-    k_force_ang(int Nl, int N, int nr, int na, int Fa, const T* __restrict__ netderiv, const T* __restrict__ ds3,
-                const T* __restrict__ ang, const T* __restrict__ der3bsupp, const T* __restrict__ der3b,
-                const int* __restrict__ im2, const T* __restrict__ alpha3b, const T* __restrict__ e3,
-                const int* __restrict__ type_map, const int* __restrict__ tipos, const int* __restrict__ actual_type,
-                const int* __restrict__ numtriplet, T* __restrict__ force, VirArgs<T> va) {
-  extern __shared__ unsigned char smem_raw[];
-  __shared__ T red[OPS_WARPS + 1];
+__global__ void __launch_bounds__(ANG_THREADS) k_force_ang(AngArgs<T> a, AngSmem<T> L, VirArgs<T> va) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ T et[16];
+  __shared__ T red[ANG_WARPS + 1];
+  typedef typename Vec4<T>::type T4;
   typedef typename Vec2<T>::type T2;
   AngStage<T> st;
-  st.ds = reinterpret_cast<T*>(smem_raw);
-  T* dsup = st.ds + nr;       // [3][nr] der3bsupp row
-  T* fnb = dsup + 3 * nr;     // [nr][3] neighbour force accumulators
-  T* nd = fnb + 3 * nr;       // [Fa]
-  st.tj = reinterpret_cast<int*>(nd + Fa);
-  int* ids = st.tj + nr;
-  st.jk = reinterpret_cast<unsigned short*>(ids + nr);
+  st.carve(smem_raw, L);
+  st.et = et;
+  exp_table_load(et);
   const size_t base = blockIdx.x;
-  const int b = (int)(base / Nl), par = (int)(base - (size_t)b * Nl);
-  const int ipar = par + species_shift(tipos, actual_type);
-  for (int k = threadIdx.x; k < nr; k += OPS_THREADS) {
-    ids[k] = im2[base * (nr + 1) + 1 + k];
-    for (int a = 0; a < 3; a++) {
-      dsup[a * nr + k] = der3bsupp[(base * 3 + a) * nr + k];
-      fnb[k * 3 + a] = T(0);
-    }
-  }
-  for (int c = threadIdx.x; c < Fa; c += OPS_THREADS) nd[c] = netderiv[base * Fa + c];
-  ang_stage(st, base, nr, na, numtriplet, im2, ds3, type_map);
-  const T2* d3 = reinterpret_cast<const T2*>(der3b) + base * 3 * na;
-  T fx = T(0), fy = T(0), fz = T(0);
-  for (int nn = threadIdx.x; nn < st.Tn; nn += OPS_THREADS) {
-    const int j = st.jk[nn] >> 8, k = st.jk[nn] & 255;
-    const int s = st.tj[j] + st.tj[k];
-    const T t = ang[base * na + nn], rj = st.ds[j], rk = st.ds[k];
-    T D = T(0), BJ = T(0), BK = T(0);
-    for (int c = 0; c < Fa; c++) {
-      const T ch = e3[s * Fa + c];
-      if (ch == T(0)) continue;
-      const T ax = alpha3b[(s * Fa + c) * 3], ay = alpha3b[(s * Fa + c) * 3 + 1], az = alpha3b[(s * Fa + c) * 3 + 2];
-      const T w = T(0.5) * nd[c] * ch;
-      const T eb = r_exp(az * t);
-      const T sim1 = r_exp(ay * rj + ax * rk), sim2 = r_exp(ax * rj + ay * rk);
-      D += w * (eb * (T(1.) + az * t) * (sim1 + sim2) * T(0.5));
-      BJ += w * ((ax * sim2 + ay * sim1) * eb * T(0.5) * t);
-      BK += w * ((ax * sim1 + ay * sim2) * eb * T(0.5) * t);
-    }
-    T fj[3], fk[3];
+  const int b = (int)(base / a.Nl), par_ = (int)(base - (size_t)b * a.Nl);
+  const int ipar = par_ + species_shift(a.tipos, a.actual_type);
+  st.init(a, base);
+  T* fnb = st.extra;  // [nr][3] force on the neighbour at sorted position k
+  for (int q = threadIdx.x; q < 3 * a.nr; q += ANG_THREADS) fnb[q] = T(0);
+  const T* t_row = a.ang + base * a.na;
+  const T2* d3 = reinterpret_cast<const T2*>(a.der3b) + base * 3 * a.na;
+  const int most = st.most_channels(a), ng = st.off[a.nt], sub = threadIdx.x & (ANG_TPO - 1);
+  for (int p0 = 0; p0 < most; p0 += a.chunk) {
+    st.tables(a, p0);
+    for (int g0 = 0; g0 < ng; g0 += ANG_THREADS / ANG_TPO) {
+      const int g = g0 + threadIdx.x / ANG_TPO;
+      T f[3] = {T(0), T(0), T(0)};
+      if (g < ng) {
+        const int kj = st.pos[g], tj = st.sp[g];
+        T sup = T(0);
+        for (int tq = 0; tq < a.nt; tq++) {
+          const int s = tj + tq;
+          if (s >= a.ncls) continue;
+          const int nch = st.channels(a, s, p0);
+          if (nch <= 0) continue;
+          const T4* par = st.par + s * a.chunk;
+          const T2* tA = st.tab + (size_t)tq * a.chunk * a.nr + g;
+          const T2* tB = st.tab + (size_t)tj * a.chunk * a.nr;
+          T w[ANG_CH];
+          T2 A[ANG_CH];
 #pragma unroll
-    for (int a = 0; a < 3; a++) {
-      const T2 id = d3[(size_t)a * na + nn];
-      fj[a] = D * id.x + BJ * dsup[a * nr + j];
-      fk[a] = D * id.y + BK * dsup[a * nr + k];
-      atomicAdd(&fnb[j * 3 + a], fj[a]);
-      atomicAdd(&fnb[k * 3 + a], fk[a]);
+          for (int c = 0; c < ANG_CH; c++) {
+            w[c] = T(0);
+            A[c].x = A[c].y = T(0);
+            if (c < nch) {
+              w[c] = T(0.25) * a.netderiv[base * a.Fa + st.act[s * a.Fa + p0 + c]] * par[c].w;
+              A[c] = tA[c * a.nr];
+              A[c].x *= w[c]; A[c].y *= w[c];
+            }
+          }
+          for (int h = st.off[tq] + sub; h < st.off[tq + 1]; h += ANG_TPO) {
+            if (h == g) continue;
+            const int kk = st.pos[h];
+            const int nn = st.slot(min(kj, kk), max(kj, kk));
+            if (nn >= st.Tn) continue;
+            const T t = t_row[nn];
+            T D = T(0), B = T(0);
+#pragma unroll
+            for (int c = 0; c < ANG_CH; c++) {
+              if (c >= nch) break;
+              const T4 pr = par[c];
+              const T2 P = tB[c * a.nr + h];
+              const T E = op_exp(pr.z * t, et);
+              const T Z1 = E * (A[c].x * P.y), Z2 = E * (A[c].y * P.x);
+              D += (T(1) + pr.z * t) * (Z1 + Z2);
+              B += pr.x * Z1 + pr.y * Z2;
+            }
+            sup += B * t;
+            const bool first = kj < kk;
+#pragma unroll
+            for (int x = 0; x < 3; x++) {
+              const T2 id = d3[(size_t)x * a.na + nn];
+              f[x] += D * (first ? id.x : id.y);
+            }
+          }
+        }
+#pragma unroll
+        for (int x = 0; x < 3; x++) f[x] += sup * a.der3bsupp[(base * 3 + x) * a.nr + kj];
+      }
+#pragma unroll
+      for (int x = 0; x < 3; x++) {
+        f[x] += __shfl_xor_sync(0xffffffffu, f[x], 1);
+        f[x] += __shfl_xor_sync(0xffffffffu, f[x], 2);
+      }
+      if (g < ng && sub < 3) fnb[st.pos[g] * 3 + sub] += sub == 0 ? f[0] : (sub == 1 ? f[1] : f[2]);
     }
-    fx -= fj[0] + fk[0];
-    fy -= fj[1] + fk[1];
-    fz -= fj[2] + fk[2];
   }
-  fx = block_sum<T, OPS_WARPS>(fx, red);
-  fy = block_sum<T, OPS_WARPS>(fy, red);
-  fz = block_sum<T, OPS_WARPS>(fz, red);
   __syncthreads();
-  T* fb = force + (size_t)b * N * 3;
-  for (int q = threadIdx.x; q < st.m * 3; q += OPS_THREADS) atomicAdd(fb + (size_t)ids[q / 3] * 3 + (q % 3), fnb[q]);
-  if (threadIdx.x == 0) {
-    atomicAdd(fb + (size_t)ipar * 3 + 0, fx);
-    atomicAdd(fb + (size_t)ipar * 3 + 1, fy);
-    atomicAdd(fb + (size_t)ipar * 3 + 2, fz);
+  chain_wait();
+  T* fb = a.out + (size_t)b * a.N * 3;
+  const int* row = a.im2 + base * (a.nr + 1) + 1;
+  T fi[3] = {T(0), T(0), T(0)};
+  for (int k = threadIdx.x; k < st.m; k += ANG_THREADS) {
+#pragma unroll
+    for (int x = 0; x < 3; x++) fi[x] -= fnb[k * 3 + x];
+  }
+  for (int q = threadIdx.x; q < st.m * 3; q += ANG_THREADS) atomicAdd(fb + (size_t)row[q / 3] * 3 + (q % 3), fnb[q]);
+#pragma unroll
+  for (int x = 0; x < 3; x++) {
+    const T v = block_sum<T, ANG_WARPS>(fi[x], red);
+    if (threadIdx.x == 0) atomicAdd(fb + (size_t)ipar * 3 + x, v);
   }
   if (va.virial && threadIdx.x < 32) {
     // W_ab -= f_ij,a r_ij,b + f_ik,a r_ik,b (force/ang/reforce.cu.cc:269-457): every force this centre puts on
@@ -283,274 +727,17 @@ __global__ void __launch_bounds__(OPS_THREADS)
     for (int c = 0; c < 9; c++) w[c] = T(0);
     for (int k = threadIdx.x; k < st.m; k += 32) {
       T r[3];
-      mic_cart(va.pos + ((size_t)b * N + ipar) * 3, va.pos + ((size_t)b * N + ids[k]) * 3, va.box + (size_t)b * 6, r);
+      mic_cart(va.pos + ((size_t)b * a.N + ipar) * 3, va.pos + ((size_t)b * a.N + row[k]) * 3, va.box + (size_t)b * 6, r);
 #pragma unroll
-      for (int a = 0; a < 3; a++)
+      for (int x = 0; x < 3; x++)
 #pragma unroll
-        for (int c = 0; c < 3; c++) w[a * 3 + c] -= fnb[k * 3 + a] * r[c];
+        for (int c = 0; c < 3; c++) w[x * 3 + c] -= fnb[k * 3 + x] * r[c];
     }
 #pragma unroll
     for (int c = 0; c < 9; c++) {
       const T v = warp_sum(w[c]);
       if (threadIdx.x == 0) atomicAdd(va.virial + (size_t)b * 9 + c, v);
     }
-  }
-}
-
-// ---------------------------------------------------------------- d/d(alpha2b) of the radial AF (ComputeTwoBodyParGrad)
-template <class T>
-__global__ void __launch_bounds__(OPS_THREADS)
-    k_grad_af_rad(int natoms, int nr, int Fr, int nt, const T* __restrict__ prevgrad, const T* __restrict__ rad,
-                  const int* __restrict__ im2, const T* __restrict__ alpha2b, const T* __restrict__ e2,
-                  const int* __restrict__ type_map, T* __restrict__ g_alpha, T* __restrict__ g_emb) {
-  const int gi = blockIdx.x * OPS_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (gi >= natoms) return;
-  const size_t base = gi;
-  int n = im2[base * (nr + 1)];
-  if (n > nr) n = nr;
-  for (int c = 0; c < Fr; c++) {
-    const T pg = prevgrad[base * Fr + c];
-    T ga[STAFB_MAX_TYPES], ge[STAFB_MAX_TYPES];
-#pragma unroll
-    for (int t = 0; t < STAFB_MAX_TYPES; t++) ga[t] = ge[t] = T(0);
-    for (int j = lane; j < n; j += 32) {
-      const T d = rad[base * nr + j];
-      const int tj = type_map[im2[base * (nr + 1) + 1 + j]];
-      const T ex = r_exp(alpha2b[tj * Fr + c] * d);
-      const T va = d * d * (ex * e2[tj * Fr + c] * pg);
-      const T ve = d * (ex * pg);
-#pragma unroll
-      for (int t = 0; t < STAFB_MAX_TYPES; t++)
-        if (t == tj) { ga[t] += va; ge[t] += ve; }
-    }
-#pragma unroll
-    for (int t = 0; t < STAFB_MAX_TYPES; t++) {
-      if (t >= nt) break;
-      const T sa = warp_sum(ga[t]), se = warp_sum(ge[t]);
-      if (lane == 0) {
-        if (sa != T(0)) atomicAdd(g_alpha + t * Fr + c, sa);
-        if (se != T(0)) atomicAdd(g_emb + t * Fr + c, se);
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------- d/d(alpha3b) of the angular AF (ComputeSortProj3bodyGrad)
-template <class T>
-__global__ void __launch_bounds__(OPS_THREADS)
-    k_grad_af_ang(int nr, int na, int Fa, int ncls, const T* __restrict__ prevgrad, const T* __restrict__ ang,
-                  const T* __restrict__ ds3, const int* __restrict__ im2, const T* __restrict__ alpha3b,
-                  const T* __restrict__ e3, const int* __restrict__ type_map, const int* __restrict__ numtriplet,
-                  T* __restrict__ g_alpha3) {
-  extern __shared__ unsigned char smem_raw[];
-  __shared__ T red[OPS_WARPS + 1];
-  AngStage<T> st;
-  st.ds = reinterpret_cast<T*>(smem_raw);
-  st.tj = reinterpret_cast<int*>(st.ds + nr);
-  st.jk = reinterpret_cast<unsigned short*>(st.tj + nr);
-  const size_t base = blockIdx.x;
-  ang_stage(st, base, nr, na, numtriplet, im2, ds3, type_map);
-  const T* t_row = ang + base * na;
-  for (int c = 0; c < Fa; c++) {
-    const T pg = prevgrad[base * Fa + c];
-    for (int s = 0; s < ncls; s++) {
-      const T ch = e3[s * Fa + c];
-      if (ch == T(0)) continue;
-      const T a1 = alpha3b[(s * Fa + c) * 3], a2 = alpha3b[(s * Fa + c) * 3 + 1], be = alpha3b[(s * Fa + c) * 3 + 2];
-      T g1 = T(0), g2 = T(0), g3 = T(0);
-      for (int nn = threadIdx.x; nn < st.Tn; nn += OPS_THREADS) {
-        const int j = st.jk[nn] >> 8, k = st.jk[nn] & 255;
-        if (st.tj[j] + st.tj[k] != s) continue;
-        const T t = t_row[nn], dj = st.ds[j], dy = st.ds[k];
-        const T e12 = r_exp(a1 * dj + a2 * dy), e21 = r_exp(a1 * dy + a2 * dj), bt = r_exp(be * t);
-        const T common = pg * ch * bt * t / T(2.);
-        g1 += common * (e12 * dj + e21 * dy);
-        g2 += common * (e12 * dy + e21 * dj);
-        g3 += common * (e12 + e21) * t;
-      }
-      g1 = block_sum<T, OPS_WARPS>(g1, red);
-      g2 = block_sum<T, OPS_WARPS>(g2, red);
-      g3 = block_sum<T, OPS_WARPS>(g3, red);
-      if (threadIdx.x == 0) {
-        atomicAdd(g_alpha3 + (s * Fa + c) * 3 + 0, g1);
-        atomicAdd(g_alpha3 + (s * Fa + c) * 3 + 1, g2);
-        atomicAdd(g_alpha3 + (s * Fa + c) * 3 + 2, g3);
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------- backward of the radial force (ComputeForceRadialGrad)
-template <class T>
-__global__ void __launch_bounds__(OPS_THREADS)
-    k_grad_force_rad(int natoms, int Nl, int N, int nr, int Fr, int nt, const T* __restrict__ prevgrad,
-                     const T* __restrict__ netderiv, const T* __restrict__ der2b, const int* __restrict__ im2,
-                     const T* __restrict__ rad, const T* __restrict__ alpha2b, const T* __restrict__ e2,
-                     const int* __restrict__ type_map, const int* __restrict__ tipos,
-                     const int* __restrict__ actual_type, T* __restrict__ gradnet, T* __restrict__ g_alpha,
-                     T* __restrict__ g_emb, VirArgs<T> va) {
-  const int gi = blockIdx.x * OPS_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (gi >= natoms) return;
-  const int b = gi / Nl, par = gi - b * Nl;
-  const int ipar = par + species_shift(tipos, actual_type);
-  const size_t base = gi;
-  int n = im2[base * (nr + 1)];
-  if (n > nr) n = nr;
-  const T* pgb = prevgrad + (size_t)b * N * 3;
-  const T pix = pgb[ipar * 3], piy = pgb[ipar * 3 + 1], piz = pgb[ipar * 3 + 2];
-  // q_j = sum_a (Fbar_j - Fbar_i)_a * 0.5 * dd/dr_{i,a}, per neighbour (two slots per lane cover nr <= 64;
-  // the loop handles any nr)
-  for (int c = 0; c < Fr; c++) {
-    const T NG = netderiv[base * Fr + c];
-    T gn = T(0);
-    T ga[STAFB_MAX_TYPES], ge[STAFB_MAX_TYPES];
-#pragma unroll
-    for (int t = 0; t < STAFB_MAX_TYPES; t++) ga[t] = ge[t] = T(0);
-    for (int j = lane; j < n; j += 32) {
-      const int nj = im2[base * (nr + 1) + 1 + j];
-      const int tj = type_map[nj];
-      const T d = rad[base * nr + j];
-      T wd[3] = {T(0), T(0), T(0)};
-      if (va.wbar) {  // the virial cotangent shifts the neighbour's force cotangent by -(Wbar r) (grad_force/rad/reforce.cu.cc:165-234)
-        T r[3];
-        mic_cart(va.pos + ((size_t)b * N + ipar) * 3, va.pos + ((size_t)b * N + nj) * 3, va.box + (size_t)b * 6, r);
-        const T* Wg = va.wbar + (size_t)b * 9;
-#pragma unroll
-        for (int a = 0; a < 3; a++) wd[a] = Wg[a * 3] * r[0] + Wg[a * 3 + 1] * r[1] + Wg[a * 3 + 2] * r[2];
-      }
-      const T q = T(0.5) * ((pgb[nj * 3] - pix - wd[0]) * der2b[(base * 3 + 0) * nr + j] +
-                            (pgb[nj * 3 + 1] - piy - wd[1]) * der2b[(base * 3 + 1) * nr + j] +
-                            (pgb[nj * 3 + 2] - piz - wd[2]) * der2b[(base * 3 + 2) * nr + j]);
-      const T al = alpha2b[Fr * tj + c], ch = e2[Fr * tj + c];
-      const T s1 = r_exp(al * d);
-      const T sds = s1 * (T(1.) + al * d);
-      const T ba = ch * s1 * d * (T(2.) + al * d);
-      gn += q * ch * sds;
-      const T va = q * NG * ba, ve = q * NG * sds;
-#pragma unroll
-      for (int t = 0; t < STAFB_MAX_TYPES; t++)
-        if (t == tj) { ga[t] += va; ge[t] += ve; }
-    }
-    gn = warp_sum(gn);
-    if (lane == 0) gradnet[base * Fr + c] = gn;
-#pragma unroll
-    for (int t = 0; t < STAFB_MAX_TYPES; t++) {
-      if (t >= nt) break;
-      const T sa = warp_sum(ga[t]), se = warp_sum(ge[t]);
-      if (lane == 0) {
-        if (sa != T(0)) atomicAdd(g_alpha + t * Fr + c, sa);
-        if (se != T(0)) atomicAdd(g_emb + t * Fr + c, se);
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------- backward of the angular force (ComputeForceTriplGrad)
-// Per triplet the force cotangent enters only through three scalars,
-//   Q  = sum_a (Fb_j-Fb_i)_a dt/d(ij)_a + (Fb_k-Fb_i)_a dt/d(ik)_a,
-//   Pj = sum_a (Fb_j-Fb_i)_a dfc_j,a,   Pk = sum_a (Fb_k-Fb_i)_a dfc_k,a,
-// staged once in shared memory; every (class, channel) sweep then costs three exponentials.
-template <class T>
-__global__ void __launch_bounds__(OPS_THREADS)
-    k_grad_force_ang(int Nl, int N, int nr, int na, int Fa, int ncls, const T* __restrict__ prevgrad,
-                     const T* __restrict__ netderiv, const T* __restrict__ ds3, const T* __restrict__ ang,
-                     const T* __restrict__ der3bsupp, const T* __restrict__ der3b, const int* __restrict__ im2,
-                     const T* __restrict__ alpha3b, const T* __restrict__ e3, const int* __restrict__ type_map,
-                     const int* __restrict__ tipos, const int* __restrict__ actual_type,
-                     const int* __restrict__ numtriplet, T* __restrict__ gradnet, T* __restrict__ g_alpha3,
-                     VirArgs<T> va) {
-  extern __shared__ unsigned char smem_raw[];
-  __shared__ T red[OPS_WARPS + 1];
-  typedef typename Vec2<T>::type T2;
-  AngStage<T> st;
-  st.ds = reinterpret_cast<T*>(smem_raw);
-  T* pn = st.ds + nr;        // [nr] Pj per neighbour
-  T* dF = pn + nr;           // [nr][3] Fbar_j - Fbar_i
-  T* Q = dF + 3 * nr;        // [na]
-  st.tj = reinterpret_cast<int*>(Q + na);
-  st.jk = reinterpret_cast<unsigned short*>(st.tj + nr);
-  const size_t base = blockIdx.x;
-  const int b = (int)(base / Nl), par = (int)(base - (size_t)b * Nl);
-  const int ipar = par + species_shift(tipos, actual_type);
-  const T* pgb = prevgrad + (size_t)b * N * 3;
-  for (int k = threadIdx.x; k < nr; k += OPS_THREADS) {
-    const int id = im2[base * (nr + 1) + 1 + k];
-    T p = T(0);
-    T wd[3] = {T(0), T(0), T(0)};
-    if (va.wbar && k < numtriplet[base]) {  // grad_force/ang/reforce.cu.cc:274-446
-      T r[3];
-      mic_cart(va.pos + ((size_t)b * N + ipar) * 3, va.pos + ((size_t)b * N + id) * 3, va.box + (size_t)b * 6, r);
-      const T* Wg = va.wbar + (size_t)b * 9;
-#pragma unroll
-      for (int a = 0; a < 3; a++) wd[a] = Wg[a * 3] * r[0] + Wg[a * 3 + 1] * r[1] + Wg[a * 3 + 2] * r[2];
-    }
-    for (int a = 0; a < 3; a++) {
-      const T d = pgb[id * 3 + a] - pgb[ipar * 3 + a] - wd[a];
-      dF[k * 3 + a] = d;
-      p += d * der3bsupp[(base * 3 + a) * nr + k];
-    }
-    pn[k] = p;
-  }
-  ang_stage(st, base, nr, na, numtriplet, im2, ds3, type_map);
-  const T2* d3 = reinterpret_cast<const T2*>(der3b) + base * 3 * na;
-  for (int nn = threadIdx.x; nn < st.Tn; nn += OPS_THREADS) {
-    const int j = st.jk[nn] >> 8, k = st.jk[nn] & 255;
-    T q = T(0);
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-      const T2 id = d3[(size_t)a * na + nn];
-      q += dF[j * 3 + a] * id.x + dF[k * 3 + a] * id.y;
-    }
-    Q[nn] = q;
-  }
-  __syncthreads();
-  const T* t_row = ang + base * na;
-  for (int c = 0; c < Fa; c++) {
-    const T NG = netderiv[base * Fa + c];
-    T gn = T(0);
-    for (int s = 0; s < ncls; s++) {
-      const T ch = e3[s * Fa + c];
-      if (ch == T(0)) continue;
-      const T ax = alpha3b[(s * Fa + c) * 3], ay = alpha3b[(s * Fa + c) * 3 + 1], az = alpha3b[(s * Fa + c) * 3 + 2];
-      T g1 = T(0), g2 = T(0), g3 = T(0);
-      for (int nn = threadIdx.x; nn < st.Tn; nn += OPS_THREADS) {
-        const int j = st.jk[nn] >> 8, k = st.jk[nn] & 255;
-        if (st.tj[j] + st.tj[k] != s) continue;
-        const T t = t_row[nn], rj = st.ds[j], rk = st.ds[k];
-        const T q = Q[nn], pj = pn[j], pk = pn[k];
-        const T eb = r_exp(az * t);
-        const T sim1 = r_exp(ay * rj + ax * rk), sim2 = r_exp(ax * rj + ay * rk);
-        const T ss = sim1 + sim2;
-        const T h = T(0.5) * ch;
-        const T opb = T(1.) + az * t;
-        const T delta = eb * opb * ss * T(0.5);
-        const T suppj = (ax * sim2 + ay * sim1) * eb, suppk = (ax * sim1 + ay * sim2) * eb;
-        const T Bj = suppj * t * T(0.5), Bk = suppk * t * T(0.5);
-        gn += h * (delta * q + Bj * pj + Bk * pk);
-        const T ba1 = eb * opb * (sim1 * rk + sim2 * rj) * T(0.5);
-        const T ba2 = eb * opb * (sim1 * rj + sim2 * rk) * T(0.5);
-        const T bb = eb * t * (T(2.) + az * t) * ss * T(0.5);
-        const T et = eb * T(0.5) * t;
-        const T a1j = (sim2 + ax * sim2 * rj + ay * sim1 * rk) * et;
-        const T a2j = (sim1 + ay * sim1 * rj + ax * sim2 * rk) * et;
-        const T a1k = (sim1 + ax * sim1 * rk + ay * sim2 * rj) * et;
-        const T a2k = (sim2 + ay * sim2 * rk + ax * sim1 * rj) * et;
-        const T hn = h * NG;
-        g1 += hn * (ba1 * q + a1j * pj + a1k * pk);
-        g2 += hn * (ba2 * q + a2j * pj + a2k * pk);
-        g3 += hn * (bb * q + Bj * t * pj + Bk * t * pk);
-      }
-      g1 = block_sum<T, OPS_WARPS>(g1, red);
-      g2 = block_sum<T, OPS_WARPS>(g2, red);
-      g3 = block_sum<T, OPS_WARPS>(g3, red);
-      if (threadIdx.x == 0) {
-        atomicAdd(g_alpha3 + (s * Fa + c) * 3 + 0, g1);
-        atomicAdd(g_alpha3 + (s * Fa + c) * 3 + 1, g2);
-        atomicAdd(g_alpha3 + (s * Fa + c) * 3 + 2, g3);
-      }
-    }
-    gn = block_sum<T, OPS_WARPS>(gn, red);
-    if (threadIdx.x == 0) gradnet[base * Fa + c] = gn;
   }
 }
 
@@ -562,9 +749,61 @@ static int ops_check(stafb_ctx* c) {
   return STAFB_OK;
 }
 
+// Dynamic shared memory above 48 KB has to be asked for, per kernel and device.
+static cudaError_t opt_in(const void* kern, size_t bytes) {
+  return bytes > 48 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)
+                           : cudaSuccess;
+}
+
 static inline int ncls_of(int nt) {
   int C = nt * (nt + 1) / 2, smax = 2 * nt - 1;
   return C < smax ? C : smax;
+}
+
+// k_rad_sums on `n` atoms: at most eight warps' worth of blocks per SM, so that a warp's parameter sums cover several
+// atoms of a large batch before they meet the other warps' in global memory.
+template <class T, int MODE>
+static int launch_rad(cudaStream_t s, const RadArgs<T>& a, VirArgs<T> va = VirArgs<T>()) {
+  const size_t wb = rad_warp_bytes<T>(a.nr, a.nt, a.Fr), sm = wb * OPS_WARPS;
+  STAFB_CUDA_OK(opt_in((const void*)k_rad_sums<T, MODE>, sm));
+  const int blocks = (a.natoms + OPS_WARPS - 1) / OPS_WARPS, cap = MODE == 0 ? blocks : 148 * 8;
+  STAFB_CUDA_OK(launch_chained(k_rad_sums<T, MODE>, blocks < cap ? blocks : cap, OPS_THREADS, sm, s, a, wb, va));
+  return STAFB_OK;
+}
+
+// Shared memory of an angular operator: as many channels per pass as fit, ANG_CH if possible.
+template <class T>
+static int ang_layout(AngArgs<T>& a, int nval, int extra, AngSmem<T>& L) {
+  for (a.chunk = ANG_CH; a.chunk >= 1; a.chunk >>= 1) {
+    L = ang_smem<T>(a.nr, a.nt, a.ncls, a.Fa, a.chunk, nval, extra);
+    if (L.total <= 200 * 1024) return STAFB_OK;
+  }
+  return STAFB_ERR_CAPACITY;
+}
+template <class T, int MODE>
+static int launch_ang(cudaStream_t s, int blocks, AngArgs<T> a, VirArgs<T> va = VirArgs<T>()) {
+  AngSmem<T> L;
+  const int rc = ang_layout<T>(a, MODE == 0 ? 8 : 32, MODE == 2 ? 4 * a.nr : 0, L);
+  if (rc != STAFB_OK) return rc;
+  STAFB_CUDA_OK(opt_in((const void*)k_ang_sums<T, MODE>, (size_t)L.total));
+  STAFB_CUDA_OK(launch_chained(k_ang_sums<T, MODE>, blocks, ANG_THREADS, (size_t)L.total, s, a, L, va));
+  return STAFB_OK;
+}
+template <class T>
+static AngArgs<T> ang_args(stafb_ctx* c, const T* ang, const T* ds3, const int* im2, const T* a3, const T* e3,
+                           const int* tm, const int* ntr, int nt, int Fa) {
+  AngArgs<T> a = {};
+  a.nr = c->nr; a.na = c->na; a.Fa = Fa; a.nt = nt; a.ncls = ncls_of(nt);
+  a.ang = ang; a.ds3 = ds3; a.im2 = im2; a.alpha3b = a3; a.e3 = e3; a.type_map = tm; a.numtriplet = ntr;
+  return a;
+}
+template <class T>
+static RadArgs<T> rad_args(stafb_ctx* c, const T* rad, const int* im2, const T* a2, const T* e2, const int* tm, int n,
+                           int nt, int Fr) {
+  RadArgs<T> a = {};
+  a.natoms = n; a.nr = c->nr; a.Fr = Fr; a.nt = nt;
+  a.rad = rad; a.im2 = im2; a.alpha2b = a2; a.e2 = e2; a.type_map = tm;
+  return a;
 }
 
 template <class T>
@@ -572,9 +811,9 @@ int op_sort_proj(stafb_ctx* c, cudaStream_t s, const T* rad, const int* im2, con
                  const int* tm, int nf, int Nl, int nt, int Fr, T* out) {
   const int n = nf * Nl;
   if (n <= 0) return STAFB_OK;
-  k_af_rad<T><<<(n + OPS_WARPS - 1) / OPS_WARPS, OPS_THREADS, 0, s>>>(n, c->nr, Fr, rad, im2, a2, e2, tm, out);
-  STAFB_CUDA_OK(cudaGetLastError());
-  return STAFB_OK;
+  RadArgs<T> a = rad_args<T>(c, rad, im2, a2, e2, tm, n, nt, Fr);
+  a.out = out;
+  return launch_rad<T, 0>(s, a);
 }
 
 template <class T>
@@ -582,23 +821,20 @@ int op_sort_proj3(stafb_ctx* c, cudaStream_t s, const T* ang, const T* ds3, cons
                   const int* tm, const int* ntr, int nf, int Nl, int nt, int Fa, T* out) {
   const int n = nf * Nl;
   if (n <= 0) return STAFB_OK;
-  size_t sm = (size_t)c->nr * (sizeof(T) + sizeof(int)) + (size_t)c->na * 2;
-  k_af_ang<T><<<n, OPS_THREADS, sm, s>>>(c->nr, c->na, Fa, ncls_of(nt), ang, ds3, im2, a3, e3, tm, ntr, out);
-  STAFB_CUDA_OK(cudaGetLastError());
-  return STAFB_OK;
+  AngArgs<T> a = ang_args<T>(c, ang, ds3, im2, a3, e3, tm, ntr, nt, Fa);
+  a.out = out;
+  return launch_ang<T, 0>(s, n, a);
 }
 
 template <class T>
 int op_force_rad(stafb_ctx* c, cudaStream_t s, const T* nd, const T* der2b, const int* im2, const T* rad,
                  const T* a2, const T* e2, const int* tm, const int* tipos, const int* at, int nf, int Nl, int N,
                  int nt, int Fr, T* force, VirArgs<T> va = VirArgs<T>()) {
-  STAFB_CUDA_OK(cudaMemsetAsync(force, 0, sizeof(T) * (size_t)nf * 3 * N, s));
-  if (va.virial) STAFB_CUDA_OK(cudaMemsetAsync(va.virial, 0, sizeof(T) * (size_t)nf * 9, s));
+  STAFB_CUDA_OK(zero_two(s, force, sizeof(T) * (size_t)nf * 3 * N, va.virial, va.virial ? sizeof(T) * (size_t)nf * 9 : 0));
   const int n = nf * Nl;
   if (n <= 0) return STAFB_OK;
-  k_force_rad<T><<<(n + OPS_WARPS - 1) / OPS_WARPS, OPS_THREADS, 0, s>>>(n, Nl, N, c->nr, Fr, nd, der2b, im2, rad, a2,
-                                                                        e2, tm, tipos, at, force, va);
-  STAFB_CUDA_OK(cudaGetLastError());
+  STAFB_CUDA_OK(launch_chained(k_force_rad<T>, (n + OPS_WARPS - 1) / OPS_WARPS, OPS_THREADS, 0, s, n, Nl, N, c->nr, Fr,
+                               nd, der2b, im2, rad, a2, e2, tm, tipos, at, force, va));
   return STAFB_OK;
 }
 
@@ -606,14 +842,16 @@ template <class T>
 int op_force_ang(stafb_ctx* c, cudaStream_t s, const T* nd, const T* ds3, const T* ang, const T* d3s, const T* d3,
                  const int* im2, const T* a3, const T* e3, const int* tm, const int* tipos, const int* at,
                  const int* ntr, int nf, int Nl, int N, int nt, int Fa, T* force, VirArgs<T> va = VirArgs<T>()) {
-  STAFB_CUDA_OK(cudaMemsetAsync(force, 0, sizeof(T) * (size_t)nf * 3 * N, s));
-  if (va.virial) STAFB_CUDA_OK(cudaMemsetAsync(va.virial, 0, sizeof(T) * (size_t)nf * 9, s));
+  STAFB_CUDA_OK(zero_two(s, force, sizeof(T) * (size_t)nf * 3 * N, va.virial, va.virial ? sizeof(T) * (size_t)nf * 9 : 0));
   const int n = nf * Nl;
   if (n <= 0) return STAFB_OK;
-  size_t sm = sizeof(T) * ((size_t)c->nr * 7 + Fa) + sizeof(int) * (size_t)c->nr * 2 + (size_t)c->na * 2;
-  k_force_ang<T><<<n, OPS_THREADS, sm, s>>>(Nl, N, c->nr, c->na, Fa, nd, ds3, ang, d3s, d3, im2, a3, e3, tm, tipos, at,
-                                            ntr, force, va);
-  STAFB_CUDA_OK(cudaGetLastError());
+  AngArgs<T> a = ang_args<T>(c, ang, ds3, im2, a3, e3, tm, ntr, nt, Fa);
+  a.Nl = Nl; a.N = N; a.netderiv = nd; a.der3bsupp = d3s; a.der3b = d3; a.tipos = tipos; a.actual_type = at; a.out = force;
+  AngSmem<T> L;
+  const int rc = ang_layout<T>(a, 0, 3 * a.nr, L);
+  if (rc != STAFB_OK) return rc;
+  STAFB_CUDA_OK(opt_in((const void*)k_force_ang<T>, (size_t)L.total));
+  STAFB_CUDA_OK(launch_chained(k_force_ang<T>, n, ANG_THREADS, (size_t)L.total, s, a, L, va));
   return STAFB_OK;
 }
 
@@ -621,29 +859,24 @@ template <class T>
 int op_grad_af_rad(stafb_ctx* c, cudaStream_t s, const T* pg, const T* rad, const int* im2, const T* a2, const T* e2,
                    const int* tm, int nf, int Nl, int nt, int Fr, T* ga, T* ge) {
   if (nt > STAFB_MAX_TYPES) return STAFB_ERR_INVALID;
-  STAFB_CUDA_OK(cudaMemsetAsync(ga, 0, sizeof(T) * nt * Fr, s));
-  STAFB_CUDA_OK(cudaMemsetAsync(ge, 0, sizeof(T) * nt * Fr, s));
+  STAFB_CUDA_OK(zero_two(s, ga, sizeof(T) * nt * Fr, ge, sizeof(T) * nt * Fr));
   const int n = nf * Nl;
   if (n <= 0) return STAFB_OK;
-  k_grad_af_rad<T><<<(n + OPS_WARPS - 1) / OPS_WARPS, OPS_THREADS, 0, s>>>(n, c->nr, Fr, nt, pg, rad, im2, a2, e2, tm,
-                                                                          ga, ge);
-  STAFB_CUDA_OK(cudaGetLastError());
-  return STAFB_OK;
+  RadArgs<T> a = rad_args<T>(c, rad, im2, a2, e2, tm, n, nt, Fr);
+  a.prevgrad = pg; a.g_alpha = ga; a.g_emb = ge;
+  return launch_rad<T, 1>(s, a);
 }
 
 template <class T>
 int op_grad_af_ang(stafb_ctx* c, cudaStream_t s, const T* pg, const T* ang, const T* ds3, const int* im2,
                    const T* a3, const T* e3, const int* tm, const int* ntr, int nf, int Nl, int nt, int Fa, T* ga,
                    T* ge) {
-  const int C = nt * (nt + 1) / 2;
-  STAFB_CUDA_OK(cudaMemsetAsync(ga, 0, sizeof(T) * C * 3 * Fa, s));
-  STAFB_CUDA_OK(cudaMemsetAsync(ge, 0, sizeof(T) * C * Fa, s));
-  const int n = nf * Nl;
+  const int C = nt * (nt + 1) / 2, n = nf * Nl;
+  STAFB_CUDA_OK(zero_two(s, ga, sizeof(T) * C * 3 * Fa, ge, n > 0 ? 0 : sizeof(T) * C * Fa));
   if (n <= 0) return STAFB_OK;
-  size_t sm = (size_t)c->nr * (sizeof(T) + sizeof(int)) + (size_t)c->na * 2;
-  k_grad_af_ang<T><<<n, OPS_THREADS, sm, s>>>(c->nr, c->na, Fa, ncls_of(nt), pg, ang, ds3, im2, a3, e3, tm, ntr, ga);
-  STAFB_CUDA_OK(cudaGetLastError());
-  return STAFB_OK;
+  AngArgs<T> a = ang_args<T>(c, ang, ds3, im2, a3, e3, tm, ntr, nt, Fa);
+  a.prevgrad = pg; a.g_alpha3 = ga; a.zero = ge; a.zero_n = C * Fa;
+  return launch_ang<T, 1>(s, n, a);
 }
 
 template <class T>
@@ -651,15 +884,13 @@ int op_grad_force_rad(stafb_ctx* c, cudaStream_t s, const T* pg, const T* nd, co
                       const T* rad, const T* a2, const T* e2, const int* tm, const int* tipos, const int* at, int nf,
                       int Nl, int N, int nt, int Fr, T* gradnet, T* ga, T* ge, VirArgs<T> va = VirArgs<T>()) {
   if (nt > STAFB_MAX_TYPES) return STAFB_ERR_INVALID;
-  STAFB_CUDA_OK(cudaMemsetAsync(ga, 0, sizeof(T) * nt * Fr, s));
-  STAFB_CUDA_OK(cudaMemsetAsync(ge, 0, sizeof(T) * nt * Fr, s));
+  STAFB_CUDA_OK(zero_two(s, ga, sizeof(T) * nt * Fr, ge, sizeof(T) * nt * Fr));
   const int n = nf * Nl;
   if (n <= 0) return STAFB_OK;
-  k_grad_force_rad<T><<<(n + OPS_WARPS - 1) / OPS_WARPS, OPS_THREADS, 0, s>>>(n, Nl, N, c->nr, Fr, nt, pg, nd, der2b,
-                                                                             im2, rad, a2, e2, tm, tipos, at, gradnet,
-                                                                             ga, ge, va);
-  STAFB_CUDA_OK(cudaGetLastError());
-  return STAFB_OK;
+  RadArgs<T> a = rad_args<T>(c, rad, im2, a2, e2, tm, n, nt, Fr);
+  a.Nl = Nl; a.N = N; a.prevgrad = pg; a.netderiv = nd; a.der2b = der2b; a.tipos = tipos; a.actual_type = at;
+  a.out = gradnet; a.g_alpha = ga; a.g_emb = ge;
+  return launch_rad<T, 2>(s, a, va);
 }
 
 template <class T>
@@ -667,24 +898,13 @@ int op_grad_force_ang(stafb_ctx* c, cudaStream_t s, const T* pg, const T* nd, co
                       const T* d3s, const T* d3, const int* im2, const T* a3, const T* e3, const int* tm,
                       const int* tipos, const int* at, const int* ntr, int nf, int Nl, int N, int nt, int Fa,
                       T* gradnet, T* ga, T* gck, VirArgs<T> va = VirArgs<T>()) {
-  const int C = nt * (nt + 1) / 2;
-  STAFB_CUDA_OK(cudaMemsetAsync(ga, 0, sizeof(T) * C * 3 * Fa, s));
-  STAFB_CUDA_OK(cudaMemsetAsync(gck, 0, sizeof(T) * C * Fa, s));
-  const int n = nf * Nl;
+  const int C = nt * (nt + 1) / 2, n = nf * Nl;
+  STAFB_CUDA_OK(zero_two(s, ga, sizeof(T) * C * 3 * Fa, gck, n > 0 ? 0 : sizeof(T) * C * Fa));
   if (n <= 0) return STAFB_OK;
-  size_t sm = sizeof(T) * ((size_t)c->nr * 5 + c->na) + sizeof(int) * (size_t)c->nr + (size_t)c->na * 2;
-  static bool attr_done[64] = {false};  // per instantiation and device: the attribute belongs to the current device
-  int dev = 0;
-  cudaGetDevice(&dev);
-  bool& done = attr_done[(dev >= 0 && dev < 64) ? dev : 0];
-  if (sm > 48 * 1024 && !done) {
-    STAFB_CUDA_OK(cudaFuncSetAttribute(k_grad_force_ang<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    done = true;
-  }
-  k_grad_force_ang<T><<<n, OPS_THREADS, sm, s>>>(Nl, N, c->nr, c->na, Fa, ncls_of(nt), pg, nd, ds3, ang, d3s, d3, im2,
-                                                 a3, e3, tm, tipos, at, ntr, gradnet, ga, va);
-  STAFB_CUDA_OK(cudaGetLastError());
-  return STAFB_OK;
+  AngArgs<T> a = ang_args<T>(c, ang, ds3, im2, a3, e3, tm, ntr, nt, Fa);
+  a.Nl = Nl; a.N = N; a.prevgrad = pg; a.netderiv = nd; a.der3bsupp = d3s; a.der3b = d3; a.tipos = tipos;
+  a.actual_type = at; a.out = gradnet; a.g_alpha3 = ga; a.zero = gck; a.zero_n = C * Fa;
+  return launch_ang<T, 2>(s, n, a, va);
 }
 
 }  // namespace stafb

@@ -16,7 +16,7 @@ from .params import ModelShape
 
 
 def _p(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 class StafModel:
@@ -33,6 +33,7 @@ class StafModel:
         self.n_centres = shape.N
         self.ctx = Context(cfg["Rc"], cfg["nr"], cfg["na"], self.n_max, cfg["Rs"], cfg["Ra"], max_batch, dtype, device)
         self.device = self.ctx.device
+        self._dev_full = torch.device("cuda", self.ctx._index)
         self.max_batch = int(max_batch)
         h = C.c_void_p()
         sd = shape.desc()
@@ -67,6 +68,8 @@ class StafModel:
 
     def _dev(self, a):
         if torch.is_tensor(a):
+            if a.dtype is self.dtype and a.device == self._dev_full and a.is_contiguous():
+                return a
             return a.to(device=self.device, dtype=self.dtype).contiguous()
         return torch.as_tensor(np.asarray(a), dtype=self.dtype).to(self.device).contiguous()
 

@@ -10,6 +10,7 @@ construct_descriptors_light(); unlike the reference it is kept per (device, dtyp
 nothing here ever exits the process - saturated buffers raise StafbError.
 """
 import ctypes as C
+import math
 
 import numpy as np
 import torch
@@ -17,6 +18,12 @@ import torch
 from . import _lib
 from ._lib import StafbError, check  # noqa: F401
 
+# The operators are called one after the other, some twenty per training step of a framework's graph, and at a few
+# microseconds of GPU time each it is the host that sets the pace: tensors that are what an operator needs already
+# pass through without a call into torch's dispatcher, pointers travel as plain integers, the stream is asked for
+# without building a Stream object (28 -> 16 us of host time per operator).
+_raw_stream = torch._C._cuda_getCurrentRawStream
+_I32 = torch.int32
 _CTX = {}
 _LAST = {}
 
@@ -34,6 +41,7 @@ class Context:
             check(_lib.lib().stafb_create(C.byref(h), 0 if self.dtype == torch.float32 else 1, self.Rc, self.Rs,
                                           self.Ra, self.nr, self.na, self.n_max, self.max_batch), "stafb_create")
         self.h = h
+        self._index = self.device.index if self.device.index is not None else torch.cuda.current_device()
 
     def close(self):
         if getattr(self, "h", None):
@@ -47,7 +55,7 @@ class Context:
             pass
 
     def stream(self):
-        return C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        return C.c_void_p(_raw_stream(self._index))
 
     def status(self):
         return _lib.lib().stafb_status(self.h, self.stream())
@@ -62,27 +70,27 @@ class Context:
 
 
 def _p(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _ctx_for(t):
-    key = (t.device.index if t.device.index is not None else torch.cuda.current_device(), t.dtype)
-    if key not in _CTX:
-        raise RuntimeError("STAF: operator called before construct_descriptors_light for %s" % (key,))
-    return _CTX[key]
+    d = t.device.index
+    ctx = _CTX.get((d if d is not None else torch.cuda.current_device(), t.dtype))
+    if ctx is None:
+        raise RuntimeError("STAF: operator called before construct_descriptors_light for %s" % ((d, t.dtype),))
+    return ctx
 
 
 def _real(ctx, *ts):
-    out = []
+    dt = ctx.dtype
     for t in ts:
-        if t.dtype != ctx.dtype or not t.is_cuda:
-            raise TypeError("expected a CUDA tensor of dtype %s" % ctx.dtype)
-        out.append(t.contiguous())
-    return out
+        if t.dtype is not dt or not t.is_cuda:
+            raise TypeError("expected a CUDA tensor of dtype %s" % dt)
+    return [t if t.is_contiguous() else t.contiguous() for t in ts]
 
 
 def _int(*ts):
-    return [t.to(torch.int32).contiguous() for t in ts]
+    return [t if t.dtype is _I32 and t.is_contiguous() else t.to(_I32).contiguous() for t in ts]
 
 
 def construct_descriptors_light(radial_cutoff, radial_buffer, angular_buffer, numpar, boxer, rs, ra, max_batch,
@@ -106,7 +114,7 @@ def compute_descriptors_light(positions, boxer, with_angular=True, ctx=None):
     nf, N = boxer.shape[0], positions.shape[1] // 3
     nr, na = ctx.nr, ctx.na
     dev, dt = positions.device, ctx.dtype
-    e = lambda *s, d=dt: torch.empty(*s, dtype=d, device=dev)
+    e = lambda *s, d=dt: torch.empty(s, dtype=d, device=dev)
     raddescr, des3bsupp = e(nf, N, nr), e(nf, N, nr)
     der2b, der3bsupp = e(nf, N, 3, nr), e(nf, N, 3, nr)
     intmap2b, numtriplet = e(nf, N, nr + 1, d=torch.int32), e(nf, N, d=torch.int32)
@@ -129,7 +137,7 @@ def compute_sort_proj(radial_descriptor, interaction_map_rad, alpha2b_parameters
     nf, Nl, nr = rd.shape
     nt, Fr = a2.shape
     assert nr == ctx.nr
-    out = torch.empty(nf, Nl, Fr, dtype=ctx.dtype, device=rd.device)
+    out = rd.new_empty((nf, Nl, Fr))
     check(_lib.lib().stafb_compute_sort_proj(ctx.h, ctx.stream(), _p(rd), _p(im2), _p(a2), _p(e2), _p(tm), nf, Nl, nt,
                                              Fr, _p(out)), "ComputeSortProj")
     return out
@@ -145,7 +153,7 @@ def compute_sort_proj3body(angular_descriptor, radial_descriptor, interaction_ma
     Fa = a3.shape[1] // 3
     nt = _nt_from_classes(a3.shape[0])
     assert na == ctx.na and rd.shape[2] == ctx.nr
-    out = torch.empty(nf, Nl, Fa, dtype=ctx.dtype, device=ad.device)
+    out = ad.new_empty((nf, Nl, Fa))
     check(_lib.lib().stafb_compute_sort_proj3body(ctx.h, ctx.stream(), _p(ad), _p(rd), _p(im3), _p(im2), _p(a3),
                                                   _p(e3), _p(tm), _p(ntr), nf, Nl, nt, Fa, _p(out)),
           "ComputeSortProj3body")
@@ -153,7 +161,7 @@ def compute_sort_proj3body(angular_descriptor, radial_descriptor, interaction_ma
 
 
 def _nt_from_classes(C_):
-    nt = int(round((np.sqrt(8 * C_ + 1) - 1) / 2))
+    nt = (math.isqrt(8 * C_ + 1) - 1) // 2
     assert nt * (nt + 1) // 2 == C_
     return nt
 
@@ -176,8 +184,10 @@ def init_grad_force_tripl(buffdim):
 
 def _dev_int(x, device):
     if torch.is_tensor(x):
-        return x.to(device=device, dtype=torch.int32).reshape(-1).contiguous()
-    return torch.tensor(np.atleast_1d(x), dtype=torch.int32, device=device)
+        if x.dtype is _I32 and x.device == device and x.dim() == 1 and x.is_contiguous():
+            return x
+        return x.to(device=device, dtype=_I32).reshape(-1).contiguous()
+    return torch.tensor(np.atleast_1d(x), dtype=_I32, device=device)
 
 
 def compute_force_radial(netderiv, descriptor_derivative_rad, interaction_map_rad, radial_descriptor,
@@ -190,7 +200,7 @@ def compute_force_radial(netderiv, descriptor_derivative_rad, interaction_map_ra
     tp, at = _dev_int(tipos, nd.device), _dev_int(actual_type, nd.device)
     nf, Nl, Fr = nd.shape
     N, nt = tm.shape[0], tp.shape[0]
-    out = torch.empty(nf, 3 * N, dtype=ctx.dtype, device=nd.device)
+    out = nd.new_empty((nf, 3 * N))
     check(_lib.lib().stafb_compute_force_radial(ctx.h, ctx.stream(), _p(nd), _p(dd), _p(im2), _p(rd), _p(a2), _p(e2),
                                                 _p(tm), _p(tp), _p(at), nf, Nl, N, nt, Fr, _p(out)),
           "ComputeForceRadial")
@@ -209,7 +219,7 @@ def compute_force_tripl(netderiv, radial_descriptor, angular_descriptor, descrip
     tp, at = _dev_int(tipos, nd.device), _dev_int(actual_type, nd.device)
     nf, Nl, Fa = nd.shape
     N, nt = tm.shape[0], tp.shape[0]
-    out = torch.empty(nf, 3 * N, dtype=ctx.dtype, device=nd.device)
+    out = nd.new_empty((nf, 3 * N))
     check(_lib.lib().stafb_compute_force_tripl(ctx.h, ctx.stream(), _p(nd), _p(rd), _p(ad), _p(ddr), _p(dda), _p(im2),
                                                _p(im3), _p(a3), _p(e3), _p(tm), _p(tp), _p(at), _p(ntr), nf, Nl, N,
                                                nt, Fa, _p(out)), "ComputeForceTripl")
@@ -239,7 +249,7 @@ def compute_sort_proj3body_grad(previous_gradient, angular_desciptors, radial_de
     nf, Nl, Fa = pg.shape
     nt = _nt_from_classes(a3.shape[0])
     ga = torch.empty_like(a3)
-    ge = torch.empty(a3.shape[0], Fa, dtype=ctx.dtype, device=pg.device)
+    ge = pg.new_empty((a3.shape[0], Fa))
     check(_lib.lib().stafb_compute_sort_proj3body_grad(ctx.h, ctx.stream(), _p(pg), _p(ad), _p(rd), _p(im3), _p(im2),
                                                        _p(a3), _p(e3), _p(tm), _p(ntr), nf, Nl, nt, Fa, _p(ga),
                                                        _p(ge)), "ComputeSortProj3bodyGrad")
@@ -276,7 +286,7 @@ def compute_force_tripl_grad(prevgrad, netderiv, radial_descriptor, angular_desc
     nf, Nl, Fa = nd.shape
     N, nt = tm.shape[0], tp.shape[0]
     gn, ga = torch.empty_like(nd), torch.empty_like(a3)
-    gck = torch.empty(a3.shape[0], Fa, dtype=ctx.dtype, device=nd.device)
+    gck = nd.new_empty((a3.shape[0], Fa))
     check(_lib.lib().stafb_compute_force_tripl_grad(ctx.h, ctx.stream(), _p(pg), _p(nd), _p(rd), _p(ad), _p(ddr),
                                                     _p(dda), _p(im2), _p(im3), _p(a3), _p(e3), _p(tm), _p(tp), _p(at),
                                                     _p(ntr), nf, Nl, N, nt, Fa, _p(gn), _p(ga), _p(gck)),
@@ -294,8 +304,8 @@ def compute_force_radial_virial(netderiv, descriptor_derivative_rad, interaction
     tp, at = _dev_int(tipos, nd.device), _dev_int(actual_type, nd.device)
     nf, Nl, Fr = nd.shape
     N, nt = tm.shape[0], tp.shape[0]
-    out = torch.empty(nf, 3 * N, dtype=ctx.dtype, device=nd.device)
-    vir = torch.empty(nf, 9, dtype=ctx.dtype, device=nd.device)
+    out = nd.new_empty((nf, 3 * N))
+    vir = nd.new_empty((nf, 9))
     check(_lib.lib().stafb_compute_force_radial_virial(ctx.h, ctx.stream(), _p(nd), _p(dd), _p(im2), _p(rd), _p(a2),
                                                        _p(e2), _p(tm), _p(tp), _p(at), _p(ps), _p(bx), nf, Nl, N, nt,
                                                        Fr, _p(out), _p(vir)), "ComputeForceRadialVirial")
@@ -315,8 +325,8 @@ def compute_force_tripl_virial(netderiv, radial_descriptor, angular_descriptor, 
     tp, at = _dev_int(tipos, nd.device), _dev_int(actual_type, nd.device)
     nf, Nl, Fa = nd.shape
     N, nt = tm.shape[0], tp.shape[0]
-    out = torch.empty(nf, 3 * N, dtype=ctx.dtype, device=nd.device)
-    vir = torch.empty(nf, 9, dtype=ctx.dtype, device=nd.device)
+    out = nd.new_empty((nf, 3 * N))
+    vir = nd.new_empty((nf, 9))
     check(_lib.lib().stafb_compute_force_tripl_virial(ctx.h, ctx.stream(), _p(nd), _p(rd), _p(ad), _p(ddr), _p(dda),
                                                       _p(im2), _p(im3), _p(a3), _p(e3), _p(tm), _p(tp), _p(at),
                                                       _p(ntr), _p(ps), _p(bx), nf, Nl, N, nt, Fa, _p(out), _p(vir)),
@@ -358,7 +368,7 @@ def compute_force_tripl_virial_grad(prevgrad, prevgrad_virial, netderiv, radial_
     nf, Nl, Fa = nd.shape
     N, nt = tm.shape[0], tp.shape[0]
     gn, ga = torch.empty_like(nd), torch.empty_like(a3)
-    gck = torch.empty(a3.shape[0], Fa, dtype=ctx.dtype, device=nd.device)
+    gck = nd.new_empty((a3.shape[0], Fa))
     check(_lib.lib().stafb_compute_force_tripl_virial_grad(ctx.h, ctx.stream(), _p(pg), _p(pv), _p(nd), _p(rd),
                                                            _p(ad), _p(ddr), _p(dda), _p(im2), _p(im3), _p(a3),
                                                            _p(e3), _p(tm), _p(tp), _p(at), _p(ntr), _p(ps), _p(bx),

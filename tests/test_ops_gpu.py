@@ -212,3 +212,49 @@ def test_descriptor_integer_outputs_are_deterministic(ops):
         c = ops.compute_descriptors_light(p, b)
         assert torch.equal(a[3], c[3]) and torch.equal(a[4], c[4]) and torch.equal(a[8], c[8])
         assert torch.equal(a[0], c[0]) and torch.equal(a[1], c[1])
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("channels", [(1, 8, 9), (0, 17, 3)])
+def test_angular_operators_with_other_channel_counts(ops, oracle, channels, dtype):
+    """Active channels per class around the number that one pass takes (8), an empty class, a second and third pass."""
+    from alphanesgpu_b200 import train as T
+    from alphanesgpu_b200.params import ModelShape
+    pos, box, tipos = synth.water_frames("water96", [1000, 1001])
+    maps = dict(map_rad_afs={0: [3, 30], 1: [1, 4]}, map_ang_afs={0: list(channels), 1: list(channels[::-1])})
+    shape = ModelShape(nt=2, tipos=list(tipos), Fr=[33, 5], Fa=[sum(channels)] * 2, widths=[8, 1])
+    theta, emb = T.init_params(shape, maps, 3)
+    pos, box, theta, emb = pos.astype(dtype), box.astype(dtype), theta.astype(dtype), emb.astype(dtype)
+    nf, N, nt, C = 2, shape.N, 2, 3
+    _ctx(ops, dtype, N, nf)
+    ref = oracle.descriptors(CFG["Rc"], CFG["Rs"], CFG["Ra"], CFG["nr"], CFG["na"], pos, box, dtype)
+    tm, tp = _t(shape.type_map.astype(np.int32)), _t(np.asarray(tipos, np.int32))
+    rng = np.random.default_rng(5)
+    for t in (0, 1):
+        d = _species_slices(ref, shape, t)
+        o, Fr, Fa = shape.offsets(t), shape.Fr[t], shape.Fa[t]
+        a2, e2 = theta[o["a2"]:o["a2"] + nt * Fr].reshape(nt, Fr), emb[o["emb"]:o["emb"] + nt * Fr].reshape(nt, Fr)
+        a3 = theta[o["a3"]:o["a3"] + C * 3 * Fa].reshape(C, 3 * Fa)
+        e3 = emb[o["emb"] + nt * Fr:o["emb"] + nt * Fr + C * Fa].reshape(C, Fa)
+        af2 = oracle.af_radial(d["raddescr"], d["intmap2b"], a2, e2, shape.type_map)
+        af3 = oracle.af_angular(d["angdescr"], d["des3bsupp"], d["intmap3b"], a3, e3, shape.type_map, d["numtriplet"])
+        g = {k: _t(v) for k, v in d.items()}
+        A2, E2, A3, E3 = (_t(np.ascontiguousarray(x)) for x in (a2, e2, a3, e3))
+        assert rel_err(ops.compute_sort_proj(g["raddescr"], g["intmap2b"], A2, E2, tm).cpu().numpy(), af2) <= TOL[dtype]
+        got = ops.compute_sort_proj3body(g["angdescr"], g["des3bsupp"], g["intmap3b"], g["intmap2b"], A3, E3, tm,
+                                         g["numtriplet"])
+        assert rel_err(got.cpu().numpy(), af3) <= TOL[dtype]
+        # forces against the oracle, and their backward by the identity <prev, F(nd)> = <gradnet(prev), nd>
+        nd = rng.normal(size=af3.shape).astype(dtype)
+        f_ref, _ = oracle.force_tripl(nd, d["des3bsupp"], d["angdescr"], d["der3bsupp"], d["der3b"], d["intmap3b"], a3,
+                                      e3, shape.type_map, d["numtriplet"], shape.shift(t), pos, box)
+        at = torch.tensor([t], dtype=torch.int32).cuda()
+        args = (g["des3bsupp"], g["angdescr"], g["der3bsupp"], g["der3b"], g["intmap2b"], g["intmap3b"], A3, E3, tm, tp,
+                at, g["numtriplet"])
+        f = ops.compute_force_tripl(_t(nd), *args)
+        assert rel_err(f.cpu().numpy(), f_ref) <= TOL[dtype]
+        prev = _t(rng.normal(size=f_ref.shape).astype(dtype))
+        gn, _, _ = ops.compute_force_tripl_grad(prev, _t(nd), *args)
+        lhs, rhs = float((prev.double() * f.double()).sum()), float((gn.double() * _t(nd).double()).sum())
+        scale = float((prev.double() * f.double()).abs().sum())
+        assert abs(lhs - rhs) <= TOL[dtype] * scale
