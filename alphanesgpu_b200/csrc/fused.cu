@@ -335,6 +335,19 @@ extern "C" int stafb_model_create(stafb_ctx* c, const int* sd, stafb_model** out
   if (m->stage < 0 || m->stage > 2 || mlp_smem_bwd(d, m->es, m->aw, m->stage) > mlp_room) { free(m); return STAFB_ERR_CAPACITY; }
   m->mlp_fwd_smem = mlp_smem_fwd(d, m->es, m->aw, m->stage);
   m->mlp_bwd_smem = mlp_smem_bwd(d, m->es, m->aw, m->stage);
+  // Layers wider than 64 in fp32: one block of the warp form (16 atoms, two per warp) fills an SM's shared memory, so
+  // past one block per SM its time doubles, and there the tile form (24 atoms a block) is the better one:
+  // 60-140-140-1, 3,072 atoms, forward 61 -> 43 us, backward 146 -> 83 us (its sum kernel included); at 2,304 atoms the
+  // warp form still takes 17 us less of an evaluation.  Bounds: shared memory, and layers that the weight ring holds
+  // eight columns of.
+  m->tile_above = -1;
+  if (c->dtype == STAFB_F32 && d.maxw > 64 && mlp_tile_smem_bwd(d, ML_TILE) <= mlp_room &&
+      mlp_tile_smem_fwd(d, ML_TILE) <= mlp_room) {
+    m->tile_above = nsm;
+    for (int t = 0; t < d.nt; t++)
+      for (int l = 0; l < d.n_dense; l++)
+        if (ml_chunk_cols(std::max(1, d.in_of(t, l))) < 8 || ml_chunk_rows(ml_ld(d.width[l])) < 1) m->tile_above = -1;
+  }
   // The tensor-core form of the MLP kernels (mlp_mma.cuh; fp32 only, one block per 16 atoms, its warps - 4;
   // STAFB_MLP_MMA_NW: 1, 2, 4, 8 - sharing the tiles) is the other arm, selected with STAFB_MLP_MMA=1: on B200
   // mma.sync.m16n8k8.tf32 issues at about one instruction per 30 cycles per SM, which leaves these kernels
@@ -369,6 +382,14 @@ extern "C" int stafb_model_create(stafb_ctx* c, const int* sd, stafb_model** out
   STAFB_CUDA_OK(cudaMalloc(&m->vrow, es * A * (m->nv > 0 ? m->nv : 1)));
   {
     size_t acts_words = mlp_blocks * ML_WARPS * m->aw * d.Hsum;
+    if (m->tile_above >= 0 && A / 16 + d.nt > (size_t)m->tile_above) {
+      const size_t tiles = A / ML_TILE + (size_t)d.nt + 1;
+      acts_words = std::max(acts_words, tiles * ML_TILE * d.Hsum);
+      // rows of the backward kernel's gradient sums: one per tile, two per SM at most
+      for (int t = 0; t < d.nt; t++) m->part_stride = std::max(m->part_stride, (m->blk_size[t] + 3) & ~3);
+      m->part_blocks = (int)std::max<size_t>(2 * d.nt, std::min<size_t>(tiles, (size_t)nsm * 2));
+      STAFB_CUDA_OK(cudaMalloc(&m->part, es * (size_t)m->part_blocks * m->part_stride));
+    }
     if (m->mma) {
       const size_t tiles = A / MM_ATOMS + (size_t)d.nt * c->max_batch + 1;
       const size_t w2 = tiles * MM_ATOMS * (size_t)mm_shape(d, 0).hoff[d.n_dense];
@@ -405,7 +426,7 @@ extern "C" int stafb_model_create(stafb_ctx* c, const int* sd, stafb_model** out
 extern "C" void stafb_model_destroy(stafb_model* m) {
   if (!m) return;
   void* ptrs[] = {m->rows, m->spar, m->af, m->nd, m->gradnet, m->gaf, m->acts, m->e_atom, m->force,
-                  m->flab, m->ebar, m->energy, m->losses_d, m->epart, m->vrow, m->wpack, m->wm, m->vlab_d};
+                  m->flab, m->ebar, m->energy, m->losses_d, m->epart, m->vrow, m->wpack, m->wm, m->vlab_d, m->part};
   for (void* p : ptrs) cudaFree(p);
   for (int k = 0; k < 3; k++) {
     cudaFreeHost(m->slot_in_h[k]);
@@ -535,7 +556,7 @@ static int run_fused(stafb_ctx* c, stafb_model* m, cudaStream_t s, const T* pos,
   rc = train ? launch_sweep<T, MODE_AFV>(m, s, sc) : launch_sweep<T, MODE_AF>(m, s, sc);
   if (rc != STAFB_OK) return rc;
   mark();  // af_fwd
-  rc = launch_mlp_fwd<T>(m, s, nf, theta, af, acts, e_atom, nd);
+  rc = launch_mlp_fwd<T>(m, s, nf, theta, af, train || !mlp_tiles(m, nf) ? acts : (T*)nullptr, e_atom, nd);
   if (rc != STAFB_OK) return rc;
   mark();  // mlp_fwd
   if (v_label && !train) return STAFB_ERR_INVALID;

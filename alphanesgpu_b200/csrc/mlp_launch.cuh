@@ -36,6 +36,42 @@ static int launch_mlp_bwd_t(stafb_model* m, cudaStream_t s, int nf, const T* the
   return STAFB_OK;
 }
 
+static int launch_mlp_fwd_tile(stafb_model* m, cudaStream_t s, int nf, const float* theta, const float* af, float* acts,
+                               float* e_atom, float* nd) {
+  const size_t sm = mlp_tile_smem_fwd(m->md, ML_TILE);
+  static size_t attr_dev[MAX_DEVICES] = {0};
+  size_t& attr = attr_dev[device_slot()];
+  if (sm > 48 * 1024 && sm > attr) {
+    STAFB_CUDA_OK(cudaFuncSetAttribute(k_mlp_fwd_tile<ML_TILE, ML_TILE_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    attr = sm;
+  }
+  STAFB_CUDA_OK(launch_chained(k_mlp_fwd_tile<ML_TILE, ML_TILE_THREADS>, species_blocks(m->md, nf, ML_TILE), ML_TILE_THREADS, sm, s, m->md, nf, theta,
+                               (const float*)m->wpack, m->wstride, af, acts, e_atom, nd));
+  m->ctx->launches++;
+  return STAFB_OK;
+}
+
+static int launch_mlp_bwd_tile(stafb_model* m, cudaStream_t s, int nf, const float* theta, const float* af,
+                               const float* acts, const float* ebar, const float* u, float* gaf, float* grad) {
+  const size_t sm = mlp_tile_smem_bwd(m->md, ML_TILE);
+  static size_t attr_dev[MAX_DEVICES] = {0};
+  size_t& attr = attr_dev[device_slot()];
+  if (sm > 48 * 1024 && sm > attr) {
+    STAFB_CUDA_OK(cudaFuncSetAttribute(k_mlp_bwd_tile<ML_TILE, ML_TILE_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    attr = sm;
+  }
+  const TilePlan tp = mlp_tile_plan(m->md, nf, ML_TILE, m->part_blocks);
+  int blocks = 0;
+  for (int t = 0; t < m->md.nt; t++) blocks += tp.nb[t];
+  STAFB_CUDA_OK(launch_chained(k_mlp_bwd_tile<ML_TILE, ML_TILE_THREADS>, blocks, ML_TILE_THREADS, sm, s, m->md, nf, theta, (const float*)m->wpack,
+                               m->wstride, af, acts, ebar, u, (const float*)m->vrow, m->nv, gaf, (float*)m->part,
+                               m->part_stride, tp));
+  STAFB_CUDA_OK(launch_chained(k_mlp_sum, (m->n_params + 31) / 32, 256, 0, s, m->md, tp, (const float*)m->part,
+                               m->part_stride, grad, m->n_params));
+  m->ctx->launches += 2;
+  return STAFB_OK;
+}
+
 static int launch_mlp_fwd_mma(stafb_model* m, cudaStream_t s, int nf, const float* theta, const float* af, float* acts,
                               float* e_atom, float* nd) {
   static size_t attr_dev[MAX_DEVICES] = {0};
@@ -72,6 +108,7 @@ int launch_mlp_fwd(stafb_model* m, cudaStream_t s, int nf, const T* theta, const
                           T* nd) {
   if constexpr (std::is_same<T, float>::value) {
     if (m->mma) return launch_mlp_fwd_mma(m, s, nf, theta, af, acts, e_atom, nd);
+    if (mlp_tiles(m, nf)) return launch_mlp_fwd_tile(m, s, nf, theta, af, acts, e_atom, nd);
   }
   const bool wg = m->stage == 0, wide = m->md.maxw > 64;  // the dense products' form: see mlp.cuh
   switch (m->aw) {
@@ -89,6 +126,7 @@ int launch_mlp_bwd(stafb_model* m, cudaStream_t s, int nf, const T* theta, const
                           const T* ebar, const T* u, T* gaf, T* grad) {
   if constexpr (std::is_same<T, float>::value) {
     if (m->mma) return launch_mlp_bwd_mma(m, s, nf, theta, af, acts, ebar, u, gaf, grad);
+    if (mlp_tiles(m, nf)) return launch_mlp_bwd_tile(m, s, nf, theta, af, acts, ebar, u, gaf, grad);
   }
   const bool wg = m->stage == 0, wide = m->md.maxw > 64;  // the dense products' form: see mlp.cuh
   switch (m->aw) {

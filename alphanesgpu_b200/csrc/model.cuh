@@ -71,6 +71,7 @@ static inline int species_blocks(const ModelDev& md, int nf, int W) {
 
 // ---------------------------------------------------------------------------- MLP head
 #include "mlp.cuh"
+#include "mlp_tile.cuh"
 #include "mlp_mma.cuh"
 
 }  // namespace stafb
@@ -86,6 +87,9 @@ struct stafb_model {
   int cap_atoms;  // atoms per frame the scratch was sized for
   int aw;   // atoms per warp of the MLP kernels (4, 2 or 1; a block of eight warps owns 8*aw atoms)
   int stage;  // Dense layers in shared memory: 2 all at kernel start, 1 one at a time, 0 none
+  int tile_above;  // the tile form of the MLP kernels (mlp_tile.cuh) takes evaluations of more 16-atom blocks; -1: none
+  void* part;  // rows of gradient sums of its backward kernel [part_blocks][part_stride]
+  int part_blocks, part_stride;
   size_t mlp_fwd_smem, mlp_bwd_smem;
   // scratch for max_batch frames
   void *rows, *af, *nd, *acts, *e_atom, *force, *flab, *ebar, *gradnet, *gaf, *energy, *vrow;
@@ -155,6 +159,30 @@ static size_t mlp_smem_fwd(const ModelDev& d, size_t es, int aw, int stage) {
 }
 static size_t mlp_smem_bwd(const ModelDev& d, size_t es, int aw, int stage) {
   return es * (ML_WARPS * ml_bwd_words(d.Fmax, d.Hsum, d.maxw, aw) + mlp_stage_words(d, stage));
+}
+
+constexpr int ML_TILE = 24, ML_TILE_THREADS = 384;
+static size_t mlp_tile_smem_fwd(const ModelDev& d, int tile) {
+  return sizeof(float) * (2 * ML_RING + (size_t)ml_tile_fwd_rows(d.Fmax, d.Hsum, d.maxw) * ml_rs(tile));
+}
+static size_t mlp_tile_smem_bwd(const ModelDev& d, int tile) {
+  return sizeof(float) * (2 * ML_RING + (size_t)ml_tile_bwd_rows(d.Fmax, d.Hsum) * ml_rs(tile));
+}
+// Which form of the MLP kernels an evaluation of nf frames takes: see stafb_model_create.
+static bool mlp_tiles(const stafb_model* m, int nf) {
+  return m->tile_above >= 0 && species_blocks(m->md, nf, 16) > m->tile_above;
+}
+// blocks of the tile form's backward kernel: one per tile, at most `slots` in all, shared out by the species' tiles
+static TilePlan mlp_tile_plan(const ModelDev& d, int nf, int tile, int slots) {
+  TilePlan p = {};
+  long long total = 0;
+  for (int t = 0; t < d.nt; t++) total += ((long long)nf * d.tipos[t] + tile - 1) / tile;
+  for (int t = 0; t < d.nt; t++) {
+    const long long n = ((long long)nf * d.tipos[t] + tile - 1) / tile;
+    const long long mine = total <= slots ? n : n * (slots - d.nt) / total + 1;
+    p.nb[t] = (int)(mine < n ? mine : n);
+  }
+  return p;
 }
 
 // cudaFuncSetAttribute applies to the device that is current when it is called, and one process may drive

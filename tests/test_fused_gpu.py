@@ -266,6 +266,28 @@ def test_train_step_losses_and_gradient(oracle, frame0, name, seeds, loss, dtype
     m.close()
 
 
+@pytest.mark.parametrize("widths", [[140, 140, 1], [72, 1], [65, 33, 100, 1]])
+def test_train_step_with_wide_layers_in_tiles(oracle, frame0, widths):
+    """More 16-atom blocks than SMs with layers wider than 64: the tile form of the MLP kernels (24 atoms a block, ragged
+    last tiles of both species; weight rings with remainders in rows and columns)."""
+    from alphanesgpu_b200 import train as T
+    from alphanesgpu_b200.model import StafModel
+    from alphanesgpu_b200.params import ModelShape
+    pos, box, shape, _, _ = _case("water768", [1100, 1101, 1102, 1103], frame0)
+    maps = dict(map_rad_afs={0: [10, 9], 1: [10, 10]}, map_ang_afs={0: [3, 2, 14], 1: [3, 2, 14]})
+    shape = ModelShape(nt=2, tipos=shape.tipos, Fr=[19, 20], Fa=[19, 19], widths=widths)
+    theta, emb = T.init_params(shape, maps, 3)
+    el, fl = synth.labels(4, shape.N)
+    kw = dict(pe=0.7, pf=1.3, pb=0.9, alpha_bound=5.0)
+    m = StafModel(shape, CFG, theta, emb, 4, dtype=torch.float32, loss="huber", **kw)
+    _check_train_step(oracle, m, shape, pos, box, el, fl, theta, emb, np.float32, "huber", kw, host_path=False)
+    ref = oracle.energy_force_grad(CFG, shape.desc(), pos, box, shape.type_map, theta, emb, np.float32,
+                                   per_atom_energy=False)
+    e, f = m.energy_force(pos.astype(np.float32), box.astype(np.float32))
+    assert rel_err(e.cpu().numpy(), ref["energy"]) <= 1e-5 and rel_err(f.cpu().numpy(), ref["force"]) <= 1e-5
+    m.close()
+
+
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("channels", [(1, 2, 3), (4, 6, 7), (8, 9, 0)])
 def test_train_step_with_other_channel_counts(oracle, frame0, channels, dtype):
