@@ -20,6 +20,8 @@
 #pragma once
 
 constexpr int MAXP = 4;  // channel PAIRS processed per pass over the pairs of a class
+constexpr int FP_CH = 5;  // channels per pass of the partner-packed fp32 force sweep: 4 FP_CH owner constants in registers
+constexpr int FP_REC = FP_CH + 2;  // 16-byte words of a partner pair's record (odd)
 // Exponential tables: entry (neighbour k, channel pair lp) at tab4[k * TSTR + lp].  Neighbour-major, so that the
 // entries of one neighbour are at constant offsets from one address; the odd stride (5 x 16 bytes) keeps the
 // 16-byte loads of lanes on consecutive neighbours free of bank conflicts.
@@ -226,19 +228,23 @@ struct SweepArgs {
   int* status;
 };
 
+// partner pairs of the fp32 force sweep at most
+__host__ __device__ inline int fp_pairs(int nr) { return (nr + STAFB_MAX_TYPES + 1) / 2; }
+
 // shared-memory layout of a sweep block (byte offsets)
 struct SweepSmem {
   int row, spar, tab, xtra, part, acc, rsum, wch, red, etab, mbar, total;
 };
 template <class T>
-static inline SweepSmem sweep_smem(const ModelDev& d, const SparLayout& sl, int nr, int mode, int nw) {
+static inline SweepSmem sweep_smem(const ModelDev& d, const SparLayout& sl, int nr, int mode, int nw, bool pack) {
   SweepSmem L;
   int o = 0;
   auto take = [&](int bytes) { int r = o; o += (bytes + 15) & ~15; return r; };
   const int es = (int)sizeof(T);
   L.row = take(row_stride_bytes(nr, es));
   L.spar = take(sl.total);
-  L.tab = take(TSTR * nr * 4 * es);
+  // PACK: the records of the partner pairs (every species group padded to a pair), channel weights and beta of a pass
+  L.tab = take(pack ? FP_REC * fp_pairs(nr) * 16 + FP_CH * 24 : TSTR * nr * 4 * es);
   L.xtra = take(mode == MODE_FORCE ? 3 * nr * es : (mode == MODE_FGRAD ? 4 * nr * es : 0));
   L.part = take(mode == MODE_FORCE && nw > 1 ? 3 * 32 * nw * es : 0);  // forces of the segments of an owner
   L.acc = take(mode == MODE_FORCE ? 0 : (d.nt * d.Frmax + d.C * 3 * d.Famax + d.Famax) * es);
@@ -398,6 +404,24 @@ __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __
   }
 }
 
+// Adds the forces of the segments of an owner, which lie on consecutive lanes, to the owner's: one thread per (owner,
+// component).  (A shared float atomic is a compare-and-swap loop: S lanes on one word cost S round trips, most of the time
+// of a force pass when four warps share an atom and S goes up to 16.)
+template <class T, int NW>
+__device__ __forceinline__ void flush_segments(int oo, int base, int S, int nseg, int lane, T fx, T fy, T fz,
+                                               T* __restrict__ fo, T* __restrict__ part) {
+  part[lane * 3] = fx; part[lane * 3 + 1] = fy; part[lane * 3 + 2] = fz;
+  block_sync<NW>();
+  const int o0 = base / S, last = min(nseg - base, 32 * NW), cnt = (base + last - 1) / S + 1 - o0;
+  for (int q = lane; q < 3 * cnt; q += 32 * NW) {
+    const int o = o0 + q / 3, c = q % 3, l1 = min((o + 1) * S - base, last);
+    T f = T(0);
+    for (int l = max(o * S - base, 0); l < l1; l++) f += part[l * 3 + c];
+    fo[(oo + o) * 3 + c] += f;
+  }
+  block_sync<NW>();
+}
+
 // ---- ordered pairs (owner j, partner k): forces.  The list of an owner's partners is cut into S segments and
 // every lane takes one (owner, segment): the owner's data - including its table entries already multiplied by the
 // channel weights - and its force accumulator stay in registers for the whole segment, all lanes run the same
@@ -492,20 +516,149 @@ __device__ __forceinline__ void pairs_force(const typename Vec4<T>::type* __rest
     } else {
       const T fx = ax + as * uj.x, fy = ay + as * uj.y, fz = az + as * uj.z;
       if (active) { fix -= fx; fiy -= fy; fiz -= fz; }
-      // the segments of an owner lie on consecutive lanes: one thread per (owner, component) adds them up.  (A shared
-      // float atomic is a compare-and-swap loop: S lanes on one word cost S round trips, most of this function's time
-      // when four warps share an atom and S goes up to 16.  One warp, S <= 4, keeps the atomics: this form costs it
-      // registers, 5 % of a force sweep.)
-      part[lane * 3] = fx; part[lane * 3 + 1] = fy; part[lane * 3 + 2] = fz;
-      block_sync<NW>();
-      const int o0 = base / S, last = min(nseg - base, 32 * NW), cnt = (base + last - 1) / S + 1 - o0;
-      for (int q = lane; q < 3 * cnt; q += 32 * NW) {
-        const int o = o0 + q / 3, c = q % 3, l1 = min((o + 1) * S - base, last);
-        T f = T(0);
-        for (int l = max(o * S - base, 0); l < l1; l++) f += part[l * 3 + c];
-        fo[(oo + o) * 3 + c] += f;
+      flush_segments<T, NW>(oo, base, S, nseg, lane, fx, fy, fz, fo, part);
+    }
+  }
+}
+
+// ---- the same in fp32 with TWO PARTNERS per packed instruction (the PACK form of the kernel, for models with FP_CH
+// channels per class or fewer: the geometry is formed once per pass of FP_CH channels, and with 13 channels the form above
+// with its eight per pass is the faster one, 73 against 78 us).  Packing channels leaves the geometry of a pair, its force
+// and the loop itself scalar and pads five channels to six; packing partners halves all of it.  For that the partners lie
+// in pairs, one record of FP_REC 16-byte words per pair: x x' y y' | z z' fc/2 fc'/2 | per channel exp(a1 fc) of both,
+// exp(a2 fc) of both.  Every species group starts a pair, an odd group ends with a partner of cutoff zero, which adds
+// nothing, and within one species the owner itself is masked the same way.  Lanes with the same segment number read the
+// same record (one address per load and segment; the odd record length keeps different segments out of each other's
+// banks).  The owner's constants are 64-bit registers that hold the value twice, made where the compiler cannot see that
+// the halves agree: left to itself it keeps one copy and spends a move per use.  Against the form above: training step of
+// 4 x 768 atoms 160.3 -> 159.0 us, of 2 x 96 85.5 -> 83.9 us, 6,144-atom domain 133.0 -> 131.0 us, 24,576-atom call 541 ->
+// 537 us: instruction issue is still the bound, and half of the sweep's instructions lie outside the pair loop.
+typedef unsigned long long f2x;
+__device__ __forceinline__ f2x x_dup(float v) {
+  f2x r;
+  asm volatile("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ f2x x_pack(float a, float b) {
+  f2x r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 x_split(f2x v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f2x x_mul(f2x a, f2x b) {
+  f2x r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2x x_fma(f2x a, f2x b, f2x c) {
+  f2x r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// Segments per owner of a pass: fewest (iterations + 2) * rounds; the 2 stands for loading the owner and flushing.  Lane s
+// weighs s + 1 segments.
+template <int NW>
+__device__ __forceinline__ int choose_segments(int no, int npt) {
+  constexpr int MOST = NW == 1 ? 4 : 16;
+  const int s = (threadIdx.x & (MOST - 1)) + 1;
+  const int sg = (npt + s - 1) / s, rounds = (no * s + 32 * NW - 1) / (32 * NW);
+  return (int)(__reduce_min_sync(0xffffffffu, (unsigned)(rounds * (sg + 2) * 32 + s)) & 31u);
+}
+template <int NCH, bool SAME, int NW>
+__device__ __forceinline__ void pairs_force2(const float4* __restrict__ U, const float4* __restrict__ V,
+                                             const float4* __restrict__ rec, const f2x* __restrict__ beta,
+                                             const float4* __restrict__ cw, int oo, int jp0, int kp0, int no, int npp,
+                                             int lane, float* __restrict__ fo, float* __restrict__ part, float& fix,
+                                             float& fiy, float& fiz) {
+  if (no <= 0 || npp <= 0) return;
+  const int S = choose_segments<NW>(no, npp), seg = (npp + S - 1) / S;
+  const int nseg = no * S;
+  const f2x one2 = x_dup(1.0f);
+  for (int base = 0; base < nseg; base += 32 * NW) {
+    const int sidx = base + lane;
+    const bool active = sidx < nseg;
+    int ow = 0;  // sidx / S (exact for these ranges)
+    if (active) {
+      if (NW == 1) ow = (S == 1) ? sidx : (S == 2) ? (sidx >> 1) : (S == 4) ? (sidx >> 2) : (sidx * 21846) >> 16;
+      else ow = (sidx * ((65535 + S) / S)) >> 16;
+    }
+    const int pos = sidx - ow * S, s0 = pos * seg;
+    const int j = oo + ow, jp = jp0 + (ow >> 1);
+    const float4 uj = U[j];
+    f2x a1w[NCH], a2w[NCH], b1w[NCH], b2w[NCH];  // w*A1_j, w*A2_j, alpha1*w*A1_j, alpha2*w*A2_j
+#pragma unroll
+    for (int c = 0; c < NCH; c++) {
+      const float* A = reinterpret_cast<const float*>(rec + jp * FP_REC + 2 + c) + (ow & 1);
+      const float4 w = cw[c];  // weight, alpha1 * weight, alpha2 * weight
+      const float A1 = A[0], A2 = A[2];
+      a1w[c] = x_dup(A1 * w.x);
+      a2w[c] = x_dup(A2 * w.x);
+      b1w[c] = x_dup(A1 * w.y);
+      b2w[c] = x_dup(A2 * w.z);
+    }
+    const f2x ux = x_dup(uj.x), uy = x_dup(uj.y), uz = x_dup(uj.z), fj = x_dup(uj.w),
+              fs = x_dup(uj.w * Ex<float>::scale());
+    f2x ax = 0, ay = 0, az = 0, ac = 0, ah = 0;  // bit patterns of (0, 0)
+    const int s1 = active ? min(s0 + seg, npp) : s0;
+    const ulonglong2* r = reinterpret_cast<const ulonglong2*>(rec + (kp0 + s0) * FP_REC);
+    const int hole = SAME ? (ow >> 1) - s0 : 0;  // the step that meets the owner itself
+#pragma unroll 1
+    for (int p = 0; p < s1 - s0; p++, r += FP_REC) {
+      const ulonglong2 g0 = r[0], g1 = r[1];
+      f2x F = g1.y;  // fc/2
+      if (SAME) {
+        float2 f = x_split(F);
+        if (p == hole) { if (ow & 1) f.y = 0.0f; else f.x = 0.0f; }
+        F = x_pack(f.x, f.y);
       }
-      block_sync<NW>();
+      const f2x cs = x_fma(ux, g0.x, x_fma(uy, g0.y, x_mul(uz, g1.x)));
+      const f2x hF = x_fma(cs, F, F);  // (1 + cos)/2 * fc_k
+      const f2x tt = x_mul(hF, fj), ts = x_mul(hF, fs);
+      f2x D = 0, B = 0;
+#pragma unroll
+      for (int c = 0; c < NCH; c++) {
+        const ulonglong2 t = r[2 + c];
+        const f2x be = beta[c];
+        const float2 arg = x_split(x_mul(be, ts));
+        const f2x E = x_pack(ex2_fast(arg.x), ex2_fast(arg.y));
+        const f2x sum = x_fma(a1w[c], t.y, x_mul(a2w[c], t.x));             // w (S2 + S1)
+        D = x_fma(x_mul(x_fma(be, tt, one2), E), sum, D);                   // w e^{bt} (1 + bt) (S1 + S2)
+        B = x_fma(E, x_fma(b1w[c], t.y, x_mul(b2w[c], t.x)), B);            // w e^{bt} (a1 S2 + a2 S1)
+      }
+      // f_ij = cjk*u_k + (...)*u_j, the owner's factors applied at the end
+      const f2x dk = x_mul(D, F);
+      ax = x_fma(dk, g0.x, ax);
+      ay = x_fma(dk, g0.y, ay);
+      az = x_fma(dk, g1.x, az);
+      ac = x_fma(cs, dk, ac);
+      ah = x_fma(hF, x_fma(fj, B, D), ah);
+    }
+    const float2 vj = *reinterpret_cast<const float2*>(V + j);  // 1/r, dfc/dr
+    const float cj = uj.w * vj.x;
+    const float2 fx2 = x_split(ax), fy2 = x_split(ay), fz2 = x_split(az), c2 = x_split(ac), h2 = x_split(ah);
+    const float asum = vj.y * (h2.x + h2.y) - cj * (c2.x + c2.y);
+    float fx = cj * (fx2.x + fx2.y) + asum * uj.x, fy = cj * (fy2.x + fy2.y) + asum * uj.y,
+          fz = cj * (fz2.x + fz2.y) + asum * uj.z;  // zero on lanes that are not active
+    fix -= fx; fiy -= fy; fiz -= fz;
+    if (NW == 1) {
+      // the segments of an owner lie on consecutive lanes; its first lane of this round collects them.  (Shared float
+      // atomics are compare-and-swap loops, S round trips each.)
+      float gx = fx, gy = fy, gz = fz;
+      for (int d = 1; d < S; d++) {
+        const float tx = __shfl_down_sync(0xffffffffu, fx, d), ty = __shfl_down_sync(0xffffffffu, fy, d),
+                    tz = __shfl_down_sync(0xffffffffu, fz, d);
+        if (pos + d < S && lane + d < 32) { gx += tx; gy += ty; gz += tz; }
+      }
+      if (active && (pos == 0 || lane == 0)) {
+        fo[j * 3] += gx; fo[j * 3 + 1] += gy; fo[j * 3 + 2] += gz;
+      }
+      __syncwarp();
+    } else {
+      flush_segments<float, NW>(oo, base, S, nseg, lane, fx, fy, fz, fo, part);
     }
   }
 }
@@ -536,8 +689,8 @@ __device__ __forceinline__ void by_channels(int nch, Fn&& fn) {
 }
 
 // One block of NW warps per central atom.  VIR (force mode only) adds the virial; it is a template parameter so
-// that the training step's force sweep does not carry its registers.
-template <class T, int MODE, bool VIR, int NW>
+// that the training step's force sweep does not carry its registers.  PACK: partner pairs (fp32 forces).
+template <class T, int MODE, bool VIR, int NW, bool PACK>
 __global__ void __launch_bounds__(32 * NW, (SweepMinBlocks<MODE, sizeof(T)>::value + NW - 1) / NW)
     k_sweep(ModelDev md, SweepArgs<T> a, SweepSmem L) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -764,7 +917,80 @@ __global__ void __launch_bounds__(32 * NW, (SweepMinBlocks<MODE, sizeof(T)>::val
   block_sync<NW>();
 
   // ------------------------------------------------------------------ angular part
-  for (int ta = 0; ta < nt; ta++) {
+  if constexpr (PACK) {
+    float4* rec = reinterpret_cast<float4*>(smem_raw + L.tab);
+    float4* cw = rec + FP_REC * fp_pairs(nr);  // the pass's channel weights and beta
+    float2* beta = reinterpret_cast<float2*>(cw + FP_CH);
+    // geometry of the angular neighbours in pairs
+    for (int q = 0, p0 = 0; q < nt; q++) {
+      const int n_ = hdr[6 + q], np_ = (n_ + 1) >> 1;
+      for (int p = tid; p < np_; p += LANES) {
+        const float4 u0 = U[off[q] + 2 * p];
+        float4 u1 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (2 * p + 1 < n_) u1 = U[off[q] + 2 * p + 1];
+        rec[FP_REC * (p0 + p)] = make_float4(u0.x, u1.x, u0.y, u1.y);
+        rec[FP_REC * (p0 + p) + 1] = make_float4(u0.z, u1.z, 0.5f * u0.w, 0.5f * u1.w);
+      }
+      p0 += np_;
+    }
+    block_sync<NW>();
+    for (int ta = 0, pa = 0; ta < nt; ta++) {
+      const int na_ = hdr[6 + ta], npa = (na_ + 1) >> 1;
+      for (int tb = ta, pn = pa; tb < nt; tb++) {
+        const int s = ta + tb, nb_ = hdr[6 + tb], npb = (nb_ + 1) >> 1, pb = pn;
+        pn += npb;
+        const bool same = (ta == tb);
+        if ((same ? na_ < 2 : na_ * nb_ == 0) || s >= md.ncls) continue;
+        const float* chq = reinterpret_cast<const float*>(chq_all + s * sl.maxp);
+        const float* chr = reinterpret_cast<const float*>(chr_all + s * sl.maxp);
+        const float* wch = reinterpret_cast<const float*>(wch_all + s * sl.maxp);
+        const int nact = nact_s[s];
+#pragma unroll 1
+        for (int c0 = 0; c0 < nact; c0 += FP_CH) {
+          const int nch = min(FP_CH, nact - c0);
+          // tables of the pairs of the two species; x / nu by a reciprocal (exact: x < 2^10)
+          const int nu = same ? npa : npa + npb, rcp = (int)__fdividef(1048576.0f, (float)nu) + 1;
+          for (int x = tid; x < nu * nch; x += LANES) {
+            const int c = (x * rcp) >> 20, r = x - c * nu, kp = r < npa ? pa + r : pb + (r - npa);
+            const int ch = c0 + c, ci = (ch >> 1) * 4 + (ch & 1);
+            const float4 g = rec[FP_REC * kp + 1];
+            const float al1 = chq[ci] * (2.0f * Ex<float>::scale()), al2 = chq[ci + 2] * (2.0f * Ex<float>::scale());
+            rec[FP_REC * kp + 2 + c] =
+                make_float4(ex2_fast(al1 * g.z), ex2_fast(al1 * g.w), ex2_fast(al2 * g.z), ex2_fast(al2 * g.w));
+          }
+          if (tid < nch) {
+            const int ch = c0 + tid, ci = (ch >> 1) * 4 + (ch & 1);
+            const float w = wch[ch];
+            cw[tid] = make_float4(w, chq[ci] * w, chq[ci + 2] * w, 0.0f);
+            beta[tid] = mk2(chr[ch], chr[ch]);
+          }
+          block_sync<NW>();
+          auto go = [&](auto tag) {
+            constexpr int NCH = decltype(tag)::value;
+            const f2x* be = reinterpret_cast<const f2x*>(beta);
+            if (same) {
+              pairs_force2<NCH, true, NW>(U, V, rec, be, cw, off[ta], pa, pa, na_, npa, tid, xtra, part, fix, fiy, fiz);
+            } else {
+#pragma unroll 1
+              for (int pass = 0; pass < 2; pass++)
+                pairs_force2<NCH, false, NW>(U, V, rec, be, cw, pass ? off[tb] : off[ta], pass ? pb : pa, pass ? pa : pb,
+                                             pass ? nb_ : na_, pass ? npa : npb, tid, xtra, part, fix, fiy, fiz);
+            }
+          };
+          switch (nch) {
+            case 1: go(std::integral_constant<int, 1>()); break;
+            case 2: go(std::integral_constant<int, 2>()); break;
+            case 3: go(std::integral_constant<int, 3>()); break;
+            case 4: go(std::integral_constant<int, 4>()); break;
+            default: go(std::integral_constant<int, 5>()); break;
+          }
+          block_sync<NW>();  // the next pass rewrites the tables
+        }
+      }
+      pa += npa;
+    }
+  }
+  for (int ta = 0; ta < (PACK ? 0 : nt); ta++) {
     for (int tb = ta; tb < nt; tb++) {
       const int s = ta + tb;
       const int na_ = hdr[6 + ta], nb_ = hdr[6 + tb], oa = off[ta], ob = off[tb];

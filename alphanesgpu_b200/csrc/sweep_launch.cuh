@@ -1,21 +1,22 @@
 // Launches of the sweeps (sweep.cuh), instantiated for REAL by sweep_f32.cu and sweep_f64.cu.
 #include "model.cuh"
 
-template <class T, int MODE, int NW>
+template <class T, int MODE, int NW, bool PACK = false>
 static int launch_sweep_nw(stafb_model* m, cudaStream_t s, const SweepCall<T>& call) {
   const ModelDev& d = m->md;
   const int nr = m->ctx->nr;
-  const SweepSmem L = sweep_smem<T>(d, m->sl, nr, MODE, NW);
+  const SweepSmem L = sweep_smem<T>(d, m->sl, nr, MODE, NW, PACK);
   const size_t sm = (size_t)L.total;
   if (sm > m->smem_limit) return STAFB_ERR_CAPACITY;
-  static bool attr_dev[MAX_DEVICES] = {false};  // per instantiation (T, MODE, NW) and device
+  constexpr bool F = MODE == MODE_FORCE;
+  static bool attr_dev[MAX_DEVICES] = {false};  // per instantiation (T, MODE, NW, PACK) and device
   bool& attr_done = attr_dev[device_slot()];
   if (sm > 48 * 1024 && !attr_done) {
-    STAFB_CUDA_OK(cudaFuncSetAttribute(k_sweep<T, MODE, false, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    STAFB_CUDA_OK(cudaFuncSetAttribute(k_sweep<T, MODE, false, NW, PACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)m->smem_limit));
-    if (MODE == MODE_FORCE)
-      STAFB_CUDA_OK(cudaFuncSetAttribute(k_sweep<T, MODE, MODE == MODE_FORCE, NW>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m->smem_limit));
+    if (F)
+      STAFB_CUDA_OK(cudaFuncSetAttribute(k_sweep<T, MODE, F, NW, PACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)m->smem_limit));
     attr_done = true;
   }
   SweepArgs<T> a;
@@ -30,10 +31,10 @@ static int launch_sweep_nw(stafb_model* m, cudaStream_t s, const SweepCall<T>& c
   a.vout = call.vout; a.nv = m->nv; a.vir = call.vir; a.status = call.status;
   a.vacc = call.vacc; a.vlab = call.vlab; a.vscale = call.vscale;
   const int blocks = call.nf * d.N;
-  if (MODE == MODE_FORCE && call.vir)
-    STAFB_CUDA_OK(launch_chained(k_sweep<T, MODE, MODE == MODE_FORCE, NW>, blocks, 32 * NW, sm, s, d, a, L));
+  if (F && call.vir)
+    STAFB_CUDA_OK(launch_chained(k_sweep<T, MODE, F, NW, PACK>, blocks, 32 * NW, sm, s, d, a, L));
   else
-    STAFB_CUDA_OK(launch_chained(k_sweep<T, MODE, false, NW>, blocks, 32 * NW, sm, s, d, a, L));
+    STAFB_CUDA_OK(launch_chained(k_sweep<T, MODE, false, NW, PACK>, blocks, 32 * NW, sm, s, d, a, L));
   m->ctx->launches++;
   return STAFB_OK;
 }
@@ -45,7 +46,13 @@ int launch_sweep(stafb_model* m, cudaStream_t s, const SweepCall<T>& call) {
   // 96 / 300 / 450 atoms: fp32 97 -> 88, 103 -> 97, 110 -> 105 us, fp64 133 -> 112, 141 -> 140, 154 -> 154 us; at 768
   // atoms one warp per atom is the faster form (119 against 141 us).
   static const int few = (sizeof(T) == 4 ? 3 : 2) * sm_count();
-  if (call.nf * m->md.N <= few) return launch_sweep_nw<T, MODE, 4>(m, s, call);
+  const bool small = call.nf * m->md.N <= few;
+  if constexpr (MODE == MODE_FORCE && sizeof(T) == 4) {
+    // FP_CH channels per class or fewer on average: partner pairs
+    if (m->md.Famax <= FP_CH * m->md.ncls)
+      return small ? launch_sweep_nw<T, MODE, 4, true>(m, s, call) : launch_sweep_nw<T, MODE, 1, true>(m, s, call);
+  }
+  if (small) return launch_sweep_nw<T, MODE, 4>(m, s, call);
   return launch_sweep_nw<T, MODE, 1>(m, s, call);
 }
 

@@ -307,6 +307,26 @@ def test_train_step_with_other_channel_counts(oracle, frame0, channels, dtype):
     m.close()
 
 
+@pytest.mark.parametrize("name,seeds", [("water96", [1000]), ("water768", [1100])])
+@pytest.mark.parametrize("channels", [(5, 5, 5), (0, 6, 9), (1, 2, 4)])
+def test_forces_of_partner_pairs(oracle, frame0, channels, name, seeds):
+    """The fp32 force sweep on partner pairs (five channels per class or fewer on average): one pass, a second pass of
+    one and of four channels, odd species groups; four warps per atom (96 atoms) and one (768)."""
+    from alphanesgpu_b200 import train as T
+    from alphanesgpu_b200.model import StafModel
+    from alphanesgpu_b200.params import ModelShape
+    pos, box, tipos = synth.water_frames(name, seeds)
+    maps = dict(map_rad_afs={0: [3, 2], 1: [1, 4]}, map_ang_afs={0: list(channels), 1: list(channels[::-1])})
+    shape = ModelShape(nt=2, tipos=list(tipos), Fr=[5, 5], Fa=[sum(channels)] * 2, widths=[16, 1])
+    theta, emb = T.init_params(shape, maps, 3)
+    m = StafModel(shape, CFG, theta, emb, 1, dtype=torch.float32)
+    ref = oracle.energy_force_grad(CFG, shape.desc(), pos, box, shape.type_map, theta, emb, np.float32,
+                                   per_atom_energy=False)
+    e, f = m.energy_force(pos.astype(np.float32), box.astype(np.float32))
+    assert rel_err(e.cpu().numpy(), ref["energy"]) <= 1e-5 and rel_err(f.cpu().numpy(), ref["force"]) <= 1e-5
+    m.close()
+
+
 def test_adam_matches_reference_formula():
     from alphanesgpu_b200.model import StafModel
     pos, box, tipos = synth.water_frames("water96", [1000])
