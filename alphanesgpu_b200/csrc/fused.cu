@@ -37,14 +37,16 @@ __global__ void k_prep(ModelDev md, const T* __restrict__ theta, const T* __rest
   // be mapped host memory (the host-buffer entry points), which is to be read exactly once
   for (size_t q = tid; q < nflab; q += st) flab_dst[q] = flab_src[q];
   {
-    const int gw = (int)(tid >> 5), lane = threadIdx.x & 31;
-    if (gw < md.nt * md.ncls) {
-      const int t = gw / md.ncls, s = gw - t * md.ncls;
-      spar_fill_class<T>(md, sl, spar + (size_t)t * spar_stride, t, s, theta, emb, lane);
+    const int lane = threadIdx.x & 31, n3 = md.nt * md.ncls, n2 = md.nt * md.nt;
+    for (int gw = (int)(tid >> 5); gw < n3 + n2; gw += (int)(st >> 5)) {
+      if (gw < n3) {
+        const int t = gw / md.ncls, s = gw - t * md.ncls;
+        spar_fill_class<T>(md, sl, spar + (size_t)t * spar_stride, t, s, theta, emb, lane);
+      } else {
+        const int t = (gw - n3) / md.nt, q = gw - n3 - t * md.nt;
+        spar_fill_radial<T>(md, sl, spar + (size_t)t * spar_stride, t, q, theta, emb, lane);
+      }
     }
-    for (int t = 0; t < md.nt; t++)
-      for (size_t idx = tid; idx < (size_t)md.nt * md.Fr[t]; idx += st)
-        spar_fill_radial<T>(md, sl, spar + (size_t)t * spar_stride, t, theta, emb, (int)idx);
   }
   for (size_t q = tid; q < na / 4; q += st) reinterpret_cast<int*>(a)[q] = 0;
   for (size_t q = tid; q < nb / 4; q += st) reinterpret_cast<int*>(b)[q] = 0;

@@ -118,18 +118,20 @@ template <> struct SweepMinBlocks<MODE_FGRAD, 8> { static constexpr int value = 
 // ---- per-species parameter block (global memory, written by k_prep at the start of every evaluation; a sweep
 // copies the block of its central species into shared memory).  Byte offsets inside a block:
 //   [0, 32)  int nact[8]            active channels (squared embedding != 0) of class s = ta + tb
+//   [32, 48) int nrad[4]            active radial channels of neighbour species q
 //   actc     uchar [ncls][Famax]    their channel numbers, compacted
 //   chq      T4 [ncls][maxp]        channel pair (2p, 2p+1) of the compacted list: alpha1 x2, alpha2 x2
 //   chr      T2 [ncls][maxp]        beta x2
 //   che      T2 [ncls][maxp]        squared embedding x2 (an odd count is padded with an all-zero channel)
-//   rpar     T4 [nt][Frmax]         radial channels: alpha2b*log2(e), alpha2b, squared embedding, 0
+//   rpar     T4 [nt][Frmax]         active radial channels, compacted: alpha2b*log2(e), alpha2b, squared embedding, channel
+//                                   number; the rest of a row is zero
 struct SparLayout {
   int actc, chq, chr, che, rpar, total, maxp;
 };
 template <class T>
 static inline SparLayout spar_layout(const ModelDev& d) {
   SparLayout L;
-  int o = 32;
+  int o = 48;
   auto take = [&](int bytes) { int r = o; o += (bytes + 15) & ~15; return r; };
   L.maxp = (d.Famax + 1) / 2 > 0 ? (d.Famax + 1) / 2 : 1;
   L.actc = take(d.ncls * (d.Famax > 0 ? d.Famax : 1));
@@ -160,11 +162,12 @@ __device__ __forceinline__ void spar_fill_class(const ModelDev& md, const SparLa
   for (int c0 = 0; c0 < Fa; c0 += 32) {
     const int c = c0 + lane;
     const T ee = c < Fa ? e3[c] : T(0);
+    // fetched beside the embedding, not after it
+    const T al1 = c < Fa ? a3[3 * c] : T(0), al2 = c < Fa ? a3[3 * c + 1] : T(0), be = c < Fa ? a3[3 * c + 2] : T(0);
     const bool p = ee != T(0);
     const unsigned bal = __ballot_sync(0xffffffffu, p);
     if (p) {
       const int slot = nact + __popc(bal & lt), pr = slot >> 1, h = slot & 1;
-      const T al1 = a3[3 * c], al2 = a3[3 * c + 1], be = a3[3 * c + 2];
       actc[slot] = (unsigned char)c;
       chq[pr * 4 + h] = al1; chq[pr * 4 + 2 + h] = al2;
       chr[pr * 2 + h] = be;
@@ -183,13 +186,27 @@ __device__ __forceinline__ void spar_fill_class(const ModelDev& md, const SparLa
   }
 }
 
+// The radial channels of (species t, neighbour species q): one warp, as above.
 template <class T>
-__device__ __forceinline__ void spar_fill_radial(const ModelDev& md, const SparLayout& sl, unsigned char* blk, int t,
-                                                 const T* __restrict__ theta, const T* __restrict__ emb, int idx) {
-  const int Fr = md.Fr[t], q = idx / Fr, c = idx - q * Fr;
-  T* rp = reinterpret_cast<T*>(blk + sl.rpar) + ((size_t)q * md.Frmax + c) * 4;
-  const T al = theta[md.off_a2[t] + idx];
-  rp[0] = al * Ex<T>::scale(); rp[1] = al; rp[2] = emb[md.off_emb[t] + idx]; rp[3] = T(0);
+__device__ __forceinline__ void spar_fill_radial(const ModelDev& md, const SparLayout& sl, unsigned char* blk, int t, int q,
+                                                 const T* __restrict__ theta, const T* __restrict__ emb, int lane) {
+  const int Fr = md.Fr[t];
+  T* row = reinterpret_cast<T*>(blk + sl.rpar) + (size_t)q * md.Frmax * 4;
+  int nact = 0;
+  for (int c0 = 0; c0 < Fr; c0 += 32) {
+    const int c = c0 + lane;
+    const T ee = c < Fr ? emb[md.off_emb[t] + q * Fr + c] : T(0);
+    const T al = c < Fr ? theta[md.off_a2[t] + q * Fr + c] : T(0);
+    const bool p = ee != T(0);
+    const unsigned bal = __ballot_sync(0xffffffffu, p);
+    if (p) {
+      T* rp = row + (nact + __popc(bal & ((1u << lane) - 1u))) * 4;
+      rp[0] = al * Ex<T>::scale(); rp[1] = al; rp[2] = ee; rp[3] = (T)c;
+    }
+    nact += __popc(bal);
+  }
+  for (int x = 4 * nact + lane; x < 4 * md.Frmax; x += 32) row[x] = T(0);
+  if (lane == 0) reinterpret_cast<int*>(blk)[8 + q] = nact;
 }
 
 // The virial of a frame is accumulated by every centre of the frame: 9 words would take one atomic add per atom
@@ -372,17 +389,16 @@ __device__ __forceinline__ void pairs_unordered(const typename Vec4<T>::type* __
       // its derivatives:  d/da1 = Z1 (sj H1 + t Pj/2) + Z2 (sk H2 + t Pk/2),  d/da2 with sj, sk and Pj, Pk
       // exchanged inside each bracket,  d/dbeta = t [Z1 (H1 + Q/2) + Z2 (H2 + Q/2)]
       // (STAF/src/grad_force/ang/reforce.cu.cc:47-231).
-      const T2 pj = *reinterpret_cast<const T2*>(V + j), pk = *reinterpret_cast<const T2*>(V + k);  // 1/r, dfc/dr
-      const T hf = T(0.5) * fcj * fck;
-      const T ajk = hf * pj.x, akj = hf * pk.x;
-      const T bjk = -cs * ajk + half * pj.y * fck;
-      const T bkj = -cs * akj + half * pk.y * fcj;
-      const T4 dFj = dF[j], dFk = dF[k];
-      const T djuk = dFj.x * uk.x + dFj.y * uk.y + dFj.z * uk.z;
-      const T dkuj = dFk.x * uj.x + dFk.y * uj.y + dFk.z * uj.z;
-      const T Qh = T(0.5) * (ajk * djuk + bjk * dFj.w + akj * dkuj + bkj * dFk.w);
-      const T Pjh = T(0.5) * tt * pj.y * dFj.w;
-      const T Pkh = T(0.5) * tt * pk.y * dFk.w;
+      // What depends on one neighbour only is formed before the pair loop: dF[k] holds W/4 with W = fc/r (dF - (dF.u) u)
+      // and q/2 with q = dfc/dr (dF.u), and
+      //   Q = fc_k W_j.u_k / 2 + fc_j W_k.u_j / 2 + (1 + cos)/2 (fc_k q_j + fc_j q_k),
+      // 13 operations where the pair's four products with dF, 1/r and dfc/dr took 27 (eight steps of 4 x 768 atoms in fp64
+      // 2,557 -> 2,498 us, of the wide model in fp32 2,730 -> 2,676 us, with the compacted radial channels).
+      const T4 Wj = dF[j], Wk = dF[k];
+      const T wju = Wj.x * uk.x + Wj.y * uk.y + Wj.z * uk.z;
+      const T wku = Wk.x * uj.x + Wk.y * uj.y + Wk.z * uj.z;
+      const T Qh = half * (fck * Wj.w + fcj * Wk.w) + (fck * wju + fcj * wku);
+      const T Pjh = tt * Wj.w, Pkh = tt * Wk.w;
       const T2 Qh2 = mk2(Qh, Qh), Pj2 = mk2(Pjh, Pjh), Pk2 = mk2(Pkh, Pkh);
 #pragma unroll
       for (int lp = 0; lp < NCHP; lp++) {
@@ -713,6 +729,7 @@ __global__ void __launch_bounds__(32 * NW, (SweepMinBlocks<MODE, sizeof(T)>::val
   const int* hdr = reinterpret_cast<const int*>(rowp + row_off_hdr(nr, ES));
   unsigned char* spb = smem_raw + L.spar;
   const int* nact_s = reinterpret_cast<const int*>(spb);
+  const int* nrad = nact_s + 8;
   const unsigned char* actc = spb + sl.actc;
   const T4* chq_all = reinterpret_cast<const T4*>(spb + sl.chq);
   const T2* chr_all = reinterpret_cast<const T2*>(spb + sl.chr);
@@ -747,7 +764,7 @@ __global__ void __launch_bounds__(32 * NW, (SweepMinBlocks<MODE, sizeof(T)>::val
   }
   if (MODE != MODE_FORCE)
     for (int q = tid; q < NACC; q += LANES) acc[q] = T(0);
-  if (NW > 1 && MODE != MODE_FORCE)
+  if (MODE != MODE_FORCE)
     for (int q = tid; q < nt * Frmax; q += LANES) rsum[q] = T(0);
   if (ES == 8 && tid < 16) et[tid] = (T)EXP16_TABLE[tid];
   chain_wait();
@@ -838,6 +855,11 @@ __global__ void __launch_bounds__(32 * NW, (SweepMinBlocks<MODE, sizeof(T)>::val
       }
       wch_all[idx] = w;
     }
+    // and 0.5 * e2 * netderiv of the radial ones
+    for (int idx = tid; idx < nt * Frmax; idx += LANES) {
+      const T4 rp = rpar[idx];
+      rsum[idx] = rp.z != T(0) ? T(0.5) * rp.z * chrow[(int)rp.w] : T(0);
+    }
   }
   block_sync<NW>();
 
@@ -854,10 +876,11 @@ __global__ void __launch_bounds__(32 * NW, (SweepMinBlocks<MODE, sizeof(T)>::val
         const T4 u = U[k], v = V[k];
         const T dk = v.z;
         T w = T(0);
-        for (int c = 0; c < Fr; c++) {
-          const T4 rp = rpar[tk * Frmax + c];
-          if (rp.z == T(0)) continue;
-          w += chrow[c] * (T(0.5) * rp.z * Ex<T>::f(rp.x * dk, et) * (T(1) + rp.y * dk));
+        const int c1 = (tk + 1) * Frmax;
+        for (int c = tk * Frmax; c < c1; c++) {
+          const T4 rp = rpar[c];
+          if (rp.z == T(0)) break;  // compacted
+          w += rsum[c] * (Ex<T>::f(rp.x * dk, et) * (T(1) + rp.y * dk));
         }
         const T g = w * v.w;
         gx = g * u.x; gy = g * u.y; gz = g * u.z;
@@ -866,48 +889,83 @@ __global__ void __launch_bounds__(32 * NW, (SweepMinBlocks<MODE, sizeof(T)>::val
       xtra[k * 3 + 0] = gx; xtra[k * 3 + 1] = gy; xtra[k * 3 + 2] = gz;
     }
   } else {
-    // one thread per (neighbour species q, channel c) walks that species' neighbours, so the sums over
-    // neighbours need no cross-lane reduction; the per-species partial sums of a channel are combined
-    // through rsum[] (several warps: each takes every NW-th neighbour).  AF, AFV: fingerprints; FGRAD: gradnet; all but
-    // AF: alpha2b terms.
-    const int nqc = nt * Fr;
-    for (int L0 = 0; L0 < nqc; L0 += 32) {
-      const int Lq = L0 + lane;
-      if (Lq < nqc) {
-        const int q = Lq / Fr, c = Lq - q * Fr;
-        const T4 rp = rpar[q * Frmax + c];
-        T gn = T(0), ga = T(0);
-        if (rp.z != T(0)) {
-          const T als = rp.x, al = rp.y;
-          const int r0_ = off[q] + (NW == 1 ? 0 : tid >> 5), r1_ = off[q + 1];
-          const T4* dF = reinterpret_cast<const T4*>(xtra);
-#pragma unroll 4
-          for (int r = r0_; r < r1_; r += NW) {
-            const T4 v = V[r];
-            const T dk = v.z;
-            const T ex = Ex<T>::f(als * dk, et);
-            if (MODE == MODE_FGRAD) {
-              const T qq = T(0.5) * v.w * dF[r].w;
-              gn += qq * ex * (T(1) + al * dk);
-              ga += qq * ex * dk * (T(2) + al * dk);
-            } else {
-              gn += dk * ex;
-              ga += ex * dk * dk;
-            }
-          }
-          gn *= rp.z;
-          ga *= (MODE == MODE_FGRAD ? chrow[c] : T(1)) * rp.z;
-        }
-        if (NW == 1) {
-          rsum[q * Frmax + c] = gn;
-          if (MODE != MODE_AF) acc[ACC_A2 + q * Frmax + c] = ga;
+    // SEG lanes per active (neighbour species q, channel c) walk that species' neighbours, as many as there are lanes for
+    // (several warps: each takes every NW-th neighbour), and add up by shuffles; the per-species sums of a channel are
+    // combined through rsum[].  AF, AFV: fingerprints; FGRAD: gradnet; all but AF: alpha2b terms.
+    // Inference and several warps per atom take one lane per row of rpar, active or not: their walks are short already and
+    // the counting costs more than it saves (24,576-atom call 545 -> 549 us, 96-atom evaluation 56 -> 57.5 us with it).
+    constexpr bool FLAT = MODE == MODE_AF || NW > 1;
+    int items = nt * Frmax;
+    if (!FLAT) {
+      items = 0;
+      for (int q = 0; q < nt; q++) items += nrad[q];
+    }
+    const int SEG = FLAT || items > 16 ? 1 : items > 10 ? 2 : items > 8 ? 3 : 4;
+    for (int L0 = 0; L0 < items; L0 += 32) {
+      const int it = L0 + (SEG == 1 ? lane : SEG == 2 ? lane >> 1 : SEG == 3 ? (lane * 21846) >> 16 : lane >> 2);
+      const int sg = lane - (it - L0) * SEG;
+      T gn = T(0), ga = T(0);
+      int q = 0, c = 0;
+      if (it < items) {
+        c = it;
+        if (FLAT) {
+          q = it / Frmax;
+          c = it - q * Frmax;
         } else {
-          atomicAdd(&rsum[q * Frmax + c], gn);
-          if (MODE != MODE_AF) atomicAdd(&acc[ACC_A2 + q * Frmax + c], ga);
+          while (c >= nrad[q]) c -= nrad[q++];
+        }
+        const T4 rp = rpar[q * Frmax + c];
+        c = (int)rp.w;
+        const T als = rp.x, al = rp.y;
+        const int r0_ = off[q] + (NW == 1 ? sg : (tid >> 5) + NW * sg), r1_ = FLAT && rp.z == T(0) ? 0 : off[q + 1];
+        const T4* dF = reinterpret_cast<const T4*>(xtra);
+#pragma unroll 4
+        for (int r = r0_; r < r1_; r += NW * SEG) {
+          const T4 v = V[r];
+          const T dk = v.z;
+          const T ex = Ex<T>::f(als * dk, et);
+          if (MODE == MODE_FGRAD) {
+            const T qq = T(0.5) * v.w * dF[r].w;
+            gn += qq * ex * (T(1) + al * dk);
+            ga += qq * ex * dk * (T(2) + al * dk);
+          } else {
+            gn += dk * ex;
+            ga += ex * dk * dk;
+          }
+        }
+        gn *= rp.z;
+        ga *= (MODE == MODE_FGRAD ? chrow[c] : T(1)) * rp.z;
+      }
+      T g1 = gn, a1 = ga;
+      for (int d = 1; d < SEG; d++) {
+        g1 += __shfl_down_sync(0xffffffffu, gn, d);
+        if (MODE != MODE_AF) a1 += __shfl_down_sync(0xffffffffu, ga, d);
+      }
+      if (it < items && sg == 0 && (!FLAT || gn != T(0) || ga != T(0))) {
+        if (NW == 1) {
+          rsum[q * Frmax + c] = g1;
+          if (MODE != MODE_AF) acc[ACC_A2 + q * Frmax + c] = a1;
+        } else {
+          atomicAdd(&rsum[q * Frmax + c], g1);
+          if (MODE != MODE_AF) atomicAdd(&acc[ACC_A2 + q * Frmax + c], a1);
         }
       }
     }
     block_sync<NW>();
+    if (MODE == MODE_FGRAD) {
+      // the pair loops want W/4 and q/2 of every neighbour (pairs_unordered)
+      T4* dF = reinterpret_cast<T4*>(xtra);
+      for (int k = tid; k < n; k += LANES) {
+        const T4 u = U[k];
+        const T2 v = *reinterpret_cast<const T2*>(V + k);  // 1/r, dfc/dr
+        const T4 d = dF[k];
+        const T w = T(0.25) * u.w * v.x;
+        T4 o;
+        o.x = w * (d.x - d.w * u.x); o.y = w * (d.y - d.w * u.y); o.z = w * (d.z - d.w * u.z);
+        o.w = T(0.5) * v.y * d.w;
+        dF[k] = o;
+      }
+    }
     for (int c = tid; c < Fr; c += LANES) {
       T v = T(0);
       for (int q = 0; q < nt; q++) v += rsum[q * Frmax + c];
@@ -1147,16 +1205,18 @@ __global__ void __launch_bounds__(32 * NW, (SweepMinBlocks<MODE, sizeof(T)>::val
     for (int c = Fr + Fa + tid; c < Fmax; c += LANES) a.out[gi * Fmax + c] = T(0);
     if (a.grad) {
       T* g2 = a.grad + md.off_a2[t];
-      for (int q = tid; q < nt * Fr; q += LANES) {
-        const T v = acc[ACC_A2 + (q / Fr) * Frmax + (q % Fr)];
-        if (v != T(0)) atomicAdd(g2 + q, v);
-      }
+      for (int q = 0; q < nt; q++)
+        for (int x = tid; x < nrad[q]; x += LANES) {
+          const int c = (int)rpar[q * Frmax + x].w;
+          atomicAdd(g2 + q * Fr + c, acc[ACC_A2 + q * Frmax + c]);
+        }
       T* g3 = a.grad + md.off_a3[t];
-      for (int q = tid; q < md.C * 3 * Fa; q += LANES) {
-        const int sc = q / 3, comp = q - sc * 3, s = sc / Fa, c = sc - s * Fa;
-        const T v = acc[ACC_A3 + (s * Famax + c) * 3 + comp];
-        if (v != T(0)) atomicAdd(g3 + q, v);
-      }
+      for (int s = 0; s < md.ncls; s++)
+        for (int x = tid; x < 3 * nact_s[s]; x += LANES) {
+          const int slot = x / 3, comp = x - 3 * slot, c = actc[s * Famax + slot];
+          const T v = acc[ACC_A3 + (s * Famax + c) * 3 + comp];
+          if (v != T(0)) atomicAdd(g3 + (s * Fa + c) * 3 + comp, v);
+        }
     }
   }
 }
