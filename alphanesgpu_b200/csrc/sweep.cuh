@@ -143,6 +143,13 @@ static inline SparLayout spar_layout(const ModelDev& d) {
   return L;
 }
 
+// What the rounding of alpha * log2(e) to fp32 drops: alike for every atom, it would not average out of the gradient.
+template <class T>
+__device__ __forceinline__ T scale_rest(T al, T als) {
+  if constexpr (sizeof(T) == 8) return T(0);
+  else return fmaf(al, 1.442695022f, -als) + al * 1.925963e-8f;
+}
+
 // Fills the block of (species t, class s): one warp; lanes over channels, ballot compaction of the active ones.
 template <class T>
 __device__ __forceinline__ void spar_fill_class(const ModelDev& md, const SparLayout& sl, unsigned char* blk, int t,
@@ -916,14 +923,14 @@ __global__ void __launch_bounds__(32 * NW, (SweepMinBlocks<MODE, sizeof(T)>::val
         }
         const T4 rp = rpar[q * Frmax + c];
         c = (int)rp.w;
-        const T als = rp.x, al = rp.y;
+        const T als = rp.x, al = rp.y, alr = scale_rest(al, als);
         const int r0_ = off[q] + (NW == 1 ? sg : (tid >> 5) + NW * sg), r1_ = FLAT && rp.z == T(0) ? 0 : off[q + 1];
         const T4* dF = reinterpret_cast<const T4*>(xtra);
 #pragma unroll 4
         for (int r = r0_; r < r1_; r += NW * SEG) {
           const T4 v = V[r];
           const T dk = v.z;
-          const T ex = Ex<T>::f(als * dk, et);
+          const T ex = Ex<T>::f(sizeof(T) == 4 ? als * dk + alr * dk : als * dk, et);
           if (MODE == MODE_FGRAD) {
             const T qq = T(0.5) * v.w * dF[r].w;
             gn += qq * ex * (T(1) + al * dk);
